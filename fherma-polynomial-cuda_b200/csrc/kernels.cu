@@ -18,8 +18,6 @@ namespace negacyclic {
 
 namespace {
 
-constexpr uint32_t kFull = 0xffffffffu;
-
 // One padded row: Lp words (16-byte aligned) from `limbs` words, zeros above.
 __device__ __forceinline__ void pad_row(const uint32_t* __restrict__ src, uint32_t* __restrict__ dst, uint32_t limbs,
                                         uint32_t padded, uint32_t lane) {
@@ -543,211 +541,253 @@ __global__ void __launch_bounds__(256) transpose_kernel(const uint32_t* __restri
 }
 
 // ---------------------------------------------------------------------------
-// Warp-wide multiword arithmetic over 32-word chunks.
-
-// Carry into this lane given per-lane generate/propagate (mutually exclusive)
-// and the chain bit entering lane 0; updates `chain` to the carry out of lane 31.
-// Treats the 32 lanes as one 32-bit addition of (g|p) + g + chain.
-__device__ __forceinline__ uint32_t chain_carry(bool generate, bool propagate, uint32_t& chain) {
-    const uint32_t lane = threadIdx.x & 31;
-    uint64_t g = __ballot_sync(kFull, generate), gp = g | __ballot_sync(kFull, propagate);
-    uint64_t full = gp + g + chain;
-    uint32_t carries = uint32_t(full ^ gp ^ g);
-    chain = uint32_t(full >> 32);
-    return (carries >> lane) & 1u;
-}
-
-__device__ __forceinline__ uint32_t word_or_zero(const uint32_t* v, int64_t at, uint32_t size) {
-    return (at >= 0 && at < int64_t(size)) ? v[at] : 0u;
-}
-
-// bits [at, at+32) of the little-endian word array v (size words)
-__device__ __forceinline__ uint32_t bits_word(const uint32_t* v, int64_t at, uint32_t size) {
-    int64_t w = at >= 0 ? at / 32 : -((-at + 31) / 32);
-    uint32_t offset = uint32_t(at - w * 32);
-    uint64_t lo = word_or_zero(v, w, size), hi = word_or_zero(v, w + 1, size);
-    return uint32_t(((hi << 32) | lo) >> offset);
-}
-
-// v[0..len) += term(w) (term < 2^32), with carry; returns the final carry.
-template <class Term>
-__device__ __forceinline__ uint32_t add_words(uint32_t* v, uint32_t len, Term term) {
-    const uint32_t lane = threadIdx.x & 31;
-    uint32_t chain = 0;
-    for (uint32_t base = 0; base < len; base += 32) {
-        uint32_t w = base + lane;
-        uint32_t x = w < len ? v[w] : 0u, y = w < len ? term(w) : 0u;
-        uint64_t sum = uint64_t(x) + y;
-        uint32_t low = uint32_t(sum);
-        uint32_t carry = chain_carry((sum >> 32) != 0, low == kFull, chain);
-        if (w < len) v[w] = low + carry;
-    }
-    __syncwarp();
-    return chain;
-}
-
-// v[0..len) -= term(w), with borrow; returns the final borrow.
-template <class Term>
-__device__ __forceinline__ uint32_t sub_words(uint32_t* v, uint32_t len, Term term) {
-    const uint32_t lane = threadIdx.x & 31;
-    uint32_t chain = 0;
-    for (uint32_t base = 0; base < len; base += 32) {
-        uint32_t w = base + lane;
-        uint32_t x = w < len ? v[w] : 0u, y = w < len ? term(w) : 0u;
-        uint32_t borrow = chain_carry(x < y, x == y, chain);
-        if (w < len) v[w] = x - y - borrow;
-    }
-    __syncwarp();
-    return chain;
-}
-
-// sign of (v - q) over len words (q[w] = 0 for w >= limbs): -1, 0, 1
-__device__ __forceinline__ int compare_q(const uint32_t* v, uint32_t len, const uint32_t* q, uint32_t limbs) {
-    const uint32_t lane = threadIdx.x & 31;
-    for (int64_t base = int64_t((len + 31) / 32 - 1) * 32; base >= 0; base -= 32) {
-        uint32_t w = uint32_t(base) + lane;
-        uint32_t x = w < len ? v[w] : 0u, y = w < limbs ? q[w] : 0u;
-        uint32_t differ = __ballot_sync(kFull, x != y);
-        if (differ) {
-            uint32_t top = 31 - __clz(differ);
-            int less = __shfl_sync(kFull, x < y ? 1 : 0, top);
-            return less ? -1 : 1;
-        }
-    }
-    return 0;
-}
-
-// One warp per coefficient; its words live in shared memory.
+// CRT quotient, carries and reduction mod q: one thread per coefficient.
 //
 // The CRT word sums split cleanly: words [0, L+2) are a carry-save form of
 // T = sum v_k M_k (< 2^(32(L+2)), so nothing carries out of them), words
 // L+2..L+4 a carry-save form of D = sum v_k floor(2^64/p_k). Hence
 //   K  = (D + 2^63) >> 64 straight from three word sums,
-//   T' = T + K*(-P mod q) in one carry pass over dots[w] + K*R[w],
-//   c  = T' - quotient*q in one signed carry pass, then at most three q's off.
-__global__ void reduce_kernel(ReduceParams prm, uint32_t stride) {
-    extern __shared__ uint32_t scratch[];
-    const uint32_t warp = threadIdx.x / 32, lane = threadIdx.x & 31;
-    const uint32_t warps = blockDim.x / 32;
-    uint32_t* v = scratch + size_t(warp) * stride;
-    const uint32_t limbs = prm.limbs, tlen = limbs + 2;
-    const uint32_t* q = prm.q;
-    for (uint32_t i = blockIdx.x * warps + warp; i < prm.n; i += gridDim.x * warps) {
-        const uint64_t* d = prm.dots + size_t(i) * prm.dots_stride;
-        // 1. K = (D + 2^63) >> 64, D = d[L+2] + d[L+3] 2^32 + d[L+4] 2^64 (each word sum < 2^56)
-        const uint64_t x0 = d[limbs + 2], x1 = d[limbs + 3], x2 = d[limbs + 4];
-        const uint64_t low = x0 + (x1 << 32);
-        const uint64_t high = (x1 >> 32) + x2 + (low < x0 ? 1 : 0);  // D = high 2^64 + low
-        const uint64_t kq = high + ((low + (1ull << 63)) < low ? 1 : 0);
-        // 2. T' = sum_w (d[w] + K R[w]) 2^(32w), collapsed to exact words in one carry pass. A lane
-        //    holds words w0 = base + 2 lane and w0 + 1 of a 64-word step: its two word sums meet
-        //    in-lane, the bits at 2^64 and up go to the next lane by a shuffle (< 2^25), and one
-        //    warp-wide carry resolution covers 64 words. The word sums come from DRAM in 16-byte
-        //    pairs, kBatch steps' worth before any is used, so one load latency covers kBatch steps
-        //    of the (serial) carry chain. K < 2r fits 32 bits.
-        constexpr uint32_t kBatch = 4;
-        const uint32_t k32 = uint32_t(kq);
-        uint32_t chain = 0, carried_high = 0;
-        for (uint32_t batch = 0; batch < tlen; batch += 64 * kBatch) {
-            uint64_t x0[kBatch], x1[kBatch];
+//   T' = T + K R (R = -P mod q), T' = x (mod q), T' < 2^48 q,
+//   c  = T' - quotient q, then at most three q's off.
+// The quotient is known before the carries are: Barrett needs the 128 bits of T' from top_shift
+// up, and the words below the window carry less than 2^26 into it. Starting the window two words
+// lower bounds the missing carry by one unit of the window's lowest bit, which can only make the
+// quotient smaller, by less than 2^-62 before the floor. So one pass over the row, lowest word
+// first, forms d[w] + K R[w] - quotient q and its carries at once.
+//
+// What bounds it: reading 8 (L+5) and writing 4 L bytes per coefficient. A thread's carry chain is
+// three dependent instructions per word, and 32 rows advance per warp instruction; a warp per
+// coefficient with a warp-wide carry resolution (the earlier form) issued 554 instructions per
+// coefficient at L = 55, 70 % of the issue slots, and took 50 us at N = 65536, L = 55 and 0.62 ms
+// at L = 1747.
+// Rows are read in chunks of 16 or 64 words through shared memory (16-byte cp.async, whole
+// 128-byte lines), two chunks ahead of the arithmetic. A pitch of 16 bytes over a multiple of 128
+// keeps the threads' 16-byte reads of their own rows free of bank conflicts, and the results go
+// back through the same slot, so that global stores are runs of 64 or 128 bytes. Measured against
+// the earlier form (stage between events): 624 -> 362 us at N = 65536, L = 1747 (1.38 GB, 3.8 TB/s),
+// 142 -> 90 us at N = 32768, L = 868, 49 -> 20.5 us at N = 65536, L = 55.
+
+// A row's step: kChunk words of every row of the warp, with the same words of q and R behind them.
+template <uint32_t kChunk>
+struct ReduceSlot {
+    static constexpr uint32_t kPitch = kChunk * 8 + 16;  // bytes per row
+    static constexpr uint32_t kBytes = 32 * kPitch + kChunk * 8;
+};
+constexpr uint32_t kReduceSlots = 3;
+
+__device__ __forceinline__ void cp_async_16(uint32_t smem, const void* global) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem), "l"(global) : "memory");
+}
+
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+
+template <int kPending>
+__device__ __forceinline__ void cp_async_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kPending) : "memory");
+}
+
+struct RowQuotient {
+    uint32_t k;         // CRT quotient K < 2r
+    uint32_t low, high; // Barrett quotient of T' by q
+};
+
+// K and the Barrett quotient of one row of word sums.
+__device__ __forceinline__ RowQuotient row_quotient(const uint64_t* d, const ReduceParams& prm) {
+    const uint32_t limbs = prm.limbs;
+    const int32_t tlen = int32_t(limbs) + 2;
+    // K = (D + 2^63) >> 64, D = d[L+2] + d[L+3] 2^32 + d[L+4] 2^64 (each word sum < 2^56)
+    const uint64_t x0 = d[limbs + 2], x1 = d[limbs + 3], x2 = d[limbs + 4];
+    const uint64_t low = x0 + (x1 << 32);
+    const uint64_t high = (x1 >> 32) + x2 + (low < x0 ? 1 : 0);  // D = high 2^64 + low
+    const uint32_t k = uint32_t(high + ((low + (1ull << 63)) < low ? 1 : 0));
+    // T' words at ws .. ws+4 (ws = floor(top_shift / 32), possibly negative), with the carry of the
+    // two words below
+    const int32_t ws = prm.top_shift >> 5;
+    const uint32_t offset = uint32_t(prm.top_shift) & 31u;
+    uint32_t z[5];
+    uint64_t acc = 0;
 #pragma unroll
-            for (uint32_t u = 0; u < kBatch; ++u) {
-                const uint32_t w0 = batch + 64 * u + 2 * lane;
-                uint64_t d0 = 0, d1 = 0;
-                if (w0 < tlen) {  // w0 + 1 < dots_stride: the row holds at least tlen + 3 words
-                    const ulonglong2 pair = *reinterpret_cast<const ulonglong2*>(d + w0);
-                    d0 = pair.x;
-                    d1 = w0 + 1 < tlen ? pair.y : 0ull;
-                }
-                const uint32_t r0 = w0 < limbs ? prm.minus_p[w0] : 0u, r1 = w0 + 1 < limbs ? prm.minus_p[w0 + 1] : 0u;
-                x0[u] = d0 + uint64_t(k32) * r0;  // < 2^57
-                x1[u] = d1 + uint64_t(k32) * r1;
-            }
-#pragma unroll
-            for (uint32_t u = 0; u < kBatch; ++u) {
-                const uint32_t base = batch + 64 * u;
-                if (base >= tlen) break;  // warp-uniform
-                const uint32_t w0 = base + 2 * lane;
-                const uint32_t top = uint32_t(x1[u] >> 32);
-                uint32_t below = __shfl_up_sync(kFull, top, 1);
-                if (lane == 0) below = carried_high;
-                carried_high = __shfl_sync(kFull, top, 31);
-                const uint64_t s0 = uint64_t(uint32_t(x0[u])) + below;                     // < 2^33
-                const uint64_t s1 = (x0[u] >> 32) + uint32_t(x1[u]) + uint32_t(s0 >> 32);  // < 2^33
-                uint32_t word0 = uint32_t(s0), word1 = uint32_t(s1);
-                const bool generate = (s1 >> 32) != 0;
-                const uint32_t carry = chain_carry(generate, !generate && (word0 & word1) == kFull, chain);
-                word0 += carry;
-                word1 += (carry != 0 && word0 == 0) ? 1u : 0u;
-                if (w0 < tlen) v[w0] = word0;
-                if (w0 + 1 < tlen) v[w0 + 1] = word1;
-            }
+    for (int32_t j = -2; j < 5; ++j) {
+        const int32_t w = ws + j;
+        if (w >= 0 && w < tlen) acc += d[w] + uint64_t(k) * prm.minus_p[w];
+        if (j >= 0) z[j] = uint32_t(acc);
+        acc >>= 32;
+    }
+    const uint64_t tl = uint64_t(__funnelshift_r(z[0], z[1], offset)) |
+                        (uint64_t(__funnelshift_r(z[1], z[2], offset)) << 32);
+    const uint64_t th = uint64_t(__funnelshift_r(z[2], z[3], offset)) |
+                        (uint64_t(__funnelshift_r(z[3], z[4], offset)) << 32);
+    const uint64_t prod_l_hi = __umul64hi(tl, prm.mu_low);
+    const uint64_t prod_h_lo = th * prm.mu_low, prod_h_hi = __umul64hi(th, prm.mu_low);
+    const uint64_t word1 = prod_l_hi + prod_h_lo;
+    const uint64_t word2 = prod_h_hi + (word1 < prod_l_hi ? 1 : 0);
+    const uint64_t quotient = th + word2 + ((tl + word1 < tl) ? 1 : 0);  // < 2^48
+    return RowQuotient{k, uint32_t(quotient), uint32_t(quotient >> 32)};
+}
+
+// Takes q off a row (limbs words in global memory, `over` above them) while it is not below q;
+// returns false if more than three subtractions were needed.
+__device__ __noinline__ bool correct_row(uint32_t* row, uint32_t over, const uint32_t* __restrict__ q,
+                                         uint32_t limbs) {
+    for (int corrections = 0;; ++corrections) {
+        if (over == 0) {
+            uint32_t w = limbs;
+            while (w > 0 && row[w - 1] == q[w - 1]) --w;
+            if (w > 0 && row[w - 1] < q[w - 1]) return true;
         }
-        __syncwarp();
-        // 3. Barrett quotient from the 128 bits of T' at q's top-64-bit window
-        const uint64_t tl = uint64_t(bits_word(v, prm.top_shift, tlen)) |
-                            (uint64_t(bits_word(v, int64_t(prm.top_shift) + 32, tlen)) << 32);
-        const uint64_t th = uint64_t(bits_word(v, int64_t(prm.top_shift) + 64, tlen)) |
-                            (uint64_t(bits_word(v, int64_t(prm.top_shift) + 96, tlen)) << 32);
-        const uint64_t prod_l_hi = __umul64hi(tl, prm.mu_low);
-        const uint64_t prod_h_lo = th * prm.mu_low, prod_h_hi = __umul64hi(th, prm.mu_low);
-        const uint64_t word1 = prod_l_hi + prod_h_lo;
-        const uint64_t word2 = prod_h_hi + (word1 < prod_l_hi ? 1 : 0);
-        const uint64_t quotient = th + word2 + ((tl + word1 < tl) ? 1 : 0);
-        const uint32_t ql = uint32_t(quotient), qh = uint32_t(quotient >> 32);
-        __syncwarp();
-        // 4. c = T' - quotient*q in one signed carry pass, two words per lane as in step 2. With
-        //    a_w = ql q[w], b_w = qh q[w-1]:
-        //    z_w = T'[w] - lo(a_w) - lo(b_w) - hi(a_{w-1}) - hi(b_{w-1})  in (-2^35, 2^32),
-        //    c_w = floor(z_w / 2^32) in [-8, 0] moves to word w + 1, leaving sw_w in [-8, 2^32) and a
-        //    one-bit borrow chain. A lane generates a borrow when sw1 < 0, or sw1 = 0 and sw0 < 0,
-        //    and passes one on when sw1 = sw0 = 0.
-        chain = 0;
-        uint64_t carry_hi = 0;  // hi(a)+hi(b) of the previous step's last word
-        int32_t carry_c = 0;    // signed word carry of the previous step's last word
-        for (uint32_t base = 0; base < tlen; base += 64) {
-            const uint32_t w0 = base + 2 * lane, w1 = w0 + 1;
-            const uint32_t qa = w0 < limbs ? q[w0] : 0u, qb = w1 < limbs ? q[w1] : 0u;
-            const uint32_t qm = (w0 >= 1 && w0 - 1 < limbs) ? q[w0 - 1] : 0u;
-            const uint64_t a0 = uint64_t(ql) * qa, b0 = uint64_t(qh) * qm;  // word w0
-            const uint64_t a1 = uint64_t(ql) * qb, b1 = uint64_t(qh) * qa;  // word w1
-            const uint64_t hi0 = (a0 >> 32) + (b0 >> 32), hi1 = (a1 >> 32) + (b1 >> 32);
-            uint64_t hi_below = (uint64_t(__shfl_up_sync(kFull, uint32_t(hi1 >> 32), 1)) << 32) |
-                                __shfl_up_sync(kFull, uint32_t(hi1), 1);
-            if (lane == 0) hi_below = carry_hi;
-            carry_hi = (uint64_t(__shfl_sync(kFull, uint32_t(hi1 >> 32), 31)) << 32) | __shfl_sync(kFull, uint32_t(hi1), 31);
-            const uint64_t e0 = (a0 & 0xffffffffull) + (b0 & 0xffffffffull) + hi_below;
-            const uint64_t e1 = (a1 & 0xffffffffull) + (b1 & 0xffffffffull) + hi0;
-            const int64_t z0 = int64_t(w0 < tlen ? v[w0] : 0u) - int64_t(e0);
-            const int64_t z1 = int64_t(w1 < tlen ? v[w1] : 0u) - int64_t(e1);
-            const int32_t c0 = int32_t(z0 >> 32), c1 = int32_t(z1 >> 32);
-            int32_t c_below = __shfl_up_sync(kFull, c1, 1);
-            if (lane == 0) c_below = carry_c;
-            carry_c = __shfl_sync(kFull, c1, 31);
-            const int64_t sw0 = int64_t(uint32_t(z0)) + c_below, sw1 = int64_t(uint32_t(z1)) + c0;
-            const bool generate = sw1 < 0 || (sw1 == 0 && sw0 < 0);
-            const uint32_t borrow = chain_carry(generate, !generate && sw1 == 0 && sw0 == 0, chain);
-            const int64_t t0 = sw0 - borrow;
-            if (w0 < tlen) v[w0] = uint32_t(t0);
-            if (w1 < tlen) v[w1] = uint32_t(sw1 - (t0 < 0 ? 1 : 0));
+        if (corrections == 3) return false;
+        uint32_t borrow = 0;
+        for (uint32_t w = 0; w < limbs; ++w) {
+            const uint64_t t = uint64_t(row[w]) - q[w] - borrow;
+            row[w] = uint32_t(t);
+            borrow = uint32_t(t >> 63);
         }
-        __syncwarp();
-        // 5. at most three subtractions of q remain
-        int corrections = 0;
-        while (compare_q(v, tlen, q, limbs) >= 0) {
-            if (++corrections > 3) {
-                if (lane == 0) atomicOr(prm.error_flag, 1u);
-                break;
-            }
-            sub_words(v, tlen, [&](uint32_t w) { return w < limbs ? q[w] : 0u; });
-        }
-        // 6. canonical result
-        uint32_t* out = prm.out + size_t(i) * limbs;
-        for (uint32_t w = lane; w < limbs; w += 32) out[w] = v[w];
-        __syncwarp();
+        over -= borrow;
     }
 }
 
+// Running state of one row's pass.
+struct RowState {
+    int64_t carry;   // signed carry into the next word
+    uint64_t below;  // hi(ql q[w-1]) + qh q[w-1], subtracted at word w
+};
+
+// Word w of T' - quotient q: d + K R - lo(ql q) - below + carry. d < 2^56, K R < 2^46 and
+// below < 2^49, so the sum stays within int64.
+__device__ __forceinline__ uint32_t row_word(RowState& st, const RowQuotient& f, uint64_t d, uint32_t r, uint32_t q) {
+    const uint64_t a = uint64_t(f.low) * q;
+    const int64_t y = int64_t(d + uint64_t(f.k) * r) - int64_t(uint32_t(a)) - int64_t(st.below);
+    st.below = (a >> 32) + uint64_t(f.high) * q;
+    const int64_t z = y + st.carry;
+    st.carry = z >> 32;
+    return uint32_t(z);
+}
+
+template <uint32_t kChunk>
+__global__ void reduce_kernel(ReduceParams prm) {
+    using Slot = ReduceSlot<kChunk>;
+    constexpr uint32_t kPitch = Slot::kPitch;
+    extern __shared__ __align__(16) uint8_t reduce_smem[];
+    const uint32_t warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    uint8_t* slots = reduce_smem + warp * (kReduceSlots * Slot::kBytes);
+    const uint32_t slots_addr = uint32_t(__cvta_generic_to_shared(slots));
+    const uint32_t row0 = (blockIdx.x * (blockDim.x / 32) + warp) * 32;
+    if (row0 >= prm.n) return;  // warp-uniform
+    const uint32_t limbs = prm.limbs, tlen = limbs + 2, rows = min(32u, prm.n - row0);
+    const uint32_t chunks = (tlen + kChunk - 1) / kChunk;
+    const uint64_t* d0 = prm.dots + size_t(row0) * prm.dots_stride;
+
+    // chunk c of the warp's rows, and of q and R, into slot c % kReduceSlots
+    auto fetch = [&](uint32_t c) {
+        if (c < chunks) {
+            constexpr uint32_t kLanes = kChunk / 2;  // per row, 16 bytes each
+            const uint32_t slot = slots_addr + (c % kReduceSlots) * Slot::kBytes;
+            const uint32_t w = c * kChunk + 2 * (lane % kLanes);
+            if (w < prm.dots_stride) {
+                const uint32_t to = slot + (lane % kLanes) * 16;
+                const uint64_t* from = d0 + w;
+#pragma unroll 8
+                for (uint32_t i = 0; i < kLanes; ++i) {
+                    const uint32_t r = i * (32 / kLanes) + lane / kLanes;
+                    if (r < rows) cp_async_16(to + r * kPitch, from + size_t(r) * prm.dots_stride);
+                }
+            }
+            if (lane < kChunk / 2) {  // q, then R: kChunk / 4 pieces of 16 bytes each
+                const uint32_t piece = lane % (kChunk / 4);
+                cp_async_16(slot + 32 * kPitch + lane * 16,
+                            (lane < kChunk / 4 ? prm.q : prm.minus_p) + c * kChunk + piece * 4);
+            }
+        }
+        cp_async_commit();
+    };
+    for (uint32_t c = 0; c < kReduceSlots; ++c) fetch(c);
+
+    const RowQuotient f = row_quotient(d0 + size_t(min(lane, rows - 1)) * prm.dots_stride, prm);
+    RowState st{0, 0};
+    const uint32_t q_words = prm.q_words;  // significant words of q
+    uint32_t over = 0, top1 = 0, top0 = 0;  // words at and above q_words (or-ed), and the two below
+    for (uint32_t c = 0; c < chunks; ++c) {
+        cp_async_wait<kReduceSlots - 1>();
+        __syncwarp();
+        uint8_t* slot = slots + (c % kReduceSlots) * Slot::kBytes;
+        uint8_t* own = slot + lane * kPitch;
+        const uint4* q4 = reinterpret_cast<const uint4*>(slot + 32 * kPitch);  // the same for every lane
+        const uint4* r4 = q4 + kChunk / 4;
+        const uint32_t base = c * kChunk;
+#pragma unroll 1
+        for (uint32_t part = 0; part < kChunk; part += 16) {  // 16 words at a time through registers
+            if (base + part >= tlen) break;
+            ulonglong2 d[8];
+            uint4 q[4], r[4];
+#pragma unroll
+            for (uint32_t g = 0; g < 4; ++g) {
+                q[g] = q4[part / 4 + g];
+                r[g] = r4[part / 4 + g];
+                d[2 * g] = *reinterpret_cast<const ulonglong2*>(own + part * 8 + g * 32);
+                d[2 * g + 1] = *reinterpret_cast<const ulonglong2*>(own + part * 8 + g * 32 + 16);
+            }
+            if (base + part + 16 > tlen) {  // the row's end: words from L+2 up are not part of T
+#pragma unroll
+                for (uint32_t g = 0; g < 8; ++g) {
+                    if (base + part + 2 * g >= tlen) d[g].x = 0;
+                    if (base + part + 2 * g + 1 >= tlen) d[g].y = 0;
+                }
+            }
+            uint32_t o[16];
+#pragma unroll
+            for (uint32_t g = 0; g < 4; ++g) {
+                o[4 * g] = row_word(st, f, d[2 * g].x, r[g].x, q[g].x);
+                o[4 * g + 1] = row_word(st, f, d[2 * g].y, r[g].y, q[g].y);
+                o[4 * g + 2] = row_word(st, f, d[2 * g + 1].x, r[g].z, q[g].z);
+                o[4 * g + 3] = row_word(st, f, d[2 * g + 1].y, r[g].w, q[g].w);
+            }
+#pragma unroll
+            for (uint32_t g = 0; g < 4; ++g)  // over words that this thread has already read
+                *reinterpret_cast<uint4*>(own + part * 4 + g * 16) =
+                    make_uint4(o[4 * g], o[4 * g + 1], o[4 * g + 2], o[4 * g + 3]);
+            if (base + part + 16 + 2 > q_words) {  // some of the top words
+#pragma unroll
+                for (uint32_t i = 0; i < 16; ++i) {
+                    const uint32_t w = base + part + i;
+                    if (w + 2 == q_words) top0 = o[i];
+                    if (w + 1 == q_words) top1 = o[i];
+                    if (w >= q_words) over |= o[i];
+                }
+            }
+        }
+        __syncwarp();
+        if constexpr (kChunk == 16) {
+            // two rows per instruction (r and r + 4: their slots' banks do not meet), 64 bytes each
+            if (base + lane % 16 < limbs) {
+                uint32_t* out = prm.out + size_t(row0) * limbs + base + lane % 16;
+#pragma unroll
+                for (uint32_t i = 0; i < 16; ++i) {
+                    const uint32_t r = (i / 4) * 8 + i % 4 + (lane / 16) * 4;
+                    if (r < rows)
+                        out[size_t(r) * limbs] = reinterpret_cast<const uint32_t*>(slot + r * kPitch)[lane % 16];
+                }
+            }
+        } else {
+#pragma unroll
+            for (uint32_t part = 0; part < kChunk; part += 32) {
+                if (base + part + lane >= limbs) continue;
+                uint32_t* out = prm.out + size_t(row0) * limbs + base + part + lane;
+#pragma unroll 8
+                for (uint32_t r = 0; r < rows; ++r)
+                    out[size_t(r) * limbs] = reinterpret_cast<const uint32_t*>(slot + r * kPitch)[part + lane];
+            }
+        }
+        __syncwarp();
+        fetch(c + kReduceSlots);
+    }
+    // a result whose top two words are below q's is canonical; the rest compare whole rows
+    const uint64_t top = (uint64_t(top1) << 32) | top0, q_top = (uint64_t(prm.q[q_words - 1]) << 32) |
+                                                                (q_words >= 2 ? prm.q[q_words - 2] : 0u);
+    if (lane < rows && (over != 0 || top >= q_top)) {
+        uint32_t* row = prm.out + size_t(row0 + lane) * limbs;
+        if (!correct_row(row, q_words < limbs ? 0u : over, prm.q, limbs)) atomicOr(prm.error_flag, 1u);
+    }
+}
 
 uint32_t log2_u32(uint32_t x) { return x ? 31 - __builtin_clz(x) : 0; }
 
@@ -880,17 +920,24 @@ void launch_transpose(const uint32_t* residues, uint32_t* crt_in, uint32_t r, ui
                                                j_count);
 }
 
-void launch_reduce(const ReduceParams& params, cudaStream_t stream) {
-    const uint32_t stride = (params.words + 1 + 31) / 32 * 32;
-    // up to 8 warps (coefficients) per block, each with `stride` words of shared memory
-    constexpr size_t kSmemBudget = 200 * 1024;
-    uint32_t warps = uint32_t(std::min<size_t>(8, std::max<size_t>(1, kSmemBudget / (stride * sizeof(uint32_t)))));
-    const size_t smem = size_t(warps) * stride * sizeof(uint32_t);
+template <uint32_t kChunk>
+static void launch_reduce_chunks(const ReduceParams& params, uint32_t warps, cudaStream_t stream) {
+    const size_t smem = size_t(warps) * kReduceSlots * ReduceSlot<kChunk>::kBytes;
     if (smem > 48 * 1024)  // per device; cheap enough to repeat
-        cudaFuncSetAttribute(reduce_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemBudget));
-    uint32_t blocks = (params.n + warps - 1) / warps;
-    if (blocks > 148u * 8) blocks = 148u * 8;
-    reduce_kernel<<<blocks, warps * 32, smem, stream>>>(params, stride);
+        cudaFuncSetAttribute(reduce_kernel<kChunk>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    const uint32_t groups = (params.n + 31) / 32;  // of 32 rows, a warp each
+    reduce_kernel<kChunk><<<(groups + warps - 1) / warps, warps * 32, smem, stream>>>(params);
+}
+
+void launch_reduce(const ReduceParams& params, cudaStream_t stream) {
+    // Chunks of 64 words (512-byte runs per row) read DRAM better than chunks of 16 (128-byte runs
+    // of rows 14 KB apart): 362 against 432 us at N = 65536, L = 1747, 22.5 against 30.4 at N = 16384,
+    // L = 301. A row of up to 64 words is better read in four steps, with more warps per SM: 20.5
+    // against 24.6 us at N = 65536, L = 55. (us of the stage between events, about 5 of them launch.)
+    if (params.limbs + 2 <= 64)
+        launch_reduce_chunks<16>(params, params.n > 32 * 148 * 2 ? 2 : 1, stream);
+    else
+        launch_reduce_chunks<64>(params, 1, stream);
 }
 
 }  // namespace negacyclic

@@ -112,13 +112,16 @@ void launch_transpose(const uint32_t* residues, uint32_t* crt_in, uint32_t r, ui
 struct ReduceParams {
     const uint64_t* dots;     // [n][dots_stride], words used
     uint32_t* out;            // [n][limbs]
-    const uint32_t* q;        // [limbs]
-    const uint32_t* minus_p;  // [limbs]  (-P) mod q
-    uint32_t n, limbs, words, dots_stride;
+    const uint32_t* q;        // [limbs], then zeros up to reduce_table_words(limbs)
+    const uint32_t* minus_p;  // [limbs]  (-P) mod q, then zeros likewise
+    uint32_t n, limbs, dots_stride;
+    uint32_t q_words;         // significant words of q
     int32_t top_shift;
     uint64_t mu_low;
     uint32_t* error_flag;     // set nonzero if a coefficient needed more corrections than proven
 };
+// Words the tables of launch_reduce hold: whole chunks of 64 covering L + 2 words.
+constexpr uint32_t reduce_table_words(uint32_t limbs) { return (limbs + 2 + 63) / 64 * 64; }
 void launch_reduce(const ReduceParams& params, cudaStream_t stream);
 
 }  // namespace negacyclic

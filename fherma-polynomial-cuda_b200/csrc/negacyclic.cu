@@ -104,7 +104,7 @@ void enqueue_output(negacyclic_plan& s, uint32_t first, uint32_t count, uint32_t
     reduce.minus_p = s.minus_p;
     reduce.n = count;
     reduce.limbs = h.limbs;
-    reduce.words = h.words;
+    reduce.q_words = (h.q_bits + 31) / 32;
     reduce.top_shift = h.top_shift;
     reduce.mu_low = h.mu_low;
     reduce.error_flag = s.status;
@@ -302,8 +302,9 @@ int negacyclic_init(uint32_t n, uint32_t w, uint32_t limbs, const uint32_t* q, c
         device_alloc(s.zeta, size_t(s.r) * h.n_sub, tables);
         device_alloc(s.convert_weights, size_t(4) * s.padded_r * s.k_convert, tables);
         device_alloc(s.crt_weights, size_t(s.crt_columns) * s.k_crt, tables);
-        device_alloc(s.q, limbs, tables);
-        device_alloc(s.minus_p, limbs, tables);
+        const uint32_t table_words = reduce_table_words(limbs);
+        device_alloc(s.q, table_words, tables);
+        device_alloc(s.minus_p, table_words, tables);
         device_alloc(s.own_status, 64, tables);
         s.status = s.own_status;
         device_alloc(s.crt_words, size_t(s.r) * h.words, work);  // freed once the CRT weights are built
@@ -323,6 +324,8 @@ int negacyclic_init(uint32_t n, uint32_t w, uint32_t limbs, const uint32_t* q, c
         }
         cudaStream_t st = s.stream;
         check(cudaMemcpyAsync(s.primes, primes.data(), s.r * sizeof(DevicePrime), cudaMemcpyHostToDevice, st), "upload");
+        check(cudaMemsetAsync(s.q, 0, table_words * 4, st), "memset");
+        check(cudaMemsetAsync(s.minus_p, 0, table_words * 4, st), "memset");
         check(cudaMemcpyAsync(s.q, h.q.data(), limbs * 4, cudaMemcpyHostToDevice, st), "upload q");
         check(cudaMemcpyAsync(s.minus_p, h.minus_p_mod_q.data(), limbs * 4, cudaMemcpyHostToDevice, st), "upload");
         check(cudaMemsetAsync(s.own_status, 0, 64 * sizeof(uint32_t), st), "memset");

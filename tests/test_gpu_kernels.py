@@ -1,0 +1,49 @@
+"""Kernel paths at the sizes where they can go wrong, against the oracle (tolerance 0)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def torch():
+    import torch as t
+    assert t.cuda.is_available(), "GPU tests need a CUDA device"
+    return t
+
+
+def device_product(fpc, torch, q, a, b, **options):
+    """One product through the device entry point, with the plan's status word checked."""
+    n, limbs = a.shape
+    with fpc.Plan(n, 32 * limbs, limbs, q, **options) as plan:
+        da, db = (torch.from_numpy(x.view(np.int32)).cuda() for x in (a, b))
+        dc = torch.full_like(da, -1)
+        plan.run_device(da.data_ptr(), db.data_ptr(), dc.data_ptr(), torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+        assert plan.status() == 0
+        return dc.cpu().numpy().view(np.uint32)
+
+
+# rows around the chunks of 16 and 64 words that the reduction reads, with its switch between them
+# (L + 2 = 64), and fewer rows than a warp has lanes
+@pytest.mark.parametrize("limbs", [1, 2, 3, 13, 14, 15, 30, 31, 46, 61, 62, 63, 64, 125, 126, 127, 190])
+@pytest.mark.parametrize("n", [1, 16, 64])
+def test_reduction_row_ends(n, limbs, fpc, inputs, oracle, torch):
+    full = inputs.random_modulus(limbs, 7 * limbs + n)
+    narrow_top = full.copy()
+    narrow_top[-1] = 1                  # results whose top word equals q's are common
+    ones = np.full(limbs, 0xFFFFFFFF, np.uint32)   # q = 2^(32 L) - 1
+    moduli = [full, ones] + ([narrow_top] if limbs > 1 else [])
+    if limbs > 2:
+        short = full.copy()
+        short[limbs // 2:] = 0          # q shorter than its limbs
+        short[limbs // 2 - 1] |= 1
+        moduli.append(short)
+    for q in moduli:
+        rng = np.random.Generator(np.random.PCG64(limbs))
+        words = np.flatnonzero(q)[-1] + 1
+        pairs = [tuple(np.pad(inputs.random_operand(rng, n, q[:words]), ((0, 0), (0, limbs - words)))
+                       for _ in range(2))]
+        pairs += [(inputs.edge_operand(n, q, x), inputs.edge_operand(n, q, y)) for x, y in inputs.EDGE_PAIRS[1:]]
+        for a, b in pairs:
+            assert np.array_equal(device_product(fpc, torch, q, a, b), oracle.kronecker(q, a, b))
