@@ -13,7 +13,7 @@
 // for K <= 33024 (checked by the plan), so s32 accumulation is exact.
 //
 // Persistent (one CTA per SM) and warp-specialised: warp 0 = TMA producer,
-// warp 1 = MMA issuer and TMEM owner (two 256-column accumulators), warps 2-5 =
+// warp 1 = MMA issuer and TMEM owner (two 256-column accumulators), warps 2-9 =
 // epilogue, so the epilogue of one tile overlaps the MMAs of the next. Every
 // mbarrier wait is bounded (TileShape::limit cycles of SM clock, ~2 s by
 // default) and also ends when another role raised the abort flag. On a timeout
@@ -37,7 +37,7 @@ constexpr uint32_t kATileBytes = kBlockM * kBlockK;                // 16 KB
 constexpr uint32_t kBTileBytes = kBlockN * kBlockK;                // 32 KB
 constexpr uint32_t kStageBytes = kATileBytes + kBTileBytes;
 constexpr uint32_t kAccColumns = 256;                            // one 128 x 256 s32 accumulator
-constexpr uint32_t kEpilogueWarps = 4;
+constexpr uint32_t kEpilogueWarps = 8;  // two per 32-row quarter of the tile, half of the columns each
 constexpr uint32_t kThreads = 64 + 32 * kEpilogueWarps;
 constexpr long long kDefaultLimitCycles = 4000000000ll;  // ~2 s at 1.9 GHz
 constexpr uint64_t kAbortDrainNs = 1000000;               // 1 ms: in-flight TMA loads land long before
@@ -217,45 +217,43 @@ __device__ __forceinline__ void epilogue_chunk(const Epilogue& epi, const uint32
         if (g0 + g < epi.words) out[g] = sum[g];
 }
 
-// One epilogue warp's share of an accumulator: 32 rows (one per lane) x 256 columns starting at
-// col0, read from TMEM at t_base in 32-column chunks.
+// One epilogue warp's share of an accumulator: 32 rows (one per lane) x 128 columns starting at
+// col0 (half a tile), read from TMEM at t_base in 32-column chunks.
 // Conversion: column group g = 4k..4k+3 holds the byte dots of prime k; the residue is
-// REDC(sum_d G_d 256^d). The tile's 64 primes are loaded once (lane l: groups l and l + 32)
-// and broadcast by shuffles, instead of one dependent table load per group.
+// REDC(sum_d G_d 256^d). The chunk's eight primes are loaded (the same address in every lane)
+// before its accumulators, so that one latency covers both.
+// What bounds it: with few K steps per tile the epilogue is the tile's longest part, and a warp by
+// itself leaves its scheduler idle four cycles out of five (2140 instructions in 10.5k cycles per
+// 256 x 256 tile with one warp per quarter). Two warps per quarter share the tile.
 __device__ __forceinline__ void epilogue_rows(const Epilogue& epi, uint32_t t_base, uint32_t col0, uint32_t columns,
-                                              bool row_ok, uint64_t out_row, uint32_t op, uint32_t column,
-                                              uint32_t lane) {
+                                              bool row_ok, uint64_t out_row, uint32_t op, uint32_t column) {
+    constexpr uint32_t kChunks = kBlockN / 32 / 2;
     if (epi.mode == kEpilogueConvert) {
-        const uint32_t g0 = col0 / 4;
-        uint32_t p_lo = 1, pinv_lo = 0, p_hi = 1, pinv_hi = 0;
-        if (g0 + lane < epi.r) {
-            p_lo = epi.primes[g0 + lane].p;
-            pinv_lo = epi.primes[g0 + lane].pinv;
-        }
-        if (g0 + 32 + lane < epi.r) {
-            p_hi = epi.primes[g0 + 32 + lane].p;
-            pinv_hi = epi.primes[g0 + 32 + lane].pinv;
-        }
-        uint32_t* out = epi.residues + size_t(op) * epi.r * epi.n + column;  // + k * N for prime k
-        for (uint32_t chunk = 0; chunk < kBlockN / 32; ++chunk) {
-            const uint32_t c_base = col0 + chunk * 32;
-            if (c_base >= columns) break;  // warp-uniform
+        const uint32_t k0 = col0 / 4;
+        uint32_t* out = epi.residues + (size_t(op) * epi.r + k0) * epi.n + column;  // + g * N for prime k0 + g
+#pragma unroll 1
+        for (uint32_t chunk = 0; chunk < kChunks; ++chunk) {
+            if (k0 + chunk * 8 >= epi.r) break;  // warp-uniform
+            uint2 prime[8];
+#pragma unroll
+            for (uint32_t g = 0; g < 8; ++g) {
+                const uint32_t k = min(k0 + chunk * 8 + g, epi.r - 1);
+                prime[g] = __ldg(reinterpret_cast<const uint2*>(&epi.primes[k].p));
+            }
             uint32_t v[32];
             tmem_load32(t_base + chunk * 32, v);
-            const uint32_t from_p = chunk < 4 ? p_lo : p_hi, from_pinv = chunk < 4 ? pinv_lo : pinv_hi;
 #pragma unroll
-            for (int g = 0; g < 8; ++g) {
-                const uint32_t source = (chunk & 3) * 8 + g, k = c_base / 4 + g;
-                const uint32_t p = __shfl_sync(0xffffffffu, from_p, source);
-                const uint32_t pinv = __shfl_sync(0xffffffffu, from_pinv, source);
+            for (uint32_t g = 0; g < 8; ++g) {
                 const uint64_t s = uint64_t(v[4 * g]) + (uint64_t(v[4 * g + 1]) << 8) +
                                    (uint64_t(v[4 * g + 2]) << 16) + (uint64_t(v[4 * g + 3]) << 24);
-                if (row_ok && k < epi.r) out[size_t(k) * epi.n] = redc(s, p, pinv);
+                if (row_ok && k0 + chunk * 8 + g < epi.r) *out = redc(s, prime[g].x, prime[g].y);
+                out += epi.n;
             }
         }
         return;
     }
-    for (uint32_t chunk = 0; chunk < kBlockN / 32; ++chunk) {
+#pragma unroll 1
+    for (uint32_t chunk = 0; chunk < kChunks; ++chunk) {
         const uint32_t c_base = col0 + chunk * 32;
         if (c_base >= columns) break;  // warp-uniform
         uint32_t v[32];
@@ -267,7 +265,7 @@ __device__ __forceinline__ void epilogue_rows(const Epilogue& epi, uint32_t t_ba
 // Persistent, warp-specialised GEMM: each CTA walks tiles blockIdx.x, +gridDim.x, ...
 //   warp 0 (one thread)  TMA producer over a kStages-deep shared-memory ring
 //   warp 1 (one thread)  MMA issuer; the whole warp allocates / frees 512 TMEM columns
-//   warps 2-5            epilogue; two 256-column accumulators alternate between tiles,
+//   warps 2-9            epilogue; two 256-column accumulators alternate between tiles,
 //                        so tile i's epilogue overlaps tile i+1's MMAs
 __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_constant__ CUtensorMap a_map,
                                                               const __grid_constant__ CUtensorMap b_map,
@@ -385,8 +383,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
             if (!mbar_wait(drain, 0, shape.limit)) record_error(shape.status, 8u);
         }
     } else {
-        // ---------------- epilogue: warp w reads TMEM lanes 32*(w%4).. (rows of the tile)
-        const uint32_t quarter = warp & 3;
+        // ---------------- epilogue: warp w reads TMEM lanes 32*(w%4).. (rows of the tile),
+        // columns 128*((w-2)/4)..
+        const uint32_t quarter = warp & 3, half = (warp - 2) >> 2;
         uint32_t local = 0;
         for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++local) {
             const uint32_t acc = local & 1, use = local >> 1;
@@ -413,8 +412,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
                 else
                     out_row = shape.rows.row(row);
             }
-            const uint32_t t_base = tmem + acc * kAccColumns + ((quarter * 32) << 16);
-            epilogue_rows(epi, t_base, col0, shape.columns, row_ok, out_row, op, column, lane);
+            const uint32_t t_base = tmem + acc * kAccColumns + half * (kBlockN / 2) + ((quarter * 32) << 16);
+            epilogue_rows(epi, t_base, col0 + half * (kBlockN / 2), shape.columns, row_ok, out_row, op, column);
             // every tcgen05.ld of this warp has completed (tmem_load32 waits): release the accumulator
             fence_before();
             __syncwarp();
@@ -442,7 +441,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
 //     which the leader arms with both CTAs' bytes;
 //   * the leader's single MMA thread commits to empty[s] / acc_full[a] in both
 //     CTAs at once (tcgen05.commit ... multicast::cluster, mask 0b11);
-//   * all eight epilogue warps of the pair release an accumulator on the
+//   * all sixteen epilogue warps of the pair release an accumulator on the
 //     leader's acc_empty[a] (cluster-scope arrive).
 constexpr uint32_t kPairStages = 7;  // 224 KB of ring: seven stages fit the 227 KB opt-in limit with the barriers
 constexpr uint32_t kPairBlockN = 256;                      // columns per pair tile
@@ -710,7 +709,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         }
     } else {
         // ---------------- epilogue: this CTA's 128 rows of each pair tile
-        const uint32_t quarter = warp & 3;
+        const uint32_t quarter = warp & 3, half = (warp - 2) >> 2;
         const uint32_t release = leader_address(&acc_empty[0]);
         for (uint32_t i = 0, local = 0;; ++i, ++local) {
             uint32_t tile = read_ring(i, false);
@@ -743,8 +742,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                 else
                     out_row = shape.rows.row(row);
             }
-            const uint32_t t_base = tmem + acc * kAccColumns + ((quarter * 32) << 16);
-            epilogue_rows(epi, t_base, col0, shape.columns, row_ok, out_row, op, column, lane);
+            const uint32_t t_base = tmem + acc * kAccColumns + half * (kBlockN / 2) + ((quarter * 32) << 16);
+            epilogue_rows(epi, t_base, col0 + half * (kBlockN / 2), shape.columns, row_ok, out_row, op, column);
             fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(release + acc * sizeof(uint64_t));
@@ -803,10 +802,6 @@ bool prepare_gemm_tensor(TensorGemmPlan& plan, const uint8_t* a, uint64_t a_pitc
     }
     if (reinterpret_cast<uintptr_t>(a) % 16 || reinterpret_cast<uintptr_t>(b) % 16) {
         why = "operands must be 16-byte aligned";
-        return false;
-    }
-    if (columns < kBlockN) {
-        why = "fewer than 256 output columns";
         return false;
     }
     uint32_t slab = m;
@@ -880,6 +875,7 @@ bool prepare_gemm_tensor(TensorGemmPlan& plan, const uint8_t* a, uint64_t a_pitc
     plan.sm_count = sms > 0 ? uint32_t(sms) : 148;
     // CTA pairs need 256-row slabs; NEGACYCLIC_GEMM_PAIRS=0 selects the single-CTA kernel
     const char* pairs_env = getenv("NEGACYCLIC_GEMM_PAIRS");
+    plan.narrow = columns < kBlockN;
     plan.pairs = !(pairs_env && pairs_env[0] == '0') && plan.sm_count >= 2 &&
                  (rows.mode == kRowsLinear || slab % 256 == 0);
     plan.ready = true;
@@ -896,8 +892,9 @@ bool gemm_tensor_accepts(const TensorGemmPlan& plan, const RowMap& rows, uint32_
 }
 
 void launch_gemm_tensor(const TensorGemmPlan& plan, const Epilogue& epilogue, cudaStream_t stream, const RowMap& rows,
-                        uint32_t m, bool allow_pairs, long long limit_cycles, uint32_t withheld) {
-    const bool pairs = allow_pairs && plan.pairs && (rows.mode == kRowsLinear || rows.span % 256 == 0);
+                        uint32_t m, bool allow_pairs, long long limit_cycles, uint32_t withheld,
+                        uint32_t pair_min_steps) {
+    const bool pairs = allow_pairs && plan.pairs && plan.k_tiles >= pair_min_steps && (rows.mode == kRowsLinear || rows.span % 256 == 0);
     const uint32_t rows_per_tile = pairs ? 256 : kBlockM;
     const uint32_t m_tiles = (m + rows_per_tile - 1) / rows_per_tile;
     // largest raster group whose A tiles fit comfortably in L2 (~48 MB)

@@ -22,6 +22,7 @@ struct TensorGemmPlan {
     uint32_t sm_count = 148;          // persistent grid size
     uint64_t a_tile_bytes = 0;        // bytes of one 128-row A tile (raster group sizing)
     bool pairs = false;               // 2-CTA (cta_group::2) 256x256 tiles
+    bool narrow = false;              // fewer columns than one tile: TMA fills the rest of B with zeros
     bool ready = false;
 };
 
@@ -40,9 +41,16 @@ void launch_gemm_tensor(const TensorGemmPlan& plan, const Epilogue& epilogue, cu
 // every pipeline wait (0 = the default, about 2 s of SM clock). withheld (diagnostics only): the
 // producer of the first CTA (pair) stops before this pipeline step, so that its consumer's wait
 // runs out; kNoWithheldStep in normal use.
+// K steps (of 128 bytes) from which the CTA-pair kernel is the faster one: it halves the B bytes each
+// SM reads, but a tile costs it a claim from the global counter and twice the tile. Conversion and
+// CRT stages, us, pairs against single CTAs: 2 steps 59 / 40 and 4 steps 28.5 / 20.5 (N=65536, L=55),
+// 10 steps 95.5 / 88 and 20 steps 54.7 / 50.6 (N=16384, L=301), 28 steps 1100 / 1115 and 57 steps
+// 547 / 573 (N=32768, L=868), 55 steps 8950 / 9580 (N=65536, L=1747).
+constexpr uint32_t kPairMinSteps = 24;
 constexpr uint32_t kNoWithheldStep = 0xffffffffu;
 void launch_gemm_tensor(const TensorGemmPlan& plan, const Epilogue& epilogue, cudaStream_t stream, const RowMap& rows,
-                        uint32_t m, bool allow_pairs, long long limit_cycles, uint32_t withheld);
+                        uint32_t m, bool allow_pairs, long long limit_cycles, uint32_t withheld,
+                        uint32_t pair_min_steps = kPairMinSteps);
 bool gemm_tensor_accepts(const TensorGemmPlan& plan, const RowMap& rows, uint32_t m);
 
 // Device word that records pipeline-wait timeouts of the tensor GEMM (0 = none).

@@ -10,7 +10,7 @@
 
 namespace negacyclic {
 
-struct DevicePrime {
+struct alignas(8) DevicePrime {  // (p, pinv) is loaded as one 8-byte word
     uint32_t p;
     uint32_t pinv;      // -p^-1 mod 2^32
     uint32_t finish;    // 2^96 N'^-1 (P/p)^-1 mod p

@@ -168,6 +168,8 @@ WorkLayout work_layout(const negacyclic_plan& s) {
     return w;
 }
 
+constexpr char kFewColumns[] = "fewer than 256 output columns";
+
 // Points the plan at a work space and re-encodes the GEMM tensor maps for it.
 // Returns an error message, or "" on success.
 std::string bind_work(negacyclic_plan& s, void* arena) {
@@ -191,6 +193,16 @@ std::string bind_work(negacyclic_plan& s, void* arena) {
                             RowMap::linear(0), h.n, s.crt_weights, s.crt_columns, s.k_crt, why_crt))
         s.crt_engine = NEGACYCLIC_GEMM_TENSOR;
     if (!s.gemm_pairs_allowed) s.convert_gemm.pairs = s.crt_gemm.pairs = false;
+    // Fewer columns than a tile: by name the tensor engines refuse them, by default they pay from 8192
+    // rows on (stages, us, SIMT / tensor: 37 / 12 for the CRT GEMM at N=32768, L=28; 10.0 / 10.4 and
+    // 8.3 / 8.7 for the two GEMMs at N=2048, L=13).
+    auto few_columns = [&](uint32_t& engine, const TensorGemmPlan& gemm, std::string& why) {
+        if (engine != NEGACYCLIC_GEMM_TENSOR || !gemm.narrow || (!s.gemm_tensor_required && gemm.m >= 8192)) return;
+        engine = NEGACYCLIC_GEMM_SIMT;
+        why = kFewColumns;
+    };
+    few_columns(s.convert_engine, s.convert_gemm, why_convert);
+    few_columns(s.crt_engine, s.crt_gemm, why_crt);
     if (s.gemm_tensor_required &&
         (s.convert_engine != NEGACYCLIC_GEMM_TENSOR || s.crt_engine != NEGACYCLIC_GEMM_TENSOR))
         return "tensor-core GEMM not available for this point: " + why_convert + (why_convert.empty() ? "" : "; ") +
@@ -823,9 +835,9 @@ int negacyclic_gemm_u8(const uint8_t* d_a, const uint8_t* d_b, int32_t* d_d, uin
         if (engine == NEGACYCLIC_GEMM_TENSOR || engine == NEGACYCLIC_GEMM_TENSOR_SINGLE) {
             TensorGemmPlan plan;
             std::string why;
-            if (!prepare_gemm_tensor(plan, d_a, k, rows, m, d_b, n, k, why))
+            if (!prepare_gemm_tensor(plan, d_a, k, rows, m, d_b, n, k, why) || (plan.narrow && !(why = kFewColumns).empty()))
                 return fail(NEGACYCLIC_EINVAL, "tensor GEMM unavailable: " + why);
-            launch_gemm_tensor(plan, raw, stream, rows, m, engine == NEGACYCLIC_GEMM_TENSOR, 0, kNoWithheldStep);
+            launch_gemm_tensor(plan, raw, stream, rows, m, engine == NEGACYCLIC_GEMM_TENSOR, 0, kNoWithheldStep, 0);
         } else {
             launch_gemm_simt(d_a, k, rows, m, d_b, n, k, raw, stream);
         }
@@ -852,7 +864,7 @@ int negacyclic_gemm_u8_withheld(const uint8_t* d_a, const uint8_t* d_b, int32_t*
         TensorGemmPlan plan;
         std::string why;
         const RowMap rows = RowMap::linear(0);
-        if (!prepare_gemm_tensor(plan, d_a, k, rows, m, d_b, n, k, why))
+        if (!prepare_gemm_tensor(plan, d_a, k, rows, m, d_b, n, k, why) || (plan.narrow && !(why = kFewColumns).empty()))
             return fail(NEGACYCLIC_EINVAL, "tensor GEMM unavailable: " + why);
         check(cudaMalloc(&status, sizeof(uint32_t)), "cudaMalloc");
         check(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking), "cudaStreamCreate");
@@ -866,7 +878,7 @@ int negacyclic_gemm_u8_withheld(const uint8_t* d_a, const uint8_t* d_b, int32_t*
         raw.status = status;
         check(cudaEventRecord(start, stream), "cudaEventRecord");
         launch_gemm_tensor(plan, raw, stream, rows, m, engine == NEGACYCLIC_GEMM_TENSOR, (long long)limit_cycles,
-                           withheld_step);
+                           withheld_step, 0);
         check(cudaGetLastError(), "gemm");
         check(cudaEventRecord(stop, stream), "cudaEventRecord");
         check(cudaStreamSynchronize(stream), "gemm");

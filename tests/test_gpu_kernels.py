@@ -47,3 +47,12 @@ def test_reduction_row_ends(n, limbs, fpc, inputs, oracle, torch):
         pairs += [(inputs.edge_operand(n, q, x), inputs.edge_operand(n, q, y)) for x, y in inputs.EDGE_PAIRS[1:]]
         for a, b in pairs:
             assert np.array_equal(device_product(fpc, torch, q, a, b), oracle.kronecker(q, a, b))
+
+
+# byte GEMMs of one partial column tile (from 8192 rows on they go to the tensor cores), of a few
+# tiles with a partial last one, and of K steps with zero-filled tails
+@pytest.mark.parametrize("n,limbs", [(4096, 1), (4096, 5), (8192, 1), (8192, 2), (8192, 27), (8192, 29), (8192, 47),
+                                     (8192, 60), (4096, 65)])
+def test_partial_column_tiles(n, limbs, fpc, inputs, oracle, torch):
+    q, a, b = inputs.instance(n, limbs, 900 + limbs, 0)
+    assert np.array_equal(device_product(fpc, torch, q, a, b), oracle.kronecker(q, a, b))
