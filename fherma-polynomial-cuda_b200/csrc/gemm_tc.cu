@@ -26,6 +26,7 @@
 #include <cstdlib>
 
 #include "gemm_tc.cuh"
+#include "launch.cuh"
 
 namespace negacyclic {
 
@@ -308,6 +309,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
     __syncthreads();
     fence_after();
     const uint32_t tmem = *tmem_slot;
+    chain_enter();
 
     if (warp == 0) {
         if (lane == 0) {
@@ -608,6 +610,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     cluster_sync();  // barriers and TMEM of both CTAs ready before any cross-CTA traffic
     fence_after();
     const uint32_t tmem = *tmem_slot;
+    chain_enter();
     const uint32_t ring_release = leader_address(&ring_empty[0]);  // + slot * 8
 
     // Reads ring slot i (every reader): the tile index, or `tiles` after a timeout or an abort.
@@ -892,9 +895,8 @@ bool gemm_tensor_accepts(const TensorGemmPlan& plan, const RowMap& rows, uint32_
 }
 
 void launch_gemm_tensor(const TensorGemmPlan& plan, const Epilogue& epilogue, cudaStream_t stream, const RowMap& rows,
-                        uint32_t m, bool allow_pairs, long long limit_cycles, uint32_t withheld,
-                        uint32_t pair_min_steps) {
-    const bool pairs = allow_pairs && plan.pairs && plan.k_tiles >= pair_min_steps && (rows.mode == kRowsLinear || rows.span % 256 == 0);
+                        uint32_t m, const TensorGemmOptions& options) {
+    const bool pairs = options.allow_pairs && plan.pairs && plan.k_tiles >= options.pair_min_steps && (rows.mode == kRowsLinear || rows.span % 256 == 0);
     const uint32_t rows_per_tile = pairs ? 256 : kBlockM;
     const uint32_t m_tiles = (m + rows_per_tile - 1) / rows_per_tile;
     // largest raster group whose A tiles fit comfortably in L2 (~48 MB)
@@ -903,26 +905,18 @@ void launch_gemm_tensor(const TensorGemmPlan& plan, const Epilogue& epilogue, cu
     TileShape shape{m,      plan.columns,       plan.k_tiles,
                     m_tiles, plan.n_tiles,      uint32_t(group),
                     rows,    plan.tile_counter, epilogue.status,
-                    limit_cycles > 0 ? limit_cycles : kDefaultLimitCycles, withheld};
+                    options.limit_cycles > 0 ? options.limit_cycles : kDefaultLimitCycles, options.withheld};
     const uint32_t tiles = m_tiles * plan.n_tiles;
     if (pairs) {
         const uint32_t max_pairs = plan.sm_count / 2;
         const uint32_t grid = 2 * (tiles < max_pairs ? tiles : max_pairs);
-        cudaMemsetAsync(plan.tile_counter, 0, sizeof(uint32_t), stream);
-        gemm_tc_pair_kernel<<<grid, kThreads, kPairSmemBytes, stream>>>(plan.a_map, plan.b_map_half, shape, epilogue);
+        if (!options.counter_cleared) cudaMemsetAsync(plan.tile_counter, 0, sizeof(uint32_t), stream);
+        launch_chained(gemm_tc_pair_kernel, grid, kThreads, kPairSmemBytes, stream, plan.a_map, plan.b_map_half, shape,
+                       epilogue);
         return;
     }
     const uint32_t grid = tiles < plan.sm_count ? tiles : plan.sm_count;
-    gemm_tc_kernel<<<grid, kThreads, kSmemBytes, stream>>>(plan.a_map, plan.b_map, shape, epilogue);
-}
-
-void launch_gemm_tensor(const TensorGemmPlan& plan, const Epilogue& epilogue, cudaStream_t stream, const RowMap& rows,
-                        uint32_t m) {
-    launch_gemm_tensor(plan, epilogue, stream, rows, m, true, 0, kNoWithheldStep);
-}
-
-void launch_gemm_tensor(const TensorGemmPlan& plan, const Epilogue& epilogue, cudaStream_t stream) {
-    launch_gemm_tensor(plan, epilogue, stream, plan.rows, plan.m);
+    launch_chained(gemm_tc_kernel, grid, kThreads, kSmemBytes, stream, plan.a_map, plan.b_map, shape, epilogue);
 }
 
 }  // namespace negacyclic

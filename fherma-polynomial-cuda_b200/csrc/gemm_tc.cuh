@@ -31,26 +31,27 @@ struct TensorGemmPlan {
 bool prepare_gemm_tensor(TensorGemmPlan& plan, const uint8_t* a, uint64_t a_pitch, RowMap rows, uint32_t m,
                          const uint8_t* b, uint32_t columns, uint32_t k_bytes, std::string& why);
 
-void launch_gemm_tensor(const TensorGemmPlan& plan, const Epilogue& epilogue, cudaStream_t stream);
-
-// A launch over part of the rows (a chunk of coefficients): `rows`/`m` describe the chunk
-// within the shape the plan was prepared for (see gemm_tensor_accepts).
-void launch_gemm_tensor(const TensorGemmPlan& plan, const Epilogue& epilogue, cudaStream_t stream, const RowMap& rows,
-                        uint32_t m);
-// allow_pairs = false forces the single-CTA kernel (diagnostics and tests). limit_cycles bounds
-// every pipeline wait (0 = the default, about 2 s of SM clock). withheld (diagnostics only): the
-// producer of the first CTA (pair) stops before this pipeline step, so that its consumer's wait
-// runs out; kNoWithheldStep in normal use.
+constexpr uint32_t kNoWithheldStep = 0xffffffffu;
 // K steps (of 128 bytes) from which the CTA-pair kernel is the faster one: it halves the B bytes each
 // SM reads, but a tile costs it a claim from the global counter and twice the tile. Conversion and
 // CRT stages, us, pairs against single CTAs: 2 steps 59 / 40 and 4 steps 28.5 / 20.5 (N=65536, L=55),
 // 10 steps 95.5 / 88 and 20 steps 54.7 / 50.6 (N=16384, L=301), 28 steps 1100 / 1115 and 57 steps
 // 547 / 573 (N=32768, L=868), 55 steps 8950 / 9580 (N=65536, L=1747).
 constexpr uint32_t kPairMinSteps = 24;
-constexpr uint32_t kNoWithheldStep = 0xffffffffu;
+struct TensorGemmOptions {
+    bool allow_pairs = true;      // false: the single-CTA kernel
+    uint32_t pair_min_steps = kPairMinSteps;  // CTA pairs from this many K steps on
+    bool counter_cleared = false; // an earlier kernel of the stream has zeroed plan.tile_counter
+    long long limit_cycles = 0;   // bound of every pipeline wait (0: about 2 s of SM clock)
+    // diagnostics only: the producer of the first CTA (pair) stops before this pipeline step, so that
+    // its consumer's wait runs out
+    uint32_t withheld = kNoWithheldStep;
+};
+
+// A launch over the plan's rows or part of them (a chunk of coefficients): `rows`/`m` describe the
+// chunk within the shape the plan was prepared for (see gemm_tensor_accepts).
 void launch_gemm_tensor(const TensorGemmPlan& plan, const Epilogue& epilogue, cudaStream_t stream, const RowMap& rows,
-                        uint32_t m, bool allow_pairs, long long limit_cycles, uint32_t withheld,
-                        uint32_t pair_min_steps = kPairMinSteps);
+                        uint32_t m, const TensorGemmOptions& options = {});
 bool gemm_tensor_accepts(const TensorGemmPlan& plan, const RowMap& rows, uint32_t m);
 
 // Device word that records pipeline-wait timeouts of the tensor GEMM (0 = none).

@@ -11,6 +11,8 @@
 //                                  zeta psi^(2 brv(m)+1) (evaluation point at output m)
 #include "kernels.cuh"
 
+#include "launch.cuh"
+
 #include <algorithm>
 #include <type_traits>
 
@@ -34,10 +36,13 @@ __device__ __forceinline__ void pad_row(const uint32_t* __restrict__ src, uint32
 }
 
 // [N][L] a and b -> [2][N][Lp] split-major: output row op*N + t*N' + j holds coefficient
-// s*j + t of operand op. One warp per output row.
+// s*j + t of operand op. One warp per output row. Also clears the GEMMs' tile counters, so that no
+// memset node stands in the product's chain.
 __global__ void pad_operands_kernel(const uint32_t* __restrict__ a, const uint32_t* __restrict__ b,
                                     uint32_t* __restrict__ out, uint32_t n, uint32_t limbs, uint32_t padded,
-                                    uint32_t log_split, uint32_t log_n_sub) {
+                                    uint32_t log_split, uint32_t log_n_sub, uint32_t* tile_counters) {
+    chain_enter();
+    if (blockIdx.x == 0 && threadIdx.x < kTileCounters) tile_counters[threadIdx.x] = 0;
     const uint32_t lane = threadIdx.x % 32, warps = gridDim.x * (blockDim.x / 32);
     const uint32_t n_sub_mask = (1u << log_n_sub) - 1;
     for (uint32_t w = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32; w < 2 * n; w += warps) {
@@ -54,6 +59,7 @@ __global__ void pad_operands_kernel(const uint32_t* __restrict__ a, const uint32
 __global__ void pad_rows_kernel(const uint32_t* __restrict__ staged, uint32_t* __restrict__ out, uint32_t n,
                                 uint32_t limbs, uint32_t padded, uint32_t log_split, uint32_t log_n_sub,
                                 uint32_t first, uint32_t count, uint32_t op_first, uint32_t op_count) {
+    chain_enter();
     const uint32_t lane = threadIdx.x % 32, warps = gridDim.x * (blockDim.x / 32);
     const uint32_t split_mask = (1u << log_split) - 1;
     for (uint32_t w = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32; w < op_count * count; w += warps) {
@@ -121,6 +127,7 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(const uint8_t* __restric
                                                         RowMap rows, uint32_t m_total,
                                                         const uint8_t* __restrict__ b, uint32_t columns,
                                                         uint32_t k_bytes, Epilogue epi) {
+    chain_enter();
     __shared__ uint32_t as[kTile][kTileK / 4 + 1];
     __shared__ uint32_t bs[kTile][kTileK / 4 + 1];
     const uint32_t tid = threadIdx.x, tr = tid / 16, tc = tid % 16;
@@ -192,6 +199,7 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(const uint8_t* __restric
 __global__ void __launch_bounds__(512) ntt_forward_kernel(uint32_t* residues, const DevicePrime* __restrict__ primes,
                                                           const uint2* __restrict__ fwd, uint32_t r, uint32_t n,
                                                           uint32_t n_sub, uint32_t t_first, uint32_t op_first) {
+    chain_enter();
     extern __shared__ uint32_t x[];
     const uint32_t t_index = t_first + blockIdx.x, k = blockIdx.y, op = op_first + blockIdx.z;
     const uint32_t p = primes[k].p;
@@ -216,6 +224,7 @@ __global__ void __launch_bounds__(512) ntt_forward_kernel(uint32_t* residues, co
 __global__ void __launch_bounds__(512) ntt_inverse_kernel(uint32_t* residues, const DevicePrime* __restrict__ primes,
                                                           const uint2* __restrict__ inv, uint32_t r, uint32_t n,
                                                           uint32_t n_sub, uint32_t v_first) {
+    chain_enter();
     extern __shared__ uint32_t x[];
     const uint32_t v_index = v_first + blockIdx.x, k = blockIdx.y;
     const DevicePrime f = primes[k];
@@ -422,6 +431,7 @@ template <uint32_t kLog>
 __global__ void __launch_bounds__(1u << (kLog - 4), (kLog >= 13 ? 2 : 4)) ntt_forward_blocked_kernel(
     uint32_t* residues, const DevicePrime* __restrict__ primes, const uint2* __restrict__ fwd, uint32_t r, uint32_t n,
     uint32_t t_first, uint32_t t_count, uint32_t op_first) {
+    chain_enter();
     extern __shared__ uint32_t xs[];
     constexpr uint32_t kN = 1u << kLog;
     const uint32_t local_op = blockIdx.x / t_count, op = op_first + local_op;
@@ -434,6 +444,7 @@ template <uint32_t kLog>
 __global__ void __launch_bounds__(1u << (kLog - 4), (kLog >= 13 ? 2 : 4)) ntt_inverse_blocked_kernel(
     uint32_t* residues, const DevicePrime* __restrict__ primes, const uint2* __restrict__ inv, uint32_t r, uint32_t n,
     uint32_t v_first, uint32_t v_count, uint32_t /*op_first: the inverse works on operand row 0 only*/) {
+    chain_enter();
     extern __shared__ uint32_t xs[];
     constexpr uint32_t kN = 1u << kLog;
     const uint32_t v_index = v_first + blockIdx.x, k = blockIdx.y;
@@ -448,6 +459,7 @@ __global__ void __launch_bounds__(1u << (kLog - 4), (kLog >= 13 ? 2 : 4)) ntt_in
 template <int S, int V>
 __global__ void pointwise_kernel(uint32_t* residues, const DevicePrime* __restrict__ primes,
                                  const uint2* __restrict__ zeta, uint32_t r, uint32_t n, uint32_t n_sub) {
+    chain_enter();
     using Word = std::conditional_t<V == 2, uint2, uint32_t>;
     const uint32_t k = blockIdx.y;
     const uint32_t m = (blockIdx.x * blockDim.x + threadIdx.x) * V;
@@ -512,6 +524,7 @@ __global__ void __launch_bounds__(256) transpose_kernel(const uint32_t* __restri
                                                         uint32_t* __restrict__ crt_in, uint32_t r, uint32_t padded_r,
                                                         uint32_t n, uint32_t log_split, uint32_t log_n_sub,
                                                         uint32_t j_first, uint32_t j_count) {
+    chain_enter();
     __shared__ uint32_t tile[kTransposeTile][kTransposeTile + 1];
     const uint32_t blocks_per_v = (j_count + kTransposeTile - 1) / kTransposeTile, v = blockIdx.x / blocks_per_v;
     const uint32_t j0 = j_first + (blockIdx.x - v * blocks_per_v) * kTransposeTile, k0 = blockIdx.y * kTransposeTile;
@@ -665,6 +678,7 @@ __device__ __forceinline__ uint32_t row_word(RowState& st, const RowQuotient& f,
 
 template <uint32_t kChunk>
 __global__ void reduce_kernel(ReduceParams prm) {
+    chain_enter();
     using Slot = ReduceSlot<kChunk>;
     constexpr uint32_t kPitch = Slot::kPitch;
     extern __shared__ __align__(16) uint8_t reduce_smem[];
@@ -794,10 +808,11 @@ uint32_t log2_u32(uint32_t x) { return x ? 31 - __builtin_clz(x) : 0; }
 }  // namespace
 
 void launch_pad_operands(const uint32_t* a, const uint32_t* b, uint32_t* out, uint32_t n, uint32_t limbs,
-                         uint32_t padded_limbs, uint32_t split, cudaStream_t stream) {
+                         uint32_t padded_limbs, uint32_t split, uint32_t* tile_counters, cudaStream_t stream) {
     const uint32_t log_split = log2_u32(split), log_n_sub = log2_u32(n) - log_split;
     const uint32_t blocks = std::min<uint32_t>((2 * n + 7) / 8, 148 * 16);  // 8 rows (warps) per block
-    pad_operands_kernel<<<blocks, 256, 0, stream>>>(a, b, out, n, limbs, padded_limbs, log_split, log_n_sub);
+    launch_chained(pad_operands_kernel, blocks, 256, 0, stream, a, b, out, n, limbs, padded_limbs, log_split, log_n_sub,
+                   tile_counters);
 }
 
 void launch_pad_rows(const uint32_t* staged, uint32_t* out, uint32_t n, uint32_t limbs, uint32_t padded_limbs,
@@ -805,7 +820,7 @@ void launch_pad_rows(const uint32_t* staged, uint32_t* out, uint32_t n, uint32_t
                      uint32_t op_count) {
     const uint32_t log_split = log2_u32(split), log_n_sub = log2_u32(n) - log_split;
     const uint32_t blocks = std::min<uint32_t>((op_count * count + 7) / 8, 148 * 16);
-    pad_rows_kernel<<<blocks, 256, 0, stream>>>(staged, out, n, limbs, padded_limbs, log_split, log_n_sub, first_row,
+    launch_chained(pad_rows_kernel, blocks, 256, 0, stream, staged, out, n, limbs, padded_limbs, log_split, log_n_sub, first_row,
                                                 count, op_first, op_count);
 }
 
@@ -830,7 +845,7 @@ void launch_crt_weights(const uint32_t* weights_words, uint32_t r, uint32_t padd
 void launch_gemm_simt(const uint8_t* a, uint64_t a_pitch, RowMap rows, uint32_t m, const uint8_t* b,
                       uint32_t columns, uint32_t k_bytes, const Epilogue& epilogue, cudaStream_t stream) {
     dim3 grid((m + kTile - 1) / kTile, (columns + kTile - 1) / kTile);
-    gemm_simt_kernel<<<grid, 256, 0, stream>>>(a, a_pitch, rows, m, b, columns, k_bytes, epilogue);
+    launch_chained(gemm_simt_kernel, grid, 256, 0, stream, a, a_pitch, rows, m, b, columns, k_bytes, epilogue);
 }
 
 static uint32_t ntt_threads(uint32_t n_sub) {
@@ -850,7 +865,7 @@ static void launch_blocked(uint32_t* residues, const DevicePrime* primes, const 
         configured = true;
     }
     dim3 grid(kForward ? op_count * count : count, r);
-    kernel<<<grid, kN / kPerThread, smem, stream>>>(residues, primes, table, r, n, first, count, op_first);
+    launch_chained(kernel, grid, kN / kPerThread, smem, stream, residues, primes, table, r, n, first, count, op_first);
 }
 
 template <bool kForward>
@@ -877,47 +892,50 @@ void launch_ntt_forward(uint32_t* residues, const DevicePrime* primes, const uin
     if (launch_blocked_any<true>(n_sub, residues, primes, fwd, r, n, t_first, t_count, stream, op_first, op_count))
         return;
     dim3 grid(t_count, r, op_count);
-    ntt_forward_kernel<<<grid, ntt_threads(n_sub), n_sub * sizeof(uint32_t), stream>>>(residues, primes, fwd, r, n,
-                                                                                          n_sub, t_first, op_first);
+    launch_chained(ntt_forward_kernel, grid, ntt_threads(n_sub), n_sub * sizeof(uint32_t), stream, residues, primes, fwd, r,
+                   n, n_sub, t_first, op_first);
 }
 
 void launch_ntt_inverse(uint32_t* residues, const DevicePrime* primes, const uint2* inv, uint32_t r, uint32_t n,
                         uint32_t n_sub, uint32_t v_first, uint32_t v_count, cudaStream_t stream) {
     if (launch_blocked_any<false>(n_sub, residues, primes, inv, r, n, v_first, v_count, stream)) return;
     dim3 grid(v_count, r);
-    ntt_inverse_kernel<<<grid, ntt_threads(n_sub), n_sub * sizeof(uint32_t), stream>>>(residues, primes, inv, r, n,
-                                                                                          n_sub, v_first);
+    launch_chained(ntt_inverse_kernel, grid, ntt_threads(n_sub), n_sub * sizeof(uint32_t), stream, residues, primes, inv, r,
+                   n, n_sub, v_first);
 }
 
 void launch_pointwise(uint32_t* residues, const DevicePrime* primes, const uint2* zeta, uint32_t r, uint32_t n,
                       uint32_t n_sub, uint32_t split, cudaStream_t stream) {
+#define NEGACYCLIC_POINTWISE(S, V) \
+    launch_chained(pointwise_kernel<S, V>, grid, 128, 0, stream, residues, primes, zeta, r, n, n_sub)
     if (n_sub % 2 == 0) {  // two evaluation points per thread
         dim3 grid((n_sub / 2 + 127) / 128, r);
         switch (split) {
-            case 1: pointwise_kernel<1, 2><<<grid, 128, 0, stream>>>(residues, primes, zeta, r, n, n_sub); break;
-            case 2: pointwise_kernel<2, 2><<<grid, 128, 0, stream>>>(residues, primes, zeta, r, n, n_sub); break;
-            case 4: pointwise_kernel<4, 2><<<grid, 128, 0, stream>>>(residues, primes, zeta, r, n, n_sub); break;
-            case 8: pointwise_kernel<8, 2><<<grid, 128, 0, stream>>>(residues, primes, zeta, r, n, n_sub); break;
-            default: pointwise_kernel<16, 2><<<grid, 128, 0, stream>>>(residues, primes, zeta, r, n, n_sub); break;
+            case 1: NEGACYCLIC_POINTWISE(1, 2); break;
+            case 2: NEGACYCLIC_POINTWISE(2, 2); break;
+            case 4: NEGACYCLIC_POINTWISE(4, 2); break;
+            case 8: NEGACYCLIC_POINTWISE(8, 2); break;
+            default: NEGACYCLIC_POINTWISE(16, 2); break;
         }
         return;
     }
     dim3 grid((n_sub + 127) / 128, r);
     switch (split) {
-        case 1: pointwise_kernel<1, 1><<<grid, 128, 0, stream>>>(residues, primes, zeta, r, n, n_sub); break;
-        case 2: pointwise_kernel<2, 1><<<grid, 128, 0, stream>>>(residues, primes, zeta, r, n, n_sub); break;
-        case 4: pointwise_kernel<4, 1><<<grid, 128, 0, stream>>>(residues, primes, zeta, r, n, n_sub); break;
-        case 8: pointwise_kernel<8, 1><<<grid, 128, 0, stream>>>(residues, primes, zeta, r, n, n_sub); break;
-        default: pointwise_kernel<16, 1><<<grid, 128, 0, stream>>>(residues, primes, zeta, r, n, n_sub); break;
+        case 1: NEGACYCLIC_POINTWISE(1, 1); break;
+        case 2: NEGACYCLIC_POINTWISE(2, 1); break;
+        case 4: NEGACYCLIC_POINTWISE(4, 1); break;
+        case 8: NEGACYCLIC_POINTWISE(8, 1); break;
+        default: NEGACYCLIC_POINTWISE(16, 1); break;
     }
+#undef NEGACYCLIC_POINTWISE
 }
 
 void launch_transpose(const uint32_t* residues, uint32_t* crt_in, uint32_t r, uint32_t padded_r, uint32_t n,
                       uint32_t split, uint32_t j_first, uint32_t j_count, cudaStream_t stream) {
     const uint32_t log_split = log2_u32(split), log_n_sub = log2_u32(n) - log_split;
     dim3 grid(split * ((j_count + kTransposeTile - 1) / kTransposeTile), (padded_r + kTransposeTile - 1) / kTransposeTile);
-    transpose_kernel<<<grid, 256, 0, stream>>>(residues, crt_in, r, padded_r, n, log_split, log_n_sub, j_first,
-                                               j_count);
+    launch_chained(transpose_kernel, grid, 256, 0, stream, residues, crt_in, r, padded_r, n, log_split, log_n_sub, j_first,
+                   j_count);
 }
 
 template <uint32_t kChunk>
@@ -926,7 +944,7 @@ static void launch_reduce_chunks(const ReduceParams& params, uint32_t warps, cud
     if (smem > 48 * 1024)  // per device; cheap enough to repeat
         cudaFuncSetAttribute(reduce_kernel<kChunk>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
     const uint32_t groups = (params.n + 31) / 32;  // of 32 rows, a warp each
-    reduce_kernel<kChunk><<<(groups + warps - 1) / warps, warps * 32, smem, stream>>>(params);
+    launch_chained(reduce_kernel<kChunk>, (groups + warps - 1) / warps, warps * 32, smem, stream, params);
 }
 
 void launch_reduce(const ReduceParams& params, cudaStream_t stream) {

@@ -77,9 +77,11 @@ struct Epilogue {
 };
 
 // a, b: [N][L] -> out: [2][N][Lp], rows split-major (coefficient s*j + t at row op*N + t*N' + j),
-// limbs padded with zeros to Lp
+// limbs padded with zeros to Lp; also zeroes tile_counters[kTileCounters]
+constexpr uint32_t kTileCounters = 2;  // of a work space: the conversion's, the CRT GEMM's
 void launch_pad_operands(const uint32_t* a, const uint32_t* b, uint32_t* out, uint32_t n,
-                         uint32_t limbs, uint32_t padded_limbs, uint32_t split, cudaStream_t stream);
+                         uint32_t limbs, uint32_t padded_limbs, uint32_t split, uint32_t* tile_counters,
+                         cudaStream_t stream);
 // rows [first_row, first_row + count) of operands [op_first, op_first + op_count) (operand stride N
 // rows) from an unpadded [2][N][L] array into the padded split-major [2][N][Lp] layout: staged in
 // coefficient order (split = s, rows are permuted) or already split-major (split = 1)

@@ -1,0 +1,42 @@
+// Chained launches: a product's kernels follow one another on a stream with programmatic dependent
+// launch, so that a kernel's blocks are placed, and its prologue runs, while the kernel before it
+// finishes.
+//
+// Rules that keep this equal to plain stream order:
+//  * every kernel of the chain calls chain_wait() in every thread before it touches memory that a
+//    kernel writes (chain_wait returns once the kernel before it has completed and its writes are
+//    visible). Since that kernel waited likewise, everything earlier on the stream has completed too;
+//  * chain_release(), which lets the next kernel's blocks be placed, comes after chain_wait(), so at
+//    most two kernels of a stream are resident, and two CTA-pair GEMMs never are: another kernel
+//    stands between them.
+#pragma once
+#include <cuda_runtime.h>
+
+namespace negacyclic {
+
+#ifdef __CUDACC__
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void chain_enter() {
+    chain_wait();
+    chain_release();
+}
+
+template <class... Params, class... Args>
+void launch_chained(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                    Args&&... args) {
+    cudaLaunchAttribute attribute{};
+    attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attribute.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t config{};
+    config.gridDim = grid;
+    config.blockDim = block;
+    config.dynamicSmemBytes = smem;
+    config.stream = stream;
+    config.attrs = &attribute;
+    config.numAttrs = 1;
+    cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);  // errors: cudaGetLastError()
+}
+#endif
+
+}  // namespace negacyclic

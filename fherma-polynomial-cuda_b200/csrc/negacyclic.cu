@@ -58,10 +58,17 @@ namespace negacyclic::detail {
 
 constexpr uint32_t kStages = 7;  // convert, forward, pointwise, inverse, transpose, crt, reduce
 
+TensorGemmOptions product_gemm(bool counter_cleared) {
+    TensorGemmOptions options;
+    options.counter_cleared = counter_cleared;
+    return options;
+}
+
 // conversion GEMM over the coefficients s*j + t, t in [t_first, t_first + t_count),
 // j in [first_j, first_j + span), of operands [op_first, op_first + op_count)
 void enqueue_convert(negacyclic_plan& s, uint32_t t_first, uint32_t t_count, uint32_t first_j, uint32_t span,
-                     cudaStream_t stream, uint32_t op_first = 0, uint32_t op_count = 2) {
+                     cudaStream_t stream, uint32_t op_first = 0, uint32_t op_count = 2,
+                     bool counter_cleared = false) {
     const HostPlan& h = s.host;
     Epilogue convert{};
     convert.mode = kEpilogueConvert;
@@ -73,7 +80,7 @@ void enqueue_convert(negacyclic_plan& s, uint32_t t_first, uint32_t t_count, uin
     const RowMap rows = RowMap::split_rows(h.n, h.n_sub, h.split, first_j, span, t_first, t_count, op_first);
     const uint32_t m = op_count * t_count * span;
     if (s.convert_engine == NEGACYCLIC_GEMM_TENSOR && gemm_tensor_accepts(s.convert_gemm, rows, m))
-        launch_gemm_tensor(s.convert_gemm, convert, stream, rows, m);
+        launch_gemm_tensor(s.convert_gemm, convert, stream, rows, m, product_gemm(counter_cleared));
     else
         launch_gemm_simt(reinterpret_cast<const uint8_t*>(s.operands), uint64_t(s.padded_limbs) * 4, rows, m,
                          s.convert_weights, 4 * s.padded_r, s.k_convert, convert, stream);
@@ -81,7 +88,7 @@ void enqueue_convert(negacyclic_plan& s, uint32_t t_first, uint32_t t_count, uin
 
 // CRT GEMM and reduction of coefficients [first, first + count) into d_c (rows indexed from 0 = coefficient 0)
 void enqueue_output(negacyclic_plan& s, uint32_t first, uint32_t count, uint32_t* d_c, cudaStream_t stream,
-                    cudaEvent_t between = nullptr) {
+                    cudaEvent_t between = nullptr, bool counter_cleared = false) {
     const HostPlan& h = s.host;
     Epilogue crt{};
     crt.mode = kEpilogueCrt;
@@ -91,7 +98,7 @@ void enqueue_output(negacyclic_plan& s, uint32_t first, uint32_t count, uint32_t
     crt.status = s.status;
     const RowMap rows = RowMap::linear(first);
     if (s.crt_engine == NEGACYCLIC_GEMM_TENSOR && gemm_tensor_accepts(s.crt_gemm, rows, count))
-        launch_gemm_tensor(s.crt_gemm, crt, stream, rows, count);
+        launch_gemm_tensor(s.crt_gemm, crt, stream, rows, count, product_gemm(counter_cleared));
     else
         launch_gemm_simt(reinterpret_cast<const uint8_t*>(s.crt_in), uint64_t(s.padded_r) * 4, rows, count,
                          s.crt_weights, s.crt_columns, s.k_crt, crt, stream);
@@ -134,17 +141,17 @@ void enqueue_middle(negacyclic_plan& s, cudaStream_t stream, cudaEvent_t* marks)
 // `marks` (optional, kStages events) are recorded after each stage.
 void enqueue_product(negacyclic_plan& s, uint32_t* d_c, cudaStream_t stream, cudaEvent_t* marks = nullptr) {
     const HostPlan& h = s.host;
-    enqueue_convert(s, 0, h.split, 0, h.n_sub, stream);
+    enqueue_convert(s, 0, h.split, 0, h.n_sub, stream, 0, 2, true);  // the pad kernel cleared the counters
     if (marks) check(cudaEventRecord(marks[0], stream), "cudaEventRecord");
     enqueue_middle(s, stream, marks ? marks + 1 : nullptr);
-    enqueue_output(s, 0, h.n, d_c, stream, marks ? marks[5] : nullptr);
+    enqueue_output(s, 0, h.n, d_c, stream, marks ? marks[5] : nullptr, true);
     if (marks) check(cudaEventRecord(marks[6], stream), "cudaEventRecord");
     check(cudaGetLastError(), "product kernels");
 }
 
 // Work-space layout of one product (256-byte aligned pieces).
 struct WorkLayout {
-    size_t operands, residues, crt_in, dots, result, tile_counter, total;
+    size_t operands, residues, crt_in, dots, result, tile_counters, total;
 };
 
 WorkLayout work_layout(const negacyclic_plan& s) {
@@ -162,8 +169,8 @@ WorkLayout work_layout(const negacyclic_plan& s) {
     at = align(at + size_t(h.n) * s.dots_stride * 8);
     w.result = at;
     at = align(at + size_t(h.n) * h.limbs * 4);
-    w.tile_counter = at;  // the tensor-core GEMMs of this work space run one after another
-    at = align(at + 4);
+    w.tile_counters = at;
+    at = align(at + kTileCounters * 4);
     w.total = at;
     return w;
 }
@@ -181,9 +188,11 @@ std::string bind_work(negacyclic_plan& s, void* arena) {
     s.crt_in = reinterpret_cast<uint32_t*>(base + w.crt_in);
     s.dots = reinterpret_cast<uint64_t*>(base + w.dots);
     s.result = reinterpret_cast<uint32_t*>(base + w.result);
+    s.tile_counters = reinterpret_cast<uint32_t*>(base + w.tile_counters);
     s.convert_engine = s.crt_engine = NEGACYCLIC_GEMM_SIMT;
     if (!s.gemm_tensor_wanted) return "";
-    s.convert_gemm.tile_counter = s.crt_gemm.tile_counter = reinterpret_cast<uint32_t*>(base + w.tile_counter);
+    s.convert_gemm.tile_counter = s.tile_counters;
+    s.crt_gemm.tile_counter = s.tile_counters + 1;
     std::string why_convert, why_crt;
     if (prepare_gemm_tensor(s.convert_gemm, reinterpret_cast<const uint8_t*>(s.operands), uint64_t(s.padded_limbs) * 4,
                             RowMap::split_rows(h.n, h.n_sub, h.split, 0, h.n_sub, 0, h.split), 2 * h.n, s.convert_weights,
@@ -212,7 +221,8 @@ std::string bind_work(negacyclic_plan& s, void* arena) {
 
 void enqueue_device_product(negacyclic_plan& s, const uint32_t* d_a, const uint32_t* d_b, uint32_t* d_c,
                             cudaStream_t stream) {
-    launch_pad_operands(d_a, d_b, s.operands, s.host.n, s.host.limbs, s.padded_limbs, s.host.split, stream);
+    launch_pad_operands(d_a, d_b, s.operands, s.host.n, s.host.limbs, s.padded_limbs, s.host.split, s.tile_counters,
+                        stream);
     enqueue_product(s, d_c, stream);
 }
 
@@ -369,6 +379,7 @@ int negacyclic_init(uint32_t n, uint32_t w, uint32_t limbs, const uint32_t* q, c
             cudaFree(probe);
             s.operands = s.residues = s.crt_in = s.result = nullptr;
             s.dots = nullptr;
+            s.tile_counters = nullptr;
             if (!why.empty()) return fail(NEGACYCLIC_EINVAL, why);
         }
     } catch (const CudaError& e) {
@@ -460,7 +471,7 @@ int negacyclic_run_device_timed(negacyclic_plan* s, const uint32_t* d_a, const u
         for (auto& e : events) check(cudaEventCreate(&e), "cudaEventCreate");
         check(cudaEventRecord(events[0], stream), "cudaEventRecord");
         launch_pad_operands(d_a, d_b, s->operands, s->host.n, s->host.limbs, s->padded_limbs, s->host.split,
-                            stream);
+                            s->tile_counters, stream);
         check(cudaEventRecord(events[1], stream), "cudaEventRecord");
         enqueue_product(*s, d_c, stream, events + 2);
         check(cudaEventSynchronize(events[kStages + 1]), "product");
@@ -837,7 +848,10 @@ int negacyclic_gemm_u8(const uint8_t* d_a, const uint8_t* d_b, int32_t* d_d, uin
             std::string why;
             if (!prepare_gemm_tensor(plan, d_a, k, rows, m, d_b, n, k, why) || (plan.narrow && !(why = kFewColumns).empty()))
                 return fail(NEGACYCLIC_EINVAL, "tensor GEMM unavailable: " + why);
-            launch_gemm_tensor(plan, raw, stream, rows, m, engine == NEGACYCLIC_GEMM_TENSOR, 0, kNoWithheldStep, 0);
+            TensorGemmOptions options;
+            options.allow_pairs = engine == NEGACYCLIC_GEMM_TENSOR;
+            options.pair_min_steps = 0;  // the caller names the kernel
+            launch_gemm_tensor(plan, raw, stream, rows, m, options);
         } else {
             launch_gemm_simt(d_a, k, rows, m, d_b, n, k, raw, stream);
         }
@@ -877,8 +891,12 @@ int negacyclic_gemm_u8_withheld(const uint8_t* d_a, const uint8_t* d_b, int32_t*
         raw.raw_ld = n;
         raw.status = status;
         check(cudaEventRecord(start, stream), "cudaEventRecord");
-        launch_gemm_tensor(plan, raw, stream, rows, m, engine == NEGACYCLIC_GEMM_TENSOR, (long long)limit_cycles,
-                           withheld_step, 0);
+        TensorGemmOptions options;
+        options.allow_pairs = engine == NEGACYCLIC_GEMM_TENSOR;
+        options.pair_min_steps = 0;  // the caller names the kernel
+        options.limit_cycles = (long long)limit_cycles;
+        options.withheld = withheld_step;
+        launch_gemm_tensor(plan, raw, stream, rows, m, options);
         check(cudaGetLastError(), "gemm");
         check(cudaEventRecord(stop, stream), "cudaEventRecord");
         check(cudaStreamSynchronize(stream), "gemm");

@@ -29,6 +29,7 @@ struct negacyclic_plan {
     // per-product work space: one arena, owned or bound by the caller (batches, servers)
     uint32_t *operands = nullptr, *residues = nullptr, *crt_in = nullptr, *result = nullptr;
     uint64_t* dots = nullptr;
+    uint32_t* tile_counters = nullptr;  // [kTileCounters], in the work space
     // status word of this plan's products (NEGACYCLIC_STATUS_* bits): the reduce kernel and both
     // tensor GEMMs set bits in it; allocated with the tables, or pointed into a batch's array
     uint32_t* status = nullptr;

@@ -101,11 +101,13 @@ void* static_work_address(int device) {
 struct Binding {
     uint32_t *operands, *residues, *crt_in, *result;
     uint64_t* dots;
+    uint32_t* tile_counters;
     uint32_t convert_engine, crt_engine;
     TensorGemmPlan convert_gemm, crt_gemm;
 
     explicit Binding(const negacyclic_plan& s)
-        : operands(s.operands), residues(s.residues), crt_in(s.crt_in), result(s.result), dots(s.dots), convert_engine(s.convert_engine), crt_engine(s.crt_engine),
+        : operands(s.operands), residues(s.residues), crt_in(s.crt_in), result(s.result), dots(s.dots),
+          tile_counters(s.tile_counters), convert_engine(s.convert_engine), crt_engine(s.crt_engine),
           convert_gemm(s.convert_gemm), crt_gemm(s.crt_gemm) {}
 
     void restore(negacyclic_plan& s) const {
@@ -114,6 +116,7 @@ struct Binding {
         s.crt_in = crt_in;
         s.result = result;
         s.dots = dots;
+        s.tile_counters = tile_counters;
         s.convert_engine = convert_engine;
         s.crt_engine = crt_engine;
         s.convert_gemm = convert_gemm;
