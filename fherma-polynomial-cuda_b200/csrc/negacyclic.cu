@@ -498,7 +498,7 @@ bool page_locked(const void* ptr) {
     return attr.type == cudaMemoryTypeHost || attr.type == cudaMemoryTypeManaged;
 }
 
-// Page-locked staging and the copy team of the host path, made on first use.
+// Page-locked staging of the host path, made on first use, and the process's copy team.
 // NEGACYCLIC_HOST_THREADS sets the team's size (by default up to 6 of the host's cores), and
 // NEGACYCLIC_HOST_SPIN_US how long its threads spin before they sleep (default 100000 us).
 // Host memory bandwidth, shared with the copy engines and the caller's output fill, is the limit:
@@ -516,7 +516,7 @@ void ensure_staging(negacyclic_plan& s) {
         std::chrono::microseconds spin = HostTeam::kSpinTime;
         if (const char* env = getenv("NEGACYCLIC_HOST_SPIN_US"))
             spin = std::chrono::microseconds(std::min<unsigned long>(10000000ul, std::strtoul(env, nullptr, 10)));
-        s.team = std::make_unique<HostTeam>(workers, spin);
+        s.team = shared_host_team(workers, spin);
     }
 }
 

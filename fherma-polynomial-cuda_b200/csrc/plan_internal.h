@@ -49,7 +49,7 @@ struct negacyclic_plan {
     // the host path's copy of the status word, written on `stream` after the last kernel, so
     // that reading it costs no extra round trip once the stream has finished
     uint32_t* status_host = nullptr;
-    std::unique_ptr<negacyclic::HostTeam> team;
+    std::shared_ptr<negacyclic::HostTeam> team;     // the process's, held while this plan lives
     std::atomic<uint32_t> packed[kMaxChunks] = {};  // pieces of input chunk k packed
     std::atomic<uint32_t> next_piece{0};            // next unclaimed piece of the running pack job
     uint64_t pack_ticket = 0;                       // the running call's pack job (0: none)
@@ -73,6 +73,7 @@ struct negacyclic_plan {
             if (out_ready[c]) cudaEventDestroy(out_ready[c]);
             if (copied_out[c]) cudaEventDestroy(copied_out[c]);
         }
+        if (team && pack_ticket) team->wait(pack_ticket);  // a call that failed part-way may still be packing
         if (stage_in) cudaFreeHost(stage_in);
         if (stage_out) cudaFreeHost(stage_out);
         if (status_host) cudaFreeHost(status_host);
