@@ -73,6 +73,8 @@ __device__ __forceinline__ uint32_t bit_reverse(uint32_t x, uint32_t bits) {
     return bits ? (__brev(x) >> (32 - bits)) : 0u;
 }
 
+__device__ uint32_t twiddle_place(uint32_t m, uint32_t log_n);
+
 __global__ void twiddles_kernel(const DevicePrime* __restrict__ primes, uint32_t r, uint32_t n_sub,
                                 uint32_t log_n, uint2* fwd, uint2* inv, uint2* zeta) {
     uint32_t k = blockIdx.y;
@@ -84,8 +86,9 @@ __global__ void twiddles_kernel(const DevicePrime* __restrict__ primes, uint32_t
         uint32_t w_inv = pow_mod(f.psi, 2ull * n_sub - e, f);
         uint32_t w_zeta = pow_mod(f.psi, 2ull * e + 1, f);
         size_t at = size_t(k) * n_sub + m;
-        fwd[at] = make_uint2(w_fwd, shoup_quotient(w_fwd, f.p));
-        inv[at] = make_uint2(w_inv, shoup_quotient(w_inv, f.p));
+        const size_t placed = size_t(k) * n_sub + twiddle_place(m, log_n);
+        fwd[placed] = make_uint2(w_fwd, shoup_quotient(w_fwd, f.p));
+        inv[placed] = make_uint2(w_inv, shoup_quotient(w_inv, f.p));
         zeta[at] = make_uint2(w_zeta, shoup_quotient(w_zeta, f.p));
     }
 }
@@ -247,19 +250,29 @@ __global__ void __launch_bounds__(512) ntt_inverse_kernel(uint32_t* residues, co
 }
 
 // ---------------------------------------------------------------------------
-// Register-blocked NTT for N' >= 256: 16 values per thread (N'/16 threads),
-// up to four butterfly stages per pass between shared-memory exchanges.
+// Register-blocked NTT for N' >= 256: 16 values per thread (32 at N' = 8192), up to four (five)
+// butterfly stages per pass between shared-memory exchanges.
 // A pass of R stages on group g (2^R values spaced t_min apart, t_min = the
 // smallest half-size in the pass) covers indices base + k*t_min, k < 2^R, with
 // base = (g / t_min) * 2^R * t_min + g % t_min.
+//
+// What bounds it, at N' = 8192: issue slots, the multiply pipe and the ALU are each about half used,
+// and shared-memory and twiddle loads take the rest. 32 values per thread take 5 + 4 + 4 stages in
+// three passes, one exchange fewer than 4 + 4 + 4 + 1, in four CTAs of 256 threads per SM instead of
+// two of 512, so that one CTA's loads and barriers fall into another's arithmetic; twiddles are loaded in
+// pairs, and those of the unit-stride pass from a table laid out for it. 16450 warp instructions per
+// transform instead of 18600. Forward 2010 -> 1840 us and inverse 1226 -> 961 us at N = 65536,
+// L = 1747 (58176 and 29088 transforms; 2.1 TB/s). Keeping the next transform's input on its way into
+// shared memory (persistent CTAs), or 16 values per thread with three CTAs of 512, were slower.
 
-constexpr uint32_t kPerThread = 16;
+constexpr uint32_t per_thread(uint32_t log) { return log == 13 ? 32 : 16; }  // values per thread
 
 // Shared-memory layout of a length-2^kLog transform: word i is stored at i ^ M(i >> 5), where M
-// XORs column b into the bank bits when bit 5 + b of i is set. The columns were found by an
-// exhaustive check of every warp access of every pass (forward and inverse, 16 values per
-// thread): with them no pass has a bank conflict, where padding one word per 32 left 2-way
-// conflicts in the passes with half-size 2 and 1 or 16. M is linear, and a pass's per-value
+// XORs column b into the bank bits when bit 5 + b of i is set. A pass's warp accesses vary five bits
+// of i; they are free of bank conflicts when the images of those bits are linearly independent. The
+// columns up to 2^12 were found by an exhaustive check of every warp access of every pass (forward
+// and inverse). At 2^13 the passes vary bits 0-4, bits 0-3 and 8, and bits 4-8, which the columns
+// below keep independent. M is linear, and a pass's per-value
 // offsets k t_min share no bits with its group base, so the swizzle of base + k t_min is the
 // swizzle of base (once per group) XOR a compile-time constant.
 template <uint32_t kLog>
@@ -269,7 +282,7 @@ __host__ __device__ constexpr uint32_t swizzle_column(int b) {
     constexpr uint32_t c10[] = {27, 13, 8, 26, 8};
     constexpr uint32_t c11[] = {11, 1, 14, 20, 24, 27};
     constexpr uint32_t c12[] = {17, 26, 2, 21, 24, 25, 27};
-    constexpr uint32_t c13[] = {7, 9, 27, 13, 8, 26, 8, 13};
+    constexpr uint32_t c13[] = {1, 2, 4, 24, 0, 0, 0, 0};
     return kLog == 8 ? c8[b] : kLog == 9 ? c9[b] : kLog == 10 ? c10[b] : kLog == 11 ? c11[b] : kLog == 12 ? c12[b] : c13[b];
 }
 
@@ -281,6 +294,30 @@ __host__ __device__ constexpr uint32_t swizzle(uint32_t i) {
     return i ^ m;
 }
 
+// Twiddle b of the `blocks` that a group uses in one stage; `stage` points at the stage's table
+// (entries m .. 2m of the prime's row), which serves groups 0 .. m / blocks. Twiddles come two at a
+// time, the odd one with the even one before it (rows and stages start on 16-byte boundaries).
+// In table order a group's twiddles are consecutive. In the unit-stride pass of length 8192, where
+// every lane has a group of its own, the table is laid out pair by pair instead (twiddle_place), so
+// that a warp's load is 512 consecutive bytes and not 32 pieces 64 bytes apart.
+constexpr uint32_t kPairedGroups = 512;  // groups of 16 in the unit-stride pass of length 8192
+
+template <int blocks, bool kPaired>
+__device__ __forceinline__ uint2 stage_twiddle(const uint2* __restrict__ stage, uint32_t group, int b) {
+    if constexpr (blocks == 1) return __ldg(stage + group);
+    const uint32_t at = kPaired ? uint32_t(b / 2) * kPairedGroups + group : (group * blocks + b) / 2;
+    const uint4 pair = __ldg(reinterpret_cast<const uint4*>(stage) + at);
+    return b % 2 ? make_uint2(pair.z, pair.w) : make_uint2(pair.x, pair.y);
+}
+
+// Where twiddle m of a length-2^log_n table is stored in the prime's row.
+__device__ uint32_t twiddle_place(uint32_t m, uint32_t log_n) {
+    if (log_n != 13 || m < 2 * kPairedGroups) return m;
+    const uint32_t stage = 1u << (31 - __clz(m)), blocks = stage / kPairedGroups, e = m - stage;
+    const uint32_t group = e / blocks, b = e % blocks;
+    return stage + ((b / 2) * kPairedGroups + group) * 2 + b % 2;
+}
+
 // Cooley-Tukey stages with half-sizes t_min*2^(R-1) .. t_min (forward, merged psi twiddles) on
 // one group of 2^R values. With j = base + k*t_min and base = group_hi * 2^(log t_min + R) + off
 // (off < t_min), butterfly (k, k + half) of stage r has twiddle m + (j >> (log t + 1))
@@ -289,60 +326,60 @@ __host__ __device__ constexpr uint32_t swizzle(uint32_t i) {
 // Values between stages are kept in [0, 2p) (2p < 2^32): each butterfly reduces its two inputs
 // once, so that u + v and u - v + p stay below 2p, and multiplies by the twiddle without
 // Shoup's final correction. Canonical inputs are a special case; the last pass reduces.
-template <int R>
+template <int R, bool kPaired, int r = 0>
 __device__ __forceinline__ void ct_stages(uint32_t (&x)[1 << R], uint32_t group_hi, uint32_t log_t_min,
                                           uint32_t log_n, const uint2* __restrict__ table, uint32_t p) {
+    constexpr int half = 1 << (R - 1 - r), blocks = 1 << r;
+    const uint32_t log_t = log_t_min + (R - 1 - r);  // this stage's half-size t = 2^log_t
+    const uint32_t m = 1u << (log_n - 1 - log_t);     // number of groups: n / (2t)
+    const uint2* stage = table + m;
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-        const int half = 1 << (R - 1 - r);
-        const uint32_t log_t = log_t_min + (R - 1 - r);  // this stage's half-size t = 2^log_t
-        const uint32_t m = 1u << (log_n - 1 - log_t);     // number of groups: n / (2t)
+    for (int b = 0; b < blocks; ++b) {
+        const uint2 w = stage_twiddle<blocks, kPaired>(stage, group_hi, b);
 #pragma unroll
-        for (int b = 0; b < (1 << r); ++b) {
-            const uint2 w = __ldg(&table[m + (group_hi << r) + b]);
-#pragma unroll
-            for (int k = b * 2 * half; k < b * 2 * half + half; ++k) {
-                const uint32_t u = reduce_once(x[k], p);
-                const uint32_t v = reduce_once(shoup_lazy(x[k + half], w.x, w.y, p), p);
-                x[k] = u + v;
-                x[k + half] = u - v + p;
-            }
+        for (int j = 0; j < half; ++j) {
+            const int k = b * 2 * half + j;
+            const uint32_t u = reduce_once(x[k], p);
+            const uint32_t v = reduce_once(shoup_lazy(x[k + half], w.x, w.y, p), p);
+            x[k] = u + v;
+            x[k + half] = u - v + p;
         }
     }
+    if constexpr (r + 1 < R) ct_stages<R, kPaired, r + 1>(x, group_hi, log_t_min, log_n, table, p);
 }
 
 // Gentleman-Sande stages with half-sizes t_min .. t_min*2^(R-1) (inverse). Stage r's butterflies
 // (k, k + 2^r) in block b = k >> (r + 1) share twiddle h + group_hi * 2^(R-1-r) + b.
 // Values between stages are in [0, 2p), as in ct_stages.
-template <int R>
+template <int R, bool kPaired, int r = 0>
 __device__ __forceinline__ void gs_stages(uint32_t (&x)[1 << R], uint32_t group_hi, uint32_t log_t_min,
                                           uint32_t log_n, const uint2* __restrict__ table, uint32_t p) {
+    constexpr int half = 1 << r;
+    const uint32_t log_t = log_t_min + r;
+    const uint32_t h = 1u << (log_n - 1 - log_t);
+    constexpr int blocks = 1 << (R - 1 - r);
+    const uint2* stage = table + h;
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-        const int half = 1 << r;
-        const uint32_t log_t = log_t_min + r;
-        const uint32_t h = 1u << (log_n - 1 - log_t);
+    for (int b = 0; b < blocks; ++b) {
+        const uint2 w = stage_twiddle<blocks, kPaired>(stage, group_hi, b);
 #pragma unroll
-        for (int b = 0; b < (1 << (R - 1 - r)); ++b) {
-            const uint2 w = __ldg(&table[h + (group_hi << (R - 1 - r)) + b]);
-#pragma unroll
-            for (int k = b * 2 * half; k < b * 2 * half + half; ++k) {
-                const uint32_t u = reduce_once(x[k], p), v = reduce_once(x[k + half], p);
-                x[k] = u + v;
-                x[k + half] = shoup_lazy(u - v + p, w.x, w.y, p);
-            }
+        for (int j = 0; j < half; ++j) {
+            const int k = b * 2 * half + j;
+            const uint32_t u = reduce_once(x[k], p), v = reduce_once(x[k + half], p);
+            x[k] = u + v;
+            x[k + half] = shoup_lazy(u - v + p, w.x, w.y, p);
         }
     }
+    if constexpr (r + 1 < R) gs_stages<R, kPaired, r + 1>(x, group_hi, log_t_min, log_n, table, p);
 }
 
-// One pass of R stages over all of this thread's groups (transform length 2^kLog,
-// 2^(kLog-4) threads). src/dst are shared (swizzled index) or global (plain index);
+// One pass of R stages over all of this thread's groups (transform length 2^kLog). src/dst are shared (swizzled index) or global (plain index);
 // kScale multiplies the values stored to global by (f, f_q).
 template <int R, bool kForward, bool kFromGlobal, bool kToGlobal, bool kScale, uint32_t kLogTMin, uint32_t kLog>
 __device__ __forceinline__ void ntt_pass(const uint32_t* src, uint32_t* dst, const uint2* __restrict__ table,
                                          uint32_t p, uint32_t f, uint32_t f_q) {
-    constexpr int G = kPerThread >> R;  // groups per thread
-    constexpr uint32_t kThreads = 1u << (kLog - 4);
+    constexpr int G = per_thread(kLog) >> R;  // groups per thread
+    constexpr uint32_t kThreads = (1u << kLog) / per_thread(kLog);
 #pragma unroll
     for (int g = 0; g < G; ++g) {
         const uint32_t group = threadIdx.x + g * kThreads;
@@ -375,10 +412,11 @@ __device__ __forceinline__ void ntt_pass(const uint32_t* src, uint32_t* dst, con
                 x[k] = kFromGlobal ? src[i] : src[placed ^ swizzle<kLog>(uint32_t(k) << kLogTMin)];
             }
         }
+        constexpr bool kPaired = kLog == 13 && kLogTMin == 0;
         if (kForward)
-            ct_stages<R>(x, group >> kLogTMin, kLogTMin, kLog, table, p);
+            ct_stages<R, kPaired>(x, group >> kLogTMin, kLogTMin, kLog, table, p);
         else
-            gs_stages<R>(x, group >> kLogTMin, kLogTMin, kLog, table, p);
+            gs_stages<R, kPaired>(x, group >> kLogTMin, kLogTMin, kLog, table, p);
 #pragma unroll
         for (int k = 0; k < (1 << R); ++k) {
             if (kScale)
@@ -388,6 +426,23 @@ __device__ __forceinline__ void ntt_pass(const uint32_t* src, uint32_t* dst, con
         }
         if constexpr (kToGlobal && kPair) {
             *reinterpret_cast<uint2*>(dst + base) = make_uint2(x[0], x[1]);
+        } else if constexpr (kToGlobal && kVector && R == 4) {
+            // neighbouring lanes trade quarters of their 16 words, so that the two of them fill
+            // whole 32-byte sectors with each store
+            const bool odd = threadIdx.x & 1;
+            uint32_t* to = dst + base - (odd ? 16 - 4 : 0);
+#pragma unroll
+            for (int q = 0; q < 16; q += 8) {
+                uint32_t first[4], second[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const uint32_t got = __shfl_xor_sync(0xffffffffu, odd ? x[q + i] : x[q + 4 + i], 1);
+                    first[i] = odd ? got : x[q + i];
+                    second[i] = odd ? x[q + 4 + i] : got;
+                }
+                *reinterpret_cast<uint4*>(to + q) = make_uint4(first[0], first[1], first[2], first[3]);
+                *reinterpret_cast<uint4*>(to + q + 16) = make_uint4(second[0], second[1], second[2], second[3]);
+            }
         } else if constexpr (kToGlobal && kVector) {
 #pragma unroll
             for (int q = 0; q < (1 << R) / 4; ++q)
@@ -408,11 +463,14 @@ __device__ __forceinline__ void ntt_pass(const uint32_t* src, uint32_t* dst, con
 // Passes kDone.. of a length-2^kLog transform: four stages per pass, and a shorter pass for the
 // remainder at the unit-stride end, where it touches global memory 2 consecutive words per
 // thread instead of 16: last in the forward transform (half-sizes large -> small), first in the
-// inverse (small -> large, which also scales its output).
+// inverse (small -> large, which also scales its output). Length 8192 takes five stages at the
+// large-stride end instead (its global accesses there are whole 128-byte lines), and four at the
+// unit-stride end, where lanes trade words so that their stores fill sectors.
 template <bool kForward, uint32_t kLog, uint32_t kDone>
 __device__ __forceinline__ void ntt_passes(uint32_t* data, uint32_t* xs, const uint2* __restrict__ table, uint32_t p,
                                            uint32_t f, uint32_t f_q) {
-    constexpr int R = (!kForward && kDone == 0 && kLog % 4 != 0) ? int(kLog % 4)
+    constexpr int R = kLog == 13 ? (kForward ? (kDone == 0 ? 5 : 4) : (kDone == 8 ? 5 : 4))
+                      : (!kForward && kDone == 0 && kLog % 4 != 0) ? int(kLog % 4)
                       : (kLog - kDone) < 4                       ? int(kLog - kDone)
                                                                   : 4;
     constexpr uint32_t kLogTMin = kForward ? kLog - kDone - R : kDone;
@@ -428,7 +486,7 @@ __device__ __forceinline__ void ntt_passes(uint32_t* data, uint32_t* xs, const u
 // grid (op_count t_count, r): x = (op - op_first)*t_count + (t - t_first), y = prime, so a prime's
 // transforms share its twiddles in L2
 template <uint32_t kLog>
-__global__ void __launch_bounds__(1u << (kLog - 4), (kLog >= 13 ? 2 : 4)) ntt_forward_blocked_kernel(
+__global__ void __launch_bounds__((1u << kLog) / per_thread(kLog), 4) ntt_forward_blocked_kernel(
     uint32_t* residues, const DevicePrime* __restrict__ primes, const uint2* __restrict__ fwd, uint32_t r, uint32_t n,
     uint32_t t_first, uint32_t t_count, uint32_t op_first) {
     chain_enter();
@@ -441,7 +499,7 @@ __global__ void __launch_bounds__(1u << (kLog - 4), (kLog >= 13 ? 2 : 4)) ntt_fo
 }
 
 template <uint32_t kLog>
-__global__ void __launch_bounds__(1u << (kLog - 4), (kLog >= 13 ? 2 : 4)) ntt_inverse_blocked_kernel(
+__global__ void __launch_bounds__((1u << kLog) / per_thread(kLog), 4) ntt_inverse_blocked_kernel(
     uint32_t* residues, const DevicePrime* __restrict__ primes, const uint2* __restrict__ inv, uint32_t r, uint32_t n,
     uint32_t v_first, uint32_t v_count, uint32_t /*op_first: the inverse works on operand row 0 only*/) {
     chain_enter();
@@ -865,7 +923,7 @@ static void launch_blocked(uint32_t* residues, const DevicePrime* primes, const 
         configured = true;
     }
     dim3 grid(kForward ? op_count * count : count, r);
-    launch_chained(kernel, grid, kN / kPerThread, smem, stream, residues, primes, table, r, n, first, count, op_first);
+    launch_chained(kernel, grid, kN / per_thread(kLog), smem, stream, residues, primes, table, r, n, first, count, op_first);
 }
 
 template <bool kForward>
