@@ -27,6 +27,7 @@
 
 #include "gemm_tc.cuh"
 #include "launch.cuh"
+#include "reduce.cuh"
 
 namespace negacyclic {
 
@@ -40,18 +41,26 @@ constexpr uint32_t kStageBytes = kATileBytes + kBTileBytes;
 constexpr uint32_t kAccColumns = 256;                            // one 128 x 256 s32 accumulator
 constexpr uint32_t kEpilogueWarps = 8;  // two per 32-row quarter of the tile, half of the columns each
 constexpr uint32_t kThreads = 64 + 32 * kEpilogueWarps;
+constexpr uint32_t kLoaderWarps = 4;                 // gathered A: 32 rows of the tile each
+constexpr uint32_t kGatherThreads = kThreads + 32 * kLoaderWarps;
+constexpr uint32_t kLoaderDepth = 3;                 // stages a loader warp keeps in flight
+constexpr uint32_t kStagingPitch = 80;               // bytes per row of an epilogue warp's 16 result words
+constexpr uint32_t kStagingBytes = 32 * kStagingPitch;
 constexpr long long kDefaultLimitCycles = 4000000000ll;  // ~2 s at 1.9 GHz
 constexpr uint64_t kAbortDrainNs = 1000000;               // 1 ms: in-flight TMA loads land long before
 constexpr size_t kSmemBytes = size_t(kStages) * kStageBytes + 1024 /*align*/ + 256 /*barriers, TMEM slot*/;
+constexpr size_t kReduceSmemBytes = kSmemBytes + kEpilogueWarps * kStagingBytes;
 
 __device__ uint32_t g_tc_error;
 __device__ uint32_t g_tile_counter;  // tile counter of GEMMs without one of their own
 
-// Instruction descriptor: D s32, A/B unsigned 8-bit, both K-major, M=128, N=256.
-constexpr uint32_t kInstrDesc = (2u << 4)              /* c_format = S32 */
-                                | (0u << 7) | (0u << 10) /* a/b format = u8 */
-                                | (0u << 15) | (0u << 16) /* K-major */
-                                | ((kBlockN >> 3) << 17) | ((kBlockM >> 4) << 24);
+// Instruction descriptor: D s32, A/B unsigned 8-bit, both K-major, M=128, N=block_n.
+constexpr uint32_t instr_desc(uint32_t block_n) {
+    return (2u << 4)                 /* c_format = S32 */
+           | (0u << 7) | (0u << 10)  /* a/b format = u8 */
+           | (0u << 15) | (0u << 16) /* K-major */
+           | ((block_n >> 3) << 17) | ((kBlockM >> 4) << 24);
+}
 
 __device__ __forceinline__ uint32_t smem_u32(const void* ptr) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(ptr));
@@ -132,12 +141,13 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, u
         : "memory");
 }
 
-__device__ __forceinline__ void mma_i8(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t accumulate) {
+__device__ __forceinline__ void mma_i8(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t instr,
+                                       uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-        "l"(desc_a), "l"(desc_b), "r"(kInstrDesc), "r"(accumulate)
+        "l"(desc_a), "l"(desc_b), "r"(instr), "r"(accumulate)
         : "memory");
 }
 
@@ -162,6 +172,27 @@ __device__ __forceinline__ void tmem_load32(uint32_t taddr, uint32_t (&v)[32]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
+// 32 rows x 4 columns (one word sum) of an accumulator; the caller waits (tmem_wait).
+__device__ __forceinline__ void tmem_load4(uint32_t taddr, uint32_t (&v)[4]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
+                 : "r"(taddr));
+}
+
+__device__ __forceinline__ void tmem_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+
+__device__ __forceinline__ uint64_t word_sum(uint32_t v0, uint32_t v1, uint32_t v2, uint32_t v3) {
+    return uint64_t(v0) + (uint64_t(v1) << 8) + (uint64_t(v2) << 16) + (uint64_t(v3) << 24);
+}
+
+__device__ __forceinline__ void cp_async_4(uint32_t smem, const void* global, uint32_t bytes) {  // 0: zero fill
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem), "l"(global), "r"(bytes) : "memory");
+}
+
+__device__ __forceinline__ void cp_async_16_or_zero(uint32_t smem, const void* global, uint32_t bytes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem), "l"(global), "r"(bytes) : "memory");
+}
+
 struct TileShape {
     uint32_t m, columns, k_tiles, m_tiles, n_tiles, group_m;
     RowMap rows;
@@ -169,6 +200,7 @@ struct TileShape {
     uint32_t* status;        // caller's status word (NEGACYCLIC_STATUS_*), or nullptr
     long long limit;         // cycles any one pipeline wait may take
     uint32_t withheld;       // diagnostics: CTA (pair) 0's producer stops before this pipeline step
+    uint32_t block_n;        // columns per tile: 256, or 128 (single-CTA kernel)
 };
 
 // Tile index -> (m tile, n tile) in groups of group_m m-tiles, m fastest, so the
@@ -218,7 +250,7 @@ __device__ __forceinline__ void epilogue_chunk(const Epilogue& epi, const uint32
         if (g0 + g < epi.words) out[g] = sum[g];
 }
 
-// One epilogue warp's share of an accumulator: 32 rows (one per lane) x 128 columns starting at
+// One epilogue warp's share of an accumulator: 32 rows (one per lane) x 32 `chunks` columns starting at
 // col0 (half a tile), read from TMEM at t_base in 32-column chunks.
 // Conversion: column group g = 4k..4k+3 holds the byte dots of prime k; the residue is
 // REDC(sum_d G_d 256^d). The chunk's eight primes are loaded (the same address in every lane)
@@ -227,13 +259,13 @@ __device__ __forceinline__ void epilogue_chunk(const Epilogue& epi, const uint32
 // itself leaves its scheduler idle four cycles out of five (2140 instructions in 10.5k cycles per
 // 256 x 256 tile with one warp per quarter). Two warps per quarter share the tile.
 __device__ __forceinline__ void epilogue_rows(const Epilogue& epi, uint32_t t_base, uint32_t col0, uint32_t columns,
-                                              bool row_ok, uint64_t out_row, uint32_t op, uint32_t column) {
-    constexpr uint32_t kChunks = kBlockN / 32 / 2;
+                                              uint32_t chunks, bool row_ok, uint64_t out_row, uint32_t op,
+                                              uint32_t column) {
     if (epi.mode == kEpilogueConvert) {
         const uint32_t k0 = col0 / 4;
         uint32_t* out = epi.residues + (size_t(op) * epi.r + k0) * epi.n + column;  // + g * N for prime k0 + g
 #pragma unroll 1
-        for (uint32_t chunk = 0; chunk < kChunks; ++chunk) {
+        for (uint32_t chunk = 0; chunk < chunks; ++chunk) {
             if (k0 + chunk * 8 >= epi.r) break;  // warp-uniform
             uint2 prime[8];
 #pragma unroll
@@ -254,7 +286,7 @@ __device__ __forceinline__ void epilogue_rows(const Epilogue& epi, uint32_t t_ba
         return;
     }
 #pragma unroll 1
-    for (uint32_t chunk = 0; chunk < kChunks; ++chunk) {
+    for (uint32_t chunk = 0; chunk < chunks; ++chunk) {
         const uint32_t c_base = col0 + chunk * 32;
         if (c_base >= columns) break;  // warp-uniform
         uint32_t v[32];
@@ -263,14 +295,90 @@ __device__ __forceinline__ void epilogue_rows(const Epilogue& epi, uint32_t t_ba
     }
 }
 
+// Reduces 32 rows mod q, one per lane, from a tile's accumulator (columns 4w .. 4w+3 hold word w):
+// lane l's coefficient is first + l * step. Sixteen words at a time go through `staging` (32 rows of
+// kStagingPitch bytes), so that global stores are 64-byte runs. The accumulator is released once
+// its last column is read.
+__device__ __forceinline__ void reduce_rows(const ReduceParams& prm, uint32_t t_base, uint32_t* staging, uint32_t first,
+                                            uint32_t step, uint64_t* release, uint32_t lane) {
+    const uint32_t limbs = prm.limbs, tlen = limbs + 2;
+    uint32_t vx[3][4], vw[kWindow][4] = {};
+#pragma unroll
+    for (int i = 0; i < 3; ++i) tmem_load4(t_base + 4 * (limbs + 2 + i), vx[i]);
+#pragma unroll
+    for (int j = 0; j < kWindow; ++j) {
+        uint32_t w;
+        if (window_word(prm, j, w)) tmem_load4(t_base + 4 * w, vw[j]);  // grid-uniform
+    }
+    tmem_wait();
+    uint64_t x[3], window[kWindow];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) x[i] = word_sum(vx[i][0], vx[i][1], vx[i][2], vx[i][3]);
+#pragma unroll
+    for (int j = 0; j < kWindow; ++j) window[j] = word_sum(vw[j][0], vw[j][1], vw[j][2], vw[j][3]);
+    const RowQuotient f = row_quotient(x, window, prm);
+    RowState st;
+    uint32_t* out = prm.out + size_t(first) * limbs;
+    const size_t pitch = size_t(step) * limbs;
+    for (uint32_t base = 0; base < tlen; base += 16) {
+        uint64_t d[16];
+        uint4 q[4], r[4];
+#pragma unroll
+        for (uint32_t g = 0; g < 4; ++g) {
+            q[g] = __ldg(reinterpret_cast<const uint4*>(prm.q + base) + g);
+            r[g] = __ldg(reinterpret_cast<const uint4*>(prm.minus_p + base) + g);
+        }
+#pragma unroll
+        for (uint32_t h = 0; h < 2; ++h) {
+            uint32_t v[32];
+            tmem_load32(t_base + 4 * base + 32 * h, v);
+#pragma unroll
+            for (uint32_t i = 0; i < 8; ++i) d[8 * h + i] = word_sum(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+        }
+        if (base + 16 >= tlen) {  // the accumulator's last columns are in registers
+            fence_before();
+            __syncwarp();
+            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(release)) : "memory");
+        }
+        uint32_t o[16];
+        st.words16(f, d, q, r, base, prm, o);
+#pragma unroll
+        for (uint32_t g = 0; g < 4; ++g)
+            reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(staging) + lane * kStagingPitch)[g] =
+                make_uint4(o[4 * g], o[4 * g + 1], o[4 * g + 2], o[4 * g + 3]);
+        __syncwarp();
+        if (base + lane % 16 < limbs) {  // two rows per instruction
+#pragma unroll
+            for (uint32_t i = 0; i < 16; ++i) {
+                const uint32_t row = 2 * i + lane / 16;
+                out[row * pitch + base + lane % 16] = staging[row * (kStagingPitch / 4) + lane % 16];
+            }
+        }
+        __syncwarp();
+    }
+    st.finish(out + lane * pitch, prm);
+}
+
 // Persistent, warp-specialised GEMM: each CTA walks tiles blockIdx.x, +gridDim.x, ...
 //   warp 0 (one thread)  TMA producer over a kStages-deep shared-memory ring
 //   warp 1 (one thread)  MMA issuer; the whole warp allocates / frees 512 TMEM columns
 //   warps 2-9            epilogue; two 256-column accumulators alternate between tiles,
 //                        so tile i's epilogue overlaps tile i+1's MMAs
-__global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_constant__ CUtensorMap a_map,
-                                                              const __grid_constant__ CUtensorMap b_map,
-                                                              TileShape shape, Epilogue epi) {
+//   warps 10-13          (gathered A) loaders: instead of TMA they fill the A tiles, 32 rows each,
+//                        with 4-byte cp.async into the 128B-swizzled layout, kLoaderDepth stages
+//                        ahead. Raw operand rows start on any 4-byte boundary, which TMA cannot
+//                        read, and residues are transposed on the way: a lane takes prime
+//                        4q + lane % 4 of row lane / 4, so an instruction reads whole 32-byte
+//                        sectors and writes all 32 banks. This replaces the pad and transpose
+//                        kernels, each a pass over the data and a link in the chain of launches;
+//                        it pays while the K steps are few, since every column tile gathers again.
+// kReduce: all of a row's columns are in one tile, and a warp of the epilogue takes whole rows, one
+// per lane, through the reduction mod q straight from TMEM (csrc/reduce.cuh); the two sets of four
+// warps take alternate tiles, so that two tiles' carry chains run side by side.
+template <int kSource, bool kReduce>
+__global__ void __launch_bounds__(kSource == kSourceTma ? kThreads : kGatherThreads, 1)
+    gemm_tc_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_constant__ CUtensorMap b_map,
+                   TileShape shape, GatherSource source, Epilogue epi) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* a_smem = smem;
@@ -288,12 +396,12 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
 
     if (threadIdx.x == 0) {
         for (uint32_t s = 0; s < kStages; ++s) {
-            mbar_init(&full[s], 1);
+            mbar_init(&full[s], kSource == kSourceTma ? 1 : 1 + kLoaderWarps);
             mbar_init(&empty[s], 1);
         }
         for (uint32_t a = 0; a < 2; ++a) {
             mbar_init(&acc_full[a], 1);
-            mbar_init(&acc_empty[a], kEpilogueWarps);
+            mbar_init(&acc_empty[a], kReduce ? kEpilogueWarps / 2 : kEpilogueWarps);
         }
         mbar_init(drain, 1);
         *abort_flag = 0;
@@ -319,9 +427,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
             for (uint32_t tile = blockIdx.x; tile < tiles && ok && !withheld; tile += gridDim.x) {
                 uint32_t m_tile, n_tile;
                 tile_coords(tile, shape, m_tile, n_tile);
-                const uint32_t row0 = m_tile * kBlockM, col0 = n_tile * kBlockN;
+                const uint32_t row0 = m_tile * kBlockM, col0 = n_tile * shape.block_n;
                 // operand row of the tile's first row; its 128 rows are consecutive in memory
-                const uint32_t a_row = uint32_t(shape.rows.row(row0));
+                const uint32_t a_row = kSource == kSourceTma ? uint32_t(shape.rows.row(row0)) : 0;
                 for (uint32_t ks = 0; ks < shape.k_tiles; ++ks, ++step) {
                     const uint32_t s = step % kStages, round = step / kStages;
                     if (blockIdx.x == 0 && step == shape.withheld) {  // diagnostics: a stage that never comes
@@ -332,8 +440,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
                         ok = false;
                         break;
                     }
-                    mbar_expect_tx(&full[s], kStageBytes);
-                    tma_load_2d(a_smem + s * kATileBytes, &a_map, &full[s], int(ks * kBlockK), int(a_row));
+                    mbar_expect_tx(&full[s], (kSource == kSourceTma ? kATileBytes : 0) + shape.block_n * kBlockK);
+                    if (kSource == kSourceTma)
+                        tma_load_2d(a_smem + s * kATileBytes, &a_map, &full[s], int(ks * kBlockK), int(a_row));
                     tma_load_2d(b_smem + s * kBTileBytes, &b_map, &full[s], int(ks * kBlockK), int(col0));
                     issued = step + 1;
                 }
@@ -342,8 +451,10 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
                 *abort_flag = 1;
                 record_error(shape.status, 1u);
                 // let the loads already issued land before the CTA can exit (each of these phases
-                // completes: this thread armed it and issued all of its bytes)
-                for (uint32_t st = (issued > kStages ? issued - kStages : 0); st < issued; ++st)
+                // completes: this thread armed it and issued all of its bytes; with gathered A the
+                // loaders may have stopped, so there only time tells)
+                if (kSource != kSourceTma) abort_drain();
+                for (uint32_t st = (issued > kStages ? issued - kStages : 0); kSource == kSourceTma && st < issued; ++st)
                     mbar_wait(&full[st % kStages], (st / kStages) & 1, shape.limit);
             }
         }
@@ -351,6 +462,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
         if (lane == 0) {
             // ---------------- MMA issuer
             uint32_t step = 0, local = 0;
+            const uint32_t instr = instr_desc(shape.block_n);
             bool ok = true;
             for (uint32_t tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x, ++local) {
                 const uint32_t acc = local & 1, use = local >> 1;
@@ -371,7 +483,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
                     const uint32_t b_addr = smem_u32(b_smem + s * kBTileBytes);
 #pragma unroll
                     for (uint32_t kk = 0; kk < kBlockK / 32; ++kk)
-                        mma_i8(d_tmem, smem_descriptor(a_addr + kk * 32), smem_descriptor(b_addr + kk * 32),
+                        mma_i8(d_tmem, smem_descriptor(a_addr + kk * 32), smem_descriptor(b_addr + kk * 32), instr,
                                (ks | kk) != 0 ? 1u : 0u);
                     mma_commit(&empty[s]);  // frees the stage once these MMAs have read it
                 }
@@ -384,6 +496,76 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
             mma_commit(drain);  // arrives once every MMA issued above has completed
             if (!mbar_wait(drain, 0, shape.limit)) record_error(shape.status, 8u);
         }
+    } else if (kSource != kSourceTma && warp >= 2 + kEpilogueWarps) {
+        // ---------------- A loaders
+        const uint32_t part = warp - (2 + kEpilogueWarps);  // rows 32 part .. 32 part + 31 of the tile
+        const uint32_t a_addr = smem_u32(a_smem) + part * 32 * kBlockK;
+        uint32_t step = 0, published = 0;
+        bool ok = true;
+        auto publish = [&]() {  // the oldest stage in flight has landed: hand it to the MMA issuer
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0)
+                asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&full[published % kStages]))
+                             : "memory");
+            ++published;
+        };
+        for (uint32_t tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
+            uint32_t m_tile, n_tile, op, t, j;
+            tile_coords(tile, shape, m_tile, n_tile);
+            shape.rows.decompose(m_tile * kBlockM, op, t, j);  // 128 consecutive j of one (op, t)
+            j += part * 32;
+            for (uint32_t ks = 0; ks < shape.k_tiles; ++ks, ++step) {
+                const uint32_t s = step % kStages, round = step / kStages;
+                ok = lane != 0 || (!*abort_flag && mbar_wait(&empty[s], (round & 1) ^ 1, shape.limit, abort_flag));
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
+                const uint32_t to = a_addr + s * kATileBytes;
+                if constexpr (kSource == kSourceRows) {
+                    const uint32_t* rows = (op ? source.rows[1] : source.rows[0]) +
+                                           (size_t(shape.rows.split) * j + t) * source.limbs;
+                    const size_t pitch = size_t(shape.rows.split) * source.limbs;
+                    if (source.aligned) {  // 16-byte rows: eight lanes per row
+                        const uint32_t word = ks * 32 + (lane % 8) * 4, bytes = word < source.limbs ? 16 : 0;
+                        const uint32_t* from = rows + (lane / 8) * pitch + (bytes ? word : 0);
+#pragma unroll
+                        for (uint32_t i = 0; i < 8; ++i) {
+                            const uint32_t row = i * 4 + lane / 8;
+                            cp_async_16_or_zero(to + row * kBlockK + (((lane ^ row) % 8) * 16), from + i * 4 * pitch, bytes);
+                        }
+                    } else {  // a word per lane
+                        const uint32_t word = ks * 32 + lane, bytes = word < source.limbs ? 4 : 0;
+                        const uint32_t* from = rows + (bytes ? word : 0);
+#pragma unroll 8
+                        for (uint32_t i = 0; i < 32; ++i)
+                            cp_async_4(to + i * kBlockK + (((lane / 4) ^ (i & 7)) * 16) + (lane % 4) * 4,
+                                       from + i * pitch, bytes);
+                    }
+                } else {
+                    const uint32_t i = lane / 4;
+                    const uint32_t* from = source.residues + size_t(t) * shape.rows.n_sub + j + i;
+#pragma unroll
+                    for (uint32_t c = 0; c < 8; ++c) {
+                        const uint32_t k = ks * 32 + 4 * c + lane % 4, bytes = k < source.r ? 4 : 0;
+                        const uint32_t* prime = from + size_t(bytes ? k : 0) * source.n;
+#pragma unroll
+                        for (uint32_t g = 0; g < 4; ++g)
+                            cp_async_4(to + (g * 8 + i) * kBlockK + ((c ^ i) * 16) + (lane % 4) * 4, prime + g * 8, bytes);
+                    }
+                }
+                cp_async_commit();
+                if (step + 1 - published == kLoaderDepth) {
+                    cp_async_wait<kLoaderDepth - 1>();
+                    publish();
+                }
+            }
+        }
+        cp_async_wait<0>();
+        while (ok && published < step) publish();
+        if (!ok && lane == 0) {
+            *abort_flag = 1;
+            record_error(shape.status, 512u);
+        }
     } else {
         // ---------------- epilogue: warp w reads TMEM lanes 32*(w%4).. (rows of the tile),
         // columns 128*((w-2)/4)..
@@ -391,9 +573,10 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
         uint32_t local = 0;
         for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++local) {
             const uint32_t acc = local & 1, use = local >> 1;
+            if (kReduce && acc != half) continue;
             uint32_t m_tile, n_tile;
             tile_coords(tile, shape, m_tile, n_tile);
-            const uint32_t row0 = m_tile * kBlockM, col0 = n_tile * kBlockN;
+            const uint32_t row0 = m_tile * kBlockM, col0 = n_tile * shape.block_n;
             bool have = !*abort_flag && mbar_wait(&acc_full[acc], use & 1, shape.limit, abort_flag);
             have = __all_sync(0xffffffffu, have);
             if (!have) {
@@ -405,6 +588,13 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
             }
             fence_after();
             const uint32_t row = row0 + quarter * 32 + lane;  // GEMM row of this lane
+            if constexpr (kReduce) {
+                uint32_t* staging = reinterpret_cast<uint32_t*>(
+                    reinterpret_cast<uint8_t*>(full) + 256 + (warp - 2) * kStagingBytes);
+                reduce_rows(epi.reduce, tmem + acc * kAccColumns + ((quarter * 32) << 16), staging,
+                            shape.rows.coefficient(row - lane), shape.rows.split, &acc_empty[acc], lane);
+                continue;
+            }
             const bool row_ok = row < shape.m;
             uint32_t op = 0, column = 0;
             uint64_t out_row = 0;
@@ -412,10 +602,11 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
                 if (epi.mode == kEpilogueConvert)
                     shape.rows.residue(row, op, column);
                 else
-                    out_row = shape.rows.row(row);
+                    out_row = kSource == kSourceResidues ? shape.rows.coefficient(row) : shape.rows.row(row);
             }
-            const uint32_t t_base = tmem + acc * kAccColumns + half * (kBlockN / 2) + ((quarter * 32) << 16);
-            epilogue_rows(epi, t_base, col0 + half * (kBlockN / 2), shape.columns, row_ok, out_row, op, column);
+            const uint32_t t_base = tmem + acc * kAccColumns + half * (shape.block_n / 2) + ((quarter * 32) << 16);
+            epilogue_rows(epi, t_base, col0 + half * (shape.block_n / 2), shape.columns, shape.block_n / 64, row_ok,
+                          out_row, op, column);
             // every tcgen05.ld of this warp has completed (tmem_load32 waits): release the accumulator
             fence_before();
             __syncwarp();
@@ -746,7 +937,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                     out_row = shape.rows.row(row);
             }
             const uint32_t t_base = tmem + acc * kAccColumns + half * (kBlockN / 2) + ((quarter * 32) << 16);
-            epilogue_rows(epi, t_base, col0 + half * (kBlockN / 2), shape.columns, row_ok, out_row, op, column);
+            epilogue_rows(epi, t_base, col0 + half * (kBlockN / 2), shape.columns, kBlockN / 64, row_ok,
+                          out_row, op, column);
             fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(release + acc * sizeof(uint64_t));
@@ -781,6 +973,32 @@ EncodeTiled encoder() {
             fn = reinterpret_cast<EncodeTiled>(ptr);
     }
     return fn;
+}
+
+// B (columns rows of k_bytes): boxes of 256 rows, and of 128.
+bool encode_b(EncodeTiled encode, TensorGemmPlan& plan, const uint8_t* b, uint32_t columns, uint32_t k_bytes,
+              std::string& why) {
+    const cuuint32_t unit[2] = {1, 1};
+    const cuuint64_t b_dims[2] = {k_bytes, columns};
+    const cuuint64_t b_strides[1] = {k_bytes};
+    const cuuint32_t b_box[2] = {kBlockK, kBlockN};
+    CUresult rb = encode(&plan.b_map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint8_t*>(b), b_dims, b_strides,
+                         b_box, unit, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    const cuuint32_t b_half_box[2] = {kBlockK, kPairBlockN / 2};
+    CUresult rh = encode(&plan.b_map_half, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint8_t*>(b), b_dims,
+                         b_strides, b_half_box, unit, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (rb == CUDA_SUCCESS && rh == CUDA_SUCCESS) return true;
+    why = "tensor map encoding failed";
+    return false;
+}
+
+uint32_t device_sm_count() {
+    int device = 0, sms = 0;
+    cudaGetDevice(&device);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    return sms > 0 ? uint32_t(sms) : 148;
 }
 
 }  // namespace
@@ -832,21 +1050,13 @@ bool prepare_gemm_tensor(TensorGemmPlan& plan, const uint8_t* a, uint64_t a_pitc
     CUresult ra = encode(&plan.a_map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint8_t*>(a), a_dims, a_strides,
                          a_box, unit, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                          CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    const cuuint64_t b_dims[2] = {k_bytes, columns};
-    const cuuint64_t b_strides[1] = {k_bytes};
-    const cuuint32_t b_box[2] = {kBlockK, kBlockN};
-    CUresult rb = encode(&plan.b_map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint8_t*>(b), b_dims, b_strides,
-                         b_box, unit, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    const cuuint32_t b_half_box[2] = {kBlockK, kPairBlockN / 2};
-    CUresult rh = encode(&plan.b_map_half, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint8_t*>(b), b_dims,
-                         b_strides, b_half_box, unit, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (ra != CUDA_SUCCESS || rb != CUDA_SUCCESS || rh != CUDA_SUCCESS) {
+    if (!encode_b(encode, plan, b, columns, k_bytes, why)) return false;
+    if (ra != CUDA_SUCCESS) {
         why = "tensor map encoding failed";
         return false;
     }
-    if (cudaFuncSetAttribute(gemm_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemBytes)) !=
+    if (cudaFuncSetAttribute(gemm_tc_kernel<kSourceTma, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             int(kSmemBytes)) !=
             cudaSuccess ||
         cudaFuncSetAttribute(gemm_tc_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              int(kPairSmemBytes)) != cudaSuccess) {
@@ -872,10 +1082,7 @@ bool prepare_gemm_tensor(TensorGemmPlan& plan, const uint8_t* a, uint64_t a_pitc
         }
         plan.tile_counter = static_cast<uint32_t*>(counter);
     }
-    int device = 0, sms = 0;
-    cudaGetDevice(&device);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    plan.sm_count = sms > 0 ? uint32_t(sms) : 148;
+    plan.sm_count = device_sm_count();
     // CTA pairs need 256-row slabs; NEGACYCLIC_GEMM_PAIRS=0 selects the single-CTA kernel
     const char* pairs_env = getenv("NEGACYCLIC_GEMM_PAIRS");
     plan.narrow = columns < kBlockN;
@@ -905,7 +1112,7 @@ void launch_gemm_tensor(const TensorGemmPlan& plan, const Epilogue& epilogue, cu
     TileShape shape{m,      plan.columns,       plan.k_tiles,
                     m_tiles, plan.n_tiles,      uint32_t(group),
                     rows,    plan.tile_counter, epilogue.status,
-                    options.limit_cycles > 0 ? options.limit_cycles : kDefaultLimitCycles, options.withheld};
+                    options.limit_cycles > 0 ? options.limit_cycles : kDefaultLimitCycles, options.withheld, kBlockN};
     const uint32_t tiles = m_tiles * plan.n_tiles;
     if (pairs) {
         const uint32_t max_pairs = plan.sm_count / 2;
@@ -916,7 +1123,76 @@ void launch_gemm_tensor(const TensorGemmPlan& plan, const Epilogue& epilogue, cu
         return;
     }
     const uint32_t grid = tiles < plan.sm_count ? tiles : plan.sm_count;
-    launch_chained(gemm_tc_kernel, grid, kThreads, kSmemBytes, stream, plan.a_map, plan.b_map, shape, epilogue);
+    launch_chained(gemm_tc_kernel<kSourceTma, false>, grid, kThreads, kSmemBytes, stream, plan.a_map, plan.b_map, shape,
+                   GatherSource{}, epilogue);
+}
+
+bool prepare_gemm_gather(TensorGemmPlan& plan, RowMap rows, uint32_t m, const uint8_t* b, uint32_t columns,
+                         uint32_t k_bytes, std::string& why) {
+    plan.ready = false;
+    EncodeTiled encode = encoder();
+    if (!encode) {
+        why = "cuTensorMapEncodeTiled unavailable";
+        return false;
+    }
+    if (k_bytes < kBlockK || k_bytes % kBlockK || reinterpret_cast<uintptr_t>(b) % 16) {
+        why = "K must be whole steps of 128 bytes";
+        return false;
+    }
+    if (rows.mode != kRowsSplit || rows.n_sub % kBlockM) {
+        why = "fewer than 128 rows per transform";
+        return false;
+    }
+    if (!encode_b(encode, plan, b, columns, k_bytes, why)) return false;
+    if (cudaFuncSetAttribute(gemm_tc_kernel<kSourceRows, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             int(kSmemBytes)) != cudaSuccess ||
+        cudaFuncSetAttribute(gemm_tc_kernel<kSourceResidues, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             int(kSmemBytes)) != cudaSuccess ||
+        cudaFuncSetAttribute(gemm_tc_kernel<kSourceResidues, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             int(kReduceSmemBytes)) != cudaSuccess) {
+        cudaGetLastError();
+        why = "cannot reserve shared memory";
+        return false;
+    }
+    plan.m = m;
+    plan.columns = columns;
+    plan.k_bytes = k_bytes;
+    plan.k_tiles = k_bytes / kBlockK;
+    plan.rows = rows;
+    plan.a_tile_bytes = uint64_t(kBlockM) * k_bytes;
+    plan.error_flag = tensor_gemm_error_flag();
+    plan.sm_count = device_sm_count();
+    plan.pairs = false;
+    plan.ready = true;
+    return true;
+}
+
+void launch_gemm_gather(const TensorGemmPlan& plan, const GatherSource& source, const Epilogue& epilogue,
+                        cudaStream_t stream, const RowMap& rows, uint32_t m) {
+    const uint32_t m_tiles = m / kBlockM;
+    // 128-column tiles where they leave less of the last wave empty, or cover all columns
+    auto cost = [&](uint32_t block_n) {
+        const uint64_t tiles = uint64_t(m_tiles) * ((plan.columns + block_n - 1) / block_n);
+        return (tiles + plan.sm_count - 1) / plan.sm_count * block_n;
+    };
+    const bool reduce = epilogue.mode == kEpilogueReduce;  // needs all columns in one tile
+    const uint32_t block_n = (reduce ? plan.columns <= 128 : cost(128) < cost(256)) ? 128 : 256;
+    const uint32_t n_tiles = (plan.columns + block_n - 1) / block_n, tiles = m_tiles * n_tiles;
+    uint64_t group = (48ull << 20) / plan.a_tile_bytes;
+    group = group < 4 ? 4 : (group > 64 ? 64 : group);
+    const TileShape shape{m,    plan.columns, plan.k_tiles,    m_tiles,             n_tiles,         uint32_t(group),
+                          rows, nullptr,      epilogue.status, kDefaultLimitCycles, kNoWithheldStep, block_n};
+    const uint32_t grid = tiles < plan.sm_count ? tiles : plan.sm_count;
+    const CUtensorMap& b_map = block_n == 128 ? plan.b_map_half : plan.b_map;
+    if (source.kind == kSourceRows)
+        launch_chained(gemm_tc_kernel<kSourceRows, false>, grid, kGatherThreads, kSmemBytes, stream, b_map, b_map, shape,
+                       source, epilogue);
+    else if (reduce)
+        launch_chained(gemm_tc_kernel<kSourceResidues, true>, grid, kGatherThreads, kReduceSmemBytes, stream, b_map, b_map,
+                       shape, source, epilogue);
+    else
+        launch_chained(gemm_tc_kernel<kSourceResidues, false>, grid, kGatherThreads, kSmemBytes, stream, b_map, b_map,
+                       shape, source, epilogue);
 }
 
 }  // namespace negacyclic

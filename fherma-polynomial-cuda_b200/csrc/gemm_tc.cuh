@@ -26,6 +26,30 @@ struct TensorGemmPlan {
     bool ready = false;
 };
 
+// Where the single-CTA kernel's A tiles come from.
+//  kSourceTma:      operand rows of k_bytes in memory, through the plan's tensor map.
+//  kSourceRows:     the unpadded operands: row m is coefficient i = s*j + t of operand op, L words
+//                   (zeros above) at rows[op] + i*L.
+//  kSourceResidues: the residues: byte 4k + d of row m is byte d of residues[k*n + t*N' + j], k < r
+//                   (zeros above).
+enum GemmSource : int { kSourceTma = 0, kSourceRows = 1, kSourceResidues = 2 };
+
+struct GatherSource {
+    GemmSource kind;
+    const uint32_t* rows[2];
+    uint32_t limbs;
+    bool aligned;  // both operands start on 16 bytes and L is a multiple of 4
+    const uint32_t* residues;
+    uint32_t r, n;
+};
+
+// A GEMM whose A operand is gathered by warps (GatherSource) instead of read by TMA: `rows` is the
+// split row map of the whole shape, k_bytes a multiple of 128. False (with `why`) outside that.
+bool prepare_gemm_gather(TensorGemmPlan& plan, RowMap rows, uint32_t m, const uint8_t* b, uint32_t columns,
+                         uint32_t k_bytes, std::string& why);
+void launch_gemm_gather(const TensorGemmPlan& plan, const GatherSource& source, const Epilogue& epilogue,
+                        cudaStream_t stream, const RowMap& rows, uint32_t m);
+
 // Builds the tensor maps; false (with `why`) when the shape is outside what the
 // kernel handles (then the SIMT kernel is used).
 bool prepare_gemm_tensor(TensorGemmPlan& plan, const uint8_t* a, uint64_t a_pitch, RowMap rows, uint32_t m,

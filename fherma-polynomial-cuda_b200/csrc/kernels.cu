@@ -12,6 +12,7 @@
 #include "kernels.cuh"
 
 #include "launch.cuh"
+#include "reduce.cuh"
 
 #include <algorithm>
 #include <type_traits>
@@ -612,19 +613,7 @@ __global__ void __launch_bounds__(256) transpose_kernel(const uint32_t* __restri
 }
 
 // ---------------------------------------------------------------------------
-// CRT quotient, carries and reduction mod q: one thread per coefficient.
-//
-// The CRT word sums split cleanly: words [0, L+2) are a carry-save form of
-// T = sum v_k M_k (< 2^(32(L+2)), so nothing carries out of them), words
-// L+2..L+4 a carry-save form of D = sum v_k floor(2^64/p_k). Hence
-//   K  = (D + 2^63) >> 64 straight from three word sums,
-//   T' = T + K R (R = -P mod q), T' = x (mod q), T' < 2^48 q,
-//   c  = T' - quotient q, then at most three q's off.
-// The quotient is known before the carries are: Barrett needs the 128 bits of T' from top_shift
-// up, and the words below the window carry less than 2^26 into it. Starting the window two words
-// lower bounds the missing carry by one unit of the window's lowest bit, which can only make the
-// quotient smaller, by less than 2^-62 before the floor. So one pass over the row, lowest word
-// first, forms d[w] + K R[w] - quotient q and its carries at once.
+// CRT quotient, carries and reduction mod q (csrc/reduce.cuh): one thread per coefficient.
 //
 // What bounds it: reading 8 (L+5) and writing 4 L bytes per coefficient. A thread's carry chain is
 // three dependent instructions per word, and 32 rows advance per warp instruction; a warp per
@@ -645,94 +634,6 @@ struct ReduceSlot {
     static constexpr uint32_t kBytes = 32 * kPitch + kChunk * 8;
 };
 constexpr uint32_t kReduceSlots = 3;
-
-__device__ __forceinline__ void cp_async_16(uint32_t smem, const void* global) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem), "l"(global) : "memory");
-}
-
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-
-template <int kPending>
-__device__ __forceinline__ void cp_async_wait() {
-    asm volatile("cp.async.wait_group %0;" ::"n"(kPending) : "memory");
-}
-
-struct RowQuotient {
-    uint32_t k;         // CRT quotient K < 2r
-    uint32_t low, high; // Barrett quotient of T' by q
-};
-
-// K and the Barrett quotient of one row of word sums.
-__device__ __forceinline__ RowQuotient row_quotient(const uint64_t* d, const ReduceParams& prm) {
-    const uint32_t limbs = prm.limbs;
-    const int32_t tlen = int32_t(limbs) + 2;
-    // K = (D + 2^63) >> 64, D = d[L+2] + d[L+3] 2^32 + d[L+4] 2^64 (each word sum < 2^56)
-    const uint64_t x0 = d[limbs + 2], x1 = d[limbs + 3], x2 = d[limbs + 4];
-    const uint64_t low = x0 + (x1 << 32);
-    const uint64_t high = (x1 >> 32) + x2 + (low < x0 ? 1 : 0);  // D = high 2^64 + low
-    const uint32_t k = uint32_t(high + ((low + (1ull << 63)) < low ? 1 : 0));
-    // T' words at ws .. ws+4 (ws = floor(top_shift / 32), possibly negative), with the carry of the
-    // two words below
-    const int32_t ws = prm.top_shift >> 5;
-    const uint32_t offset = uint32_t(prm.top_shift) & 31u;
-    uint32_t z[5];
-    uint64_t acc = 0;
-#pragma unroll
-    for (int32_t j = -2; j < 5; ++j) {
-        const int32_t w = ws + j;
-        if (w >= 0 && w < tlen) acc += d[w] + uint64_t(k) * prm.minus_p[w];
-        if (j >= 0) z[j] = uint32_t(acc);
-        acc >>= 32;
-    }
-    const uint64_t tl = uint64_t(__funnelshift_r(z[0], z[1], offset)) |
-                        (uint64_t(__funnelshift_r(z[1], z[2], offset)) << 32);
-    const uint64_t th = uint64_t(__funnelshift_r(z[2], z[3], offset)) |
-                        (uint64_t(__funnelshift_r(z[3], z[4], offset)) << 32);
-    const uint64_t prod_l_hi = __umul64hi(tl, prm.mu_low);
-    const uint64_t prod_h_lo = th * prm.mu_low, prod_h_hi = __umul64hi(th, prm.mu_low);
-    const uint64_t word1 = prod_l_hi + prod_h_lo;
-    const uint64_t word2 = prod_h_hi + (word1 < prod_l_hi ? 1 : 0);
-    const uint64_t quotient = th + word2 + ((tl + word1 < tl) ? 1 : 0);  // < 2^48
-    return RowQuotient{k, uint32_t(quotient), uint32_t(quotient >> 32)};
-}
-
-// Takes q off a row (limbs words in global memory, `over` above them) while it is not below q;
-// returns false if more than three subtractions were needed.
-__device__ __noinline__ bool correct_row(uint32_t* row, uint32_t over, const uint32_t* __restrict__ q,
-                                         uint32_t limbs) {
-    for (int corrections = 0;; ++corrections) {
-        if (over == 0) {
-            uint32_t w = limbs;
-            while (w > 0 && row[w - 1] == q[w - 1]) --w;
-            if (w > 0 && row[w - 1] < q[w - 1]) return true;
-        }
-        if (corrections == 3) return false;
-        uint32_t borrow = 0;
-        for (uint32_t w = 0; w < limbs; ++w) {
-            const uint64_t t = uint64_t(row[w]) - q[w] - borrow;
-            row[w] = uint32_t(t);
-            borrow = uint32_t(t >> 63);
-        }
-        over -= borrow;
-    }
-}
-
-// Running state of one row's pass.
-struct RowState {
-    int64_t carry;   // signed carry into the next word
-    uint64_t below;  // hi(ql q[w-1]) + qh q[w-1], subtracted at word w
-};
-
-// Word w of T' - quotient q: d + K R - lo(ql q) - below + carry. d < 2^56, K R < 2^46 and
-// below < 2^49, so the sum stays within int64.
-__device__ __forceinline__ uint32_t row_word(RowState& st, const RowQuotient& f, uint64_t d, uint32_t r, uint32_t q) {
-    const uint64_t a = uint64_t(f.low) * q;
-    const int64_t y = int64_t(d + uint64_t(f.k) * r) - int64_t(uint32_t(a)) - int64_t(st.below);
-    st.below = (a >> 32) + uint64_t(f.high) * q;
-    const int64_t z = y + st.carry;
-    st.carry = z >> 32;
-    return uint32_t(z);
-}
 
 template <uint32_t kChunk>
 __global__ void reduce_kernel(ReduceParams prm) {
@@ -774,10 +675,16 @@ __global__ void reduce_kernel(ReduceParams prm) {
     };
     for (uint32_t c = 0; c < kReduceSlots; ++c) fetch(c);
 
-    const RowQuotient f = row_quotient(d0 + size_t(min(lane, rows - 1)) * prm.dots_stride, prm);
-    RowState st{0, 0};
-    const uint32_t q_words = prm.q_words;  // significant words of q
-    uint32_t over = 0, top1 = 0, top0 = 0;  // words at and above q_words (or-ed), and the two below
+    const uint64_t* d = d0 + size_t(min(lane, rows - 1)) * prm.dots_stride;
+    const uint64_t x[3] = {d[limbs + 2], d[limbs + 3], d[limbs + 4]};
+    uint64_t window[kWindow];
+#pragma unroll
+    for (int j = 0; j < kWindow; ++j) {
+        uint32_t w;
+        window[j] = window_word(prm, j, w) ? d[w] : 0;
+    }
+    const RowQuotient f = row_quotient(x, window, prm);
+    RowState st;
     for (uint32_t c = 0; c < chunks; ++c) {
         cp_async_wait<kReduceSlots - 1>();
         __syncwarp();
@@ -789,43 +696,25 @@ __global__ void reduce_kernel(ReduceParams prm) {
 #pragma unroll 1
         for (uint32_t part = 0; part < kChunk; part += 16) {  // 16 words at a time through registers
             if (base + part >= tlen) break;
-            ulonglong2 d[8];
+            uint64_t sums[16];
             uint4 q[4], r[4];
 #pragma unroll
             for (uint32_t g = 0; g < 4; ++g) {
                 q[g] = q4[part / 4 + g];
                 r[g] = r4[part / 4 + g];
-                d[2 * g] = *reinterpret_cast<const ulonglong2*>(own + part * 8 + g * 32);
-                d[2 * g + 1] = *reinterpret_cast<const ulonglong2*>(own + part * 8 + g * 32 + 16);
             }
-            if (base + part + 16 > tlen) {  // the row's end: words from L+2 up are not part of T
 #pragma unroll
-                for (uint32_t g = 0; g < 8; ++g) {
-                    if (base + part + 2 * g >= tlen) d[g].x = 0;
-                    if (base + part + 2 * g + 1 >= tlen) d[g].y = 0;
-                }
+            for (uint32_t g = 0; g < 8; ++g) {
+                const ulonglong2 pair = *reinterpret_cast<const ulonglong2*>(own + part * 8 + g * 16);
+                sums[2 * g] = pair.x;
+                sums[2 * g + 1] = pair.y;
             }
             uint32_t o[16];
-#pragma unroll
-            for (uint32_t g = 0; g < 4; ++g) {
-                o[4 * g] = row_word(st, f, d[2 * g].x, r[g].x, q[g].x);
-                o[4 * g + 1] = row_word(st, f, d[2 * g].y, r[g].y, q[g].y);
-                o[4 * g + 2] = row_word(st, f, d[2 * g + 1].x, r[g].z, q[g].z);
-                o[4 * g + 3] = row_word(st, f, d[2 * g + 1].y, r[g].w, q[g].w);
-            }
+            st.words16(f, sums, q, r, base + part, prm, o);
 #pragma unroll
             for (uint32_t g = 0; g < 4; ++g)  // over words that this thread has already read
                 *reinterpret_cast<uint4*>(own + part * 4 + g * 16) =
                     make_uint4(o[4 * g], o[4 * g + 1], o[4 * g + 2], o[4 * g + 3]);
-            if (base + part + 16 + 2 > q_words) {  // some of the top words
-#pragma unroll
-                for (uint32_t i = 0; i < 16; ++i) {
-                    const uint32_t w = base + part + i;
-                    if (w + 2 == q_words) top0 = o[i];
-                    if (w + 1 == q_words) top1 = o[i];
-                    if (w >= q_words) over |= o[i];
-                }
-            }
         }
         __syncwarp();
         if constexpr (kChunk == 16) {
@@ -852,13 +741,7 @@ __global__ void reduce_kernel(ReduceParams prm) {
         __syncwarp();
         fetch(c + kReduceSlots);
     }
-    // a result whose top two words are below q's is canonical; the rest compare whole rows
-    const uint64_t top = (uint64_t(top1) << 32) | top0, q_top = (uint64_t(prm.q[q_words - 1]) << 32) |
-                                                                (q_words >= 2 ? prm.q[q_words - 2] : 0u);
-    if (lane < rows && (over != 0 || top >= q_top)) {
-        uint32_t* row = prm.out + size_t(row0 + lane) * limbs;
-        if (!correct_row(row, q_words < limbs ? 0u : over, prm.q, limbs)) atomicOr(prm.error_flag, 1u);
-    }
+    if (lane < rows) st.finish(prm.out + size_t(row0 + lane) * limbs, prm);
 }
 
 uint32_t log2_u32(uint32_t x) { return x ? 31 - __builtin_clz(x) : 0; }

@@ -46,6 +46,12 @@ struct RowMap {
         decompose(m, op, t, j);
         return uint64_t(op) * n + uint64_t(t) * n_sub + j;
     }
+    // coefficient of GEMM row m (split rows)
+    __device__ __forceinline__ uint32_t coefficient(uint32_t m) const {
+        uint32_t op, t, j;
+        decompose(m, op, t, j);
+        return split * j + t;
+    }
     // conversion output position of GEMM row m: residue row `op`, column t*N' + j
     __device__ __forceinline__ void residue(uint32_t m, uint32_t& op, uint32_t& column) const {
         uint32_t t, j;
@@ -56,7 +62,19 @@ struct RowMap {
 
 // Epilogues of the byte-sliced GEMM. Output column group g (4 consecutive
 // columns 4g..4g+3) of row m holds int32 dots G_d; S = sum_d G_d 256^d.
-enum EpilogueMode : int { kEpilogueRaw = 0, kEpilogueConvert = 1, kEpilogueCrt = 2 };
+enum EpilogueMode : int { kEpilogueRaw = 0, kEpilogueConvert = 1, kEpilogueCrt = 2, kEpilogueReduce = 3 };
+
+struct ReduceParams {
+    const uint64_t* dots;     // [n][dots_stride], words used
+    uint32_t* out;            // [n][limbs]
+    const uint32_t* q;        // [limbs], then zeros up to reduce_table_words(limbs)
+    const uint32_t* minus_p;  // [limbs]  (-P) mod q, then zeros likewise
+    uint32_t n, limbs, dots_stride;
+    uint32_t q_words;         // significant words of q
+    int32_t top_shift;
+    uint64_t mu_low;
+    uint32_t* error_flag;     // set nonzero if a coefficient needed more corrections than proven
+};
 
 struct Epilogue {
     int mode;
@@ -69,8 +87,12 @@ struct Epilogue {
     uint32_t r, n;
     // crt: dots[row * dots_stride + g] = S (u64), g < words, row = the operand row of GEMM row m;
     //      dots_stride is words rounded up to a multiple of 8 (64-byte rows)
+    // (split rows: row = the coefficient of GEMM row m)
     uint64_t* dots;
     uint32_t words, dots_stride;
+    // reduce: a tile holds all of a row's word sums; coefficient i of GEMM row m is reduced mod q into
+    // reduce.out[i * limbs ..] (reduce.dots is not used)
+    ReduceParams reduce;
     // every mode: the product's status word (NEGACYCLIC_STATUS_*); the tensor-core kernels set
     // NEGACYCLIC_STATUS_GEMM_MASK bits in it when a pipeline wait gives up (nullptr: none kept)
     uint32_t* status;
@@ -111,17 +133,6 @@ void launch_ntt_inverse(uint32_t* residues, const DevicePrime* primes, const uin
 void launch_transpose(const uint32_t* residues, uint32_t* crt_in, uint32_t r, uint32_t padded_r,
                       uint32_t n, uint32_t split, uint32_t j_first, uint32_t j_count, cudaStream_t stream);
 
-struct ReduceParams {
-    const uint64_t* dots;     // [n][dots_stride], words used
-    uint32_t* out;            // [n][limbs]
-    const uint32_t* q;        // [limbs], then zeros up to reduce_table_words(limbs)
-    const uint32_t* minus_p;  // [limbs]  (-P) mod q, then zeros likewise
-    uint32_t n, limbs, dots_stride;
-    uint32_t q_words;         // significant words of q
-    int32_t top_shift;
-    uint64_t mu_low;
-    uint32_t* error_flag;     // set nonzero if a coefficient needed more corrections than proven
-};
 // Words the tables of launch_reduce hold: whole chunks of 64 covering L + 2 words.
 constexpr uint32_t reduce_table_words(uint32_t limbs) { return (limbs + 2 + 63) / 64 * 64; }
 void launch_reduce(const ReduceParams& params, cudaStream_t stream);

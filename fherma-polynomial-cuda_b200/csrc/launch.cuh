@@ -1,3 +1,5 @@
+// Asynchronous copies into shared memory, and chained launches.
+//
 // Chained launches: a product's kernels follow one another on a stream with programmatic dependent
 // launch, so that a kernel's blocks are placed, and its prologue runs, while the kernel before it
 // finishes.
@@ -20,6 +22,17 @@ __device__ __forceinline__ void chain_release() { asm volatile("griddepcontrol.l
 __device__ __forceinline__ void chain_enter() {
     chain_wait();
     chain_release();
+}
+
+__device__ __forceinline__ void cp_async_16(uint32_t smem, const void* global) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem), "l"(global) : "memory");
+}
+
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+
+template <int kPending>
+__device__ __forceinline__ void cp_async_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kPending) : "memory");
 }
 
 template <class... Params, class... Args>

@@ -65,9 +65,10 @@ TensorGemmOptions product_gemm(bool counter_cleared) {
 }
 
 // conversion GEMM over the coefficients s*j + t, t in [t_first, t_first + t_count),
-// j in [first_j, first_j + span), of operands [op_first, op_first + op_count)
-void enqueue_convert(negacyclic_plan& s, uint32_t t_first, uint32_t t_count, uint32_t first_j, uint32_t span,
-                     cudaStream_t stream, uint32_t op_first = 0, uint32_t op_count = 2,
+// j in [first_j, first_j + span), of operands [op_first, op_first + op_count). `a` and `b` are the
+// unpadded operands, which a plan with convert_rows reads; others read s.operands.
+void enqueue_convert(negacyclic_plan& s, const uint32_t* a, const uint32_t* b, uint32_t t_first, uint32_t t_count,
+                     uint32_t first_j, uint32_t span, cudaStream_t stream, uint32_t op_first = 0, uint32_t op_count = 2,
                      bool counter_cleared = false) {
     const HostPlan& h = s.host;
     Epilogue convert{};
@@ -79,30 +80,24 @@ void enqueue_convert(negacyclic_plan& s, uint32_t t_first, uint32_t t_count, uin
     convert.status = s.status;
     const RowMap rows = RowMap::split_rows(h.n, h.n_sub, h.split, first_j, span, t_first, t_count, op_first);
     const uint32_t m = op_count * t_count * span;
-    if (s.convert_engine == NEGACYCLIC_GEMM_TENSOR && gemm_tensor_accepts(s.convert_gemm, rows, m))
+    if (s.convert_rows.ready) {  // its callers pass whole tiles (gather_span)
+        GatherSource source{};
+        source.kind = kSourceRows;
+        source.rows[0] = a;
+        source.rows[1] = b;
+        source.limbs = h.limbs;
+        source.aligned = h.limbs % 4 == 0 && (reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) % 16 == 0;
+        launch_gemm_gather(s.convert_rows, source, convert, stream, rows, m);
+    } else if (s.convert_engine == NEGACYCLIC_GEMM_TENSOR && gemm_tensor_accepts(s.convert_gemm, rows, m)) {
         launch_gemm_tensor(s.convert_gemm, convert, stream, rows, m, product_gemm(counter_cleared));
-    else
+    } else {
         launch_gemm_simt(reinterpret_cast<const uint8_t*>(s.operands), uint64_t(s.padded_limbs) * 4, rows, m,
                          s.convert_weights, 4 * s.padded_r, s.k_convert, convert, stream);
+    }
 }
 
-// CRT GEMM and reduction of coefficients [first, first + count) into d_c (rows indexed from 0 = coefficient 0)
-void enqueue_output(negacyclic_plan& s, uint32_t first, uint32_t count, uint32_t* d_c, cudaStream_t stream,
-                    cudaEvent_t between = nullptr, bool counter_cleared = false) {
+ReduceParams reduce_params(const negacyclic_plan& s, uint32_t first, uint32_t count, uint32_t* d_c) {
     const HostPlan& h = s.host;
-    Epilogue crt{};
-    crt.mode = kEpilogueCrt;
-    crt.dots = s.dots;
-    crt.words = h.words;
-    crt.dots_stride = s.dots_stride;
-    crt.status = s.status;
-    const RowMap rows = RowMap::linear(first);
-    if (s.crt_engine == NEGACYCLIC_GEMM_TENSOR && gemm_tensor_accepts(s.crt_gemm, rows, count))
-        launch_gemm_tensor(s.crt_gemm, crt, stream, rows, count, product_gemm(counter_cleared));
-    else
-        launch_gemm_simt(reinterpret_cast<const uint8_t*>(s.crt_in), uint64_t(s.padded_r) * 4, rows, count,
-                         s.crt_weights, s.crt_columns, s.k_crt, crt, stream);
-    if (between) check(cudaEventRecord(between, stream), "cudaEventRecord");
     ReduceParams reduce{};
     reduce.dots = s.dots + size_t(first) * s.dots_stride;
     reduce.dots_stride = s.dots_stride;
@@ -115,7 +110,60 @@ void enqueue_output(negacyclic_plan& s, uint32_t first, uint32_t count, uint32_t
     reduce.top_shift = h.top_shift;
     reduce.mu_low = h.mu_low;
     reduce.error_flag = s.status;
-    launch_reduce(reduce, stream);
+    return reduce;
+}
+
+Epilogue crt_epilogue(const negacyclic_plan& s) {
+    Epilogue crt{};
+    crt.mode = kEpilogueCrt;
+    crt.dots = s.dots;
+    crt.words = s.host.words;
+    crt.dots_stride = s.dots_stride;
+    crt.status = s.status;
+    return crt;
+}
+
+// word sums of coefficients [first, first + count) from the CRT inputs
+void enqueue_crt_sums(negacyclic_plan& s, uint32_t first, uint32_t count, cudaStream_t stream, bool counter_cleared) {
+    const Epilogue crt = crt_epilogue(s);
+    const RowMap rows = RowMap::linear(first);
+    if (s.crt_engine == NEGACYCLIC_GEMM_TENSOR && gemm_tensor_accepts(s.crt_gemm, rows, count))
+        launch_gemm_tensor(s.crt_gemm, crt, stream, rows, count, product_gemm(counter_cleared));
+    else
+        launch_gemm_simt(reinterpret_cast<const uint8_t*>(s.crt_in), uint64_t(s.padded_r) * 4, rows, count,
+                         s.crt_weights, s.crt_columns, s.k_crt, crt, stream);
+}
+
+// Whether coefficients [first, first + count) are whole 128-row tiles of every transform.
+bool gather_span(const negacyclic_plan& s, uint32_t first, uint32_t count) {
+    const uint32_t split = s.host.split;
+    return first % split == 0 && count % split == 0 && count / split % 128 == 0;
+}
+
+// CRT GEMM and reduction of coefficients [first, first + count) into d_c (rows indexed from 0 = coefficient 0).
+// With `gather` (crt_gather, whole tiles: gather_span) the CRT inputs come from the residues, else
+// from s.crt_in.
+void enqueue_output(negacyclic_plan& s, uint32_t first, uint32_t count, uint32_t* d_c, cudaStream_t stream, bool gather,
+                    cudaEvent_t between = nullptr, bool counter_cleared = false) {
+    const HostPlan& h = s.host;
+    if (gather) {
+        GatherSource source{};
+        source.kind = kSourceResidues;
+        source.residues = s.residues;
+        source.r = s.r;
+        source.n = h.n;
+        Epilogue crt = crt_epilogue(s);
+        if (s.crt_reduces) {
+            crt.mode = kEpilogueReduce;
+            crt.reduce = reduce_params(s, 0, h.n, d_c);
+        }
+        const RowMap rows = RowMap::split_rows(h.n, h.n_sub, h.split, first / h.split, count / h.split, 0, h.split);
+        launch_gemm_gather(s.crt_gather, source, crt, stream, rows, count);
+    } else {
+        enqueue_crt_sums(s, first, count, stream, counter_cleared);
+    }
+    if (between) check(cudaEventRecord(between, stream), "cudaEventRecord");
+    if (!gather || !s.crt_reduces) launch_reduce(reduce_params(s, first, count, d_c), stream);
 }
 
 // forward NTTs, pointwise products, inverse NTTs, transpose, all transforms
@@ -133,18 +181,27 @@ void enqueue_middle(negacyclic_plan& s, cudaStream_t stream, cudaEvent_t* marks)
     mark();
     launch_ntt_inverse(s.residues, s.primes, s.inv, s.r, n, h.n_sub, 0, h.split, stream);
     mark();
-    launch_transpose(s.residues, s.crt_in, s.r, s.padded_r, n, h.split, 0, h.n_sub, stream);
+    if (!s.crt_gather.ready) launch_transpose(s.residues, s.crt_in, s.r, s.padded_r, n, h.split, 0, h.n_sub, stream);
     mark();
 }
 
-// Enqueues the whole product on `stream`. `operands` already holds the padded inputs.
+// Pads the operands on `stream`, where the conversion reads them padded.
+void enqueue_pad(negacyclic_plan& s, const uint32_t* d_a, const uint32_t* d_b, cudaStream_t stream) {
+    if (s.convert_rows.ready) return;
+    launch_pad_operands(d_a, d_b, s.operands, s.host.n, s.host.limbs, s.padded_limbs, s.host.split, s.tile_counters,
+                        stream);
+}
+
+// Enqueues the whole product after enqueue_pad on `stream`.
 // `marks` (optional, kStages events) are recorded after each stage.
-void enqueue_product(negacyclic_plan& s, uint32_t* d_c, cudaStream_t stream, cudaEvent_t* marks = nullptr) {
+void enqueue_product(negacyclic_plan& s, const uint32_t* d_a, const uint32_t* d_b, uint32_t* d_c, cudaStream_t stream,
+                     cudaEvent_t* marks = nullptr) {
     const HostPlan& h = s.host;
-    enqueue_convert(s, 0, h.split, 0, h.n_sub, stream, 0, 2, true);  // the pad kernel cleared the counters
+    const bool cleared = !s.convert_rows.ready;  // the pad kernel cleared the tile counters
+    enqueue_convert(s, d_a, d_b, 0, h.split, 0, h.n_sub, stream, 0, 2, cleared);
     if (marks) check(cudaEventRecord(marks[0], stream), "cudaEventRecord");
     enqueue_middle(s, stream, marks ? marks + 1 : nullptr);
-    enqueue_output(s, 0, h.n, d_c, stream, marks ? marks[5] : nullptr, true);
+    enqueue_output(s, 0, h.n, d_c, stream, s.crt_gather.ready, marks ? marks[5] : nullptr, cleared);
     if (marks) check(cudaEventRecord(marks[6], stream), "cudaEventRecord");
     check(cudaGetLastError(), "product kernels");
 }
@@ -173,6 +230,27 @@ WorkLayout work_layout(const negacyclic_plan& s) {
     at = align(at + kTileCounters * 4);
     w.total = at;
     return w;
+}
+
+// K steps (of 128 bytes) up to which the GEMMs gather their A tiles; every column tile gathers them
+// again, so the pad and transpose kernels win beyond. Product, us, gathered against not. Conversion:
+// 91.8 / 105.9 at one step (N=65536, L=28), 164.9 / 177.8 at two (L=55), 332 / 329 at three (L=96),
+// 468 / 452 at four (L=128). CRT GEMM without the reduction: 45.9 / 47.1 at seven steps (N=4096,
+// L=94), 66.7 / 69.7 (N=8192), 324 / 322 (N=65536); 89.1 / 85.8 at nine (N=8192, L=128). With the
+// reduction in its epilogue: 59.1 / 70.0 (N=32768, L=28), 165.5 / 183.0 (N=65536, L=55).
+constexpr uint32_t kGatherRowSteps = 2, kGatherResidueSteps = 8;
+
+// The gathering GEMMs of a plan: they read tables only, so they do not depend on the work space.
+void prepare_gather(negacyclic_plan& s) {
+    const HostPlan& h = s.host;
+    std::string why;
+    const RowMap both = RowMap::split_rows(h.n, h.n_sub, h.split, 0, h.n_sub, 0, h.split);
+    // (rows that the host path sends in transform order arrive permuted, and are padded)
+    if (s.k_convert <= kGatherRowSteps * 128 && !wide_rows(ChunkShape{h.n, h.n_sub, h.split, h.limbs, s.chunks}))
+        prepare_gemm_gather(s.convert_rows, both, 2 * h.n, s.convert_weights, 4 * s.r, s.k_convert, why);
+    if (s.k_crt <= kGatherResidueSteps * 128)
+        prepare_gemm_gather(s.crt_gather, both, h.n, s.crt_weights, 4 * h.words, s.k_crt, why);
+    s.crt_reduces = s.crt_gather.ready && 4 * h.words <= 256;
 }
 
 constexpr char kFewColumns[] = "fewer than 256 output columns";
@@ -221,9 +299,8 @@ std::string bind_work(negacyclic_plan& s, void* arena) {
 
 void enqueue_device_product(negacyclic_plan& s, const uint32_t* d_a, const uint32_t* d_b, uint32_t* d_c,
                             cudaStream_t stream) {
-    launch_pad_operands(d_a, d_b, s.operands, s.host.n, s.host.limbs, s.padded_limbs, s.host.split, s.tile_counters,
-                        stream);
-    enqueue_product(s, d_c, stream);
+    enqueue_pad(s, d_a, d_b, stream);
+    enqueue_product(s, d_a, d_b, d_c, stream);
 }
 
 int cuda_failure(const CudaError& e) {
@@ -364,6 +441,7 @@ int negacyclic_init(uint32_t n, uint32_t w, uint32_t limbs, const uint32_t* q, c
         s.gemm_tensor_wanted = o.gemm != NEGACYCLIC_GEMM_SIMT;
         s.gemm_tensor_required = o.gemm == NEGACYCLIC_GEMM_TENSOR || o.gemm == NEGACYCLIC_GEMM_TENSOR_SINGLE;
         s.gemm_pairs_allowed = o.gemm != NEGACYCLIC_GEMM_TENSOR_SINGLE;
+        if (s.gemm_tensor_wanted) prepare_gather(s);
         if (s.work_arena) {
             // padding columns of the operands never reach the product (their conversion weights
             // are zero), so the arena needs no clearing; zero it anyway for deterministic dumps
@@ -437,11 +515,12 @@ int negacyclic_get_info(const negacyclic_plan* s, negacyclic_info* info) {
     info->split = h.split;
     info->n_sub = h.n_sub;
     info->words = h.words;
-    info->gemm = (s->convert_engine == NEGACYCLIC_GEMM_TENSOR ? 1u : 0u) | (s->crt_engine == NEGACYCLIC_GEMM_TENSOR ? 2u : 0u);
+    info->gemm = (s->convert_engine == NEGACYCLIC_GEMM_TENSOR || s->convert_rows.ready ? 1u : 0u) |
+                 (s->crt_engine == NEGACYCLIC_GEMM_TENSOR || s->crt_gather.ready ? 2u : 0u);
     info->q_bits = h.q_bits;
     info->device_bytes = s->device_bytes;
     info->table_bytes = s->table_bytes;
-    info->kernels_per_product = kStages + 1;  // + the pad kernel of the device entry point
+    info->kernels_per_product = s->kernels_per_product();
     return NEGACYCLIC_OK;
 }
 
@@ -470,10 +549,9 @@ int negacyclic_run_device_timed(negacyclic_plan* s, const uint32_t* d_a, const u
     try {
         for (auto& e : events) check(cudaEventCreate(&e), "cudaEventCreate");
         check(cudaEventRecord(events[0], stream), "cudaEventRecord");
-        launch_pad_operands(d_a, d_b, s->operands, s->host.n, s->host.limbs, s->padded_limbs, s->host.split,
-                            s->tile_counters, stream);
+        enqueue_pad(*s, d_a, d_b, stream);
         check(cudaEventRecord(events[1], stream), "cudaEventRecord");
-        enqueue_product(*s, d_c, stream, events + 2);
+        enqueue_product(*s, d_a, d_b, d_c, stream, events + 2);
         check(cudaEventSynchronize(events[kStages + 1]), "product");
         for (uint32_t i = 0; i <= kStages; ++i)
             check(cudaEventElapsedTime(&stage_ms[i], events[i], events[i + 1]), "cudaEventElapsedTime");
@@ -632,7 +710,7 @@ void host_begin(negacyclic_plan& s, const uint32_t* a, const uint32_t* b, uint32
             check(cudaStreamWaitEvent(st, s.in_ready[k], 0), "cudaStreamWaitEvent");
             if (!direct)
                 launch_pad_rows(staged, s.operands, h.n, h.limbs, s.padded_limbs, 1, uint32_t(buf_row0), ch.span, st);
-            enqueue_convert(s, ch.t, 1, ch.j0, ch.span, st);
+            enqueue_convert(s, nullptr, nullptr, ch.t, 1, ch.j0, ch.span, st);
             if (k + 1 == in.size() || in[k + 1].t != ch.t)  // transform t complete: its forward NTTs
                 launch_ntt_forward(s.residues, s.primes, s.fwd, s.r, h.n, n_sub, ch.t, 1, st);
         }
@@ -653,11 +731,12 @@ void host_begin(negacyclic_plan& s, const uint32_t* a, const uint32_t* b, uint32
             }
             check(cudaEventRecord(s.in_ready[k], s.copy_in), "cudaEventRecord");
             check(cudaStreamWaitEvent(st, s.in_ready[k], 0), "cudaStreamWaitEvent");
-            if (!direct)
+            if (!direct && !s.convert_rows.ready)
                 launch_pad_rows(staged, s.operands, h.n, h.limbs, s.padded_limbs, split, uint32_t(first),
                                 uint32_t(count), st, op_first, op_count);
             // coefficients [first, first + count): j in [first / s, (first + count) / s) of every transform
-            enqueue_convert(s, 0, split, uint32_t(first / split), uint32_t(count / split), st, op_first, op_count);
+            enqueue_convert(s, staged, staged + words, 0, split, uint32_t(first / split), uint32_t(count / split), st,
+                            op_first, op_count);
             if (k + 1 == in.size() || in[k + 1].op != in[k].op)  // these operands are complete
                 launch_ntt_forward(s.residues, s.primes, s.fwd, s.r, h.n, n_sub, 0, split, st, op_first, op_count);
         }
@@ -668,14 +747,17 @@ void host_begin(negacyclic_plan& s, const uint32_t* a, const uint32_t* b, uint32
     // chunk's work. With wide rows the transpose also goes chunk by chunk, so only the first
     // chunk's share sits between the inverse NTT and the first copy-out.
     uint32_t* dst = s.outputs_staged ? s.stage_out : c;
-    const bool transpose_per_chunk = wide_rows(chunk_shape(s));
-    if (!transpose_per_chunk) launch_transpose(s.residues, s.crt_in, s.r, s.padded_r, h.n, split, 0, n_sub, st);
+    bool gather = s.crt_gather.ready;
+    for (const OutChunk& ch : out) gather = gather && gather_span(s, ch.first, ch.count);
+    const bool transpose_per_chunk = wide_rows(chunk_shape(s)) && !gather;
+    if (!transpose_per_chunk && !gather)
+        launch_transpose(s.residues, s.crt_in, s.r, s.padded_r, h.n, split, 0, n_sub, st);
     for (uint32_t k = 0; k <= out.size(); ++k) {
         if (k < out.size()) {
             if (transpose_per_chunk)  // chunk coefficients are whole multiples of s
                 launch_transpose(s.residues, s.crt_in, s.r, s.padded_r, h.n, split, out[k].first / split,
                                  out[k].count / split, st);
-            enqueue_output(s, out[k].first, out[k].count, s.result, st);
+            enqueue_output(s, out[k].first, out[k].count, s.result, st, gather);
             check(cudaEventRecord(s.out_ready[k], st), "cudaEventRecord");
         }
         if (k >= 1) {
@@ -824,6 +906,12 @@ int negacyclic_debug_read(negacyclic_plan* s, int which, void* host, size_t* byt
     }
     if (*bytes < size) return fail(NEGACYCLIC_EINVAL, "host buffer too small");
     DeviceGuard guard(s->device);
+    if (which >= 1 && s->crt_gather.ready) {  // the product kept neither buffer: make them from its residues
+        launch_transpose(s->residues, s->crt_in, s->r, s->padded_r, h.n, h.split, 0, h.n_sub, s->stream);
+        if (which == 2) enqueue_crt_sums(*s, 0, h.n, s->stream, false);
+        if (cudaStreamSynchronize(s->stream) != cudaSuccess)
+            return fail(NEGACYCLIC_ECUDA, cudaGetErrorString(cudaGetLastError()));
+    }
     cudaError_t e = which == 2  // word sums: rows of dots_stride words on the device, words returned
                         ? cudaMemcpy2D(host, size_t(h.words) * 8, src, size_t(s->dots_stride) * 8, size_t(h.words) * 8,
                                        h.n, cudaMemcpyDeviceToHost)

@@ -56,6 +56,14 @@ struct negacyclic_plan {
     bool outputs_staged = false;    // the running host product copies c through stage_out
     size_t device_bytes = 0, table_bytes = 0;
     negacyclic::TensorGemmPlan convert_gemm, crt_gemm;
+    // Short K steps: GEMMs that gather their A tiles themselves (ready: in use). The conversion then
+    // reads the unpadded operands and the CRT GEMM the residues, without pad and transpose kernels;
+    // where a row's word sums fit one tile (crt_reduces) the CRT GEMM also reduces mod q.
+    negacyclic::TensorGemmPlan convert_rows, crt_gather;
+    bool crt_reduces = false;
+    uint32_t kernels_per_product() const {
+        return 8 - (convert_rows.ready ? 1 : 0) - (crt_gather.ready ? 1 : 0) - (crt_reduces ? 1 : 0);
+    }
 
     ~negacyclic_plan() {
         int previous = 0;

@@ -56,3 +56,40 @@ def test_reduction_row_ends(n, limbs, fpc, inputs, oracle, torch):
 def test_partial_column_tiles(n, limbs, fpc, inputs, oracle, torch):
     q, a, b = inputs.instance(n, limbs, 900 + limbs, 0)
     assert np.array_equal(device_product(fpc, torch, q, a, b), oracle.kronecker(q, a, b))
+
+
+# the gathering GEMMs: rows of one and two K steps with and without 16-byte rows, the switch between
+# the fused reduction (L + 5 <= 64 words) and word sums, and the largest gathered CRT GEMM (L = 123)
+@pytest.mark.parametrize("n,split", [(128, 1), (2048, 1), (2048, 4), (4096, 2)])
+@pytest.mark.parametrize("limbs", [1, 4, 27, 28, 31, 32, 33, 56, 59, 60, 64, 65, 100, 123, 124])
+def test_gathered_tiles(n, split, limbs, fpc, inputs, oracle, torch):
+    q, a, b = inputs.instance(n, limbs, 70 + limbs, 0)
+    want = oracle.kronecker(q, a, b)
+    assert np.array_equal(device_product(fpc, torch, q, a, b, split=split), want)
+    with fpc.Plan(n, 32 * limbs, limbs, q, split=split) as plan:
+        assert np.array_equal(plan.run(a, b), want)
+
+
+@pytest.mark.parametrize("limbs", [4, 28, 55])
+def test_operands_on_any_word_boundary(limbs, fpc, inputs, oracle, torch):
+    n = 1024
+    q, a, b = inputs.instance(n, limbs, 5, 0)
+    want = oracle.kronecker(q, a, b)
+    stream = torch.cuda.current_stream().cuda_stream
+    with fpc.Plan(n, 32 * limbs, limbs, q) as plan:
+        for shift in ((0, 0, 0), (1, 0, 0), (0, 3, 1), (2, 2, 2)):
+            buffers = [torch.zeros(n * limbs + 4, dtype=torch.int32, device="cuda") for _ in range(3)]
+            views = [t[k:k + n * limbs] for t, k in zip(buffers, shift)]
+            views[0].copy_(torch.from_numpy(a.view(np.int32).ravel()))
+            views[1].copy_(torch.from_numpy(b.view(np.int32).ravel()))
+            plan.run_device(*(v.data_ptr() for v in views), stream)
+            torch.cuda.synchronize()
+            assert np.array_equal(views[2].cpu().numpy().view(np.uint32).reshape(n, limbs), want)
+
+
+def test_host_chunks_below_a_gathered_tile(fpc, inputs, oracle):
+    """N=16384 in 16 transforms: the host path's output chunks are 64 positions of each transform."""
+    n, limbs = 16384, 20
+    q, a, b = inputs.instance(n, limbs, 8, 0)
+    with fpc.Plan(n, 32 * limbs, limbs, q, split=16) as plan:
+        assert np.array_equal(plan.run(a, b), oracle.kronecker(q, a, b))
