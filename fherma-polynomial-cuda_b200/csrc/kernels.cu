@@ -627,55 +627,63 @@ __global__ void __launch_bounds__(256) transpose_kernel(const uint32_t* __restri
 // the earlier form (stage between events): 624 -> 362 us at N = 65536, L = 1747 (1.38 GB, 3.8 TB/s),
 // 142 -> 90 us at N = 32768, L = 868, 49 -> 20.5 us at N = 65536, L = 55.
 
-// A row's step: kChunk words of every row of the warp, with the same words of q and R behind them.
-template <uint32_t kChunk>
+//
+// Few rows: a thread's chain of L + 2 words is then all there is to wait for, so a row is cut into
+// kSegments segments, one lane each. A segment starts with no carry; afterwards each passes its carry
+// up, where it is added to the stored words and almost always ends in the first one. N = 256, L =
+// 1747: product 187 -> 131 us.
+
+// A row's step: kChunk words of every lane's segment, with the same words of q and R behind them.
+template <uint32_t kChunk, uint32_t kSegments>
 struct ReduceSlot {
-    static constexpr uint32_t kPitch = kChunk * 8 + 16;  // bytes per row
-    static constexpr uint32_t kBytes = 32 * kPitch + kChunk * 8;
+    static constexpr uint32_t kPitch = kChunk * 8 + 16;       // bytes per lane
+    static constexpr uint32_t kTablePitch = kChunk * 8 + (kSegments > 1 ? 16 : 0);  // bytes per segment: q, then R
+    static constexpr uint32_t kBytes = 32 * kPitch + kSegments * kTablePitch;
 };
 constexpr uint32_t kReduceSlots = 3;
 
-template <uint32_t kChunk>
+template <uint32_t kChunk, uint32_t kSegments>
 __global__ void reduce_kernel(ReduceParams prm) {
     chain_enter();
-    using Slot = ReduceSlot<kChunk>;
-    constexpr uint32_t kPitch = Slot::kPitch;
+    using Slot = ReduceSlot<kChunk, kSegments>;
+    constexpr uint32_t kPitch = Slot::kPitch, kRows = 32 / kSegments;
     extern __shared__ __align__(16) uint8_t reduce_smem[];
     const uint32_t warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     uint8_t* slots = reduce_smem + warp * (kReduceSlots * Slot::kBytes);
     const uint32_t slots_addr = uint32_t(__cvta_generic_to_shared(slots));
-    const uint32_t row0 = (blockIdx.x * (blockDim.x / 32) + warp) * 32;
+    const uint32_t row0 = (blockIdx.x * (blockDim.x / 32) + warp) * kRows;
     if (row0 >= prm.n) return;  // warp-uniform
-    const uint32_t limbs = prm.limbs, tlen = limbs + 2, rows = min(32u, prm.n - row0);
-    const uint32_t chunks = (tlen + kChunk - 1) / kChunk;
+    const uint32_t limbs = prm.limbs, tlen = limbs + 2, rows = min(kRows, prm.n - row0);
+    // segment g of a row is its words [g span, (g + 1) span)
+    const uint32_t chunks = ((tlen + kSegments - 1) / kSegments + kChunk - 1) / kChunk, span = chunks * kChunk;
+    const uint32_t own_row = lane / kSegments, own_segment = lane % kSegments;
     const uint64_t* d0 = prm.dots + size_t(row0) * prm.dots_stride;
 
-    // chunk c of the warp's rows, and of q and R, into slot c % kReduceSlots
+    // chunk c of every lane's segment, and of q and R, into slot c % kReduceSlots
     auto fetch = [&](uint32_t c) {
         if (c < chunks) {
-            constexpr uint32_t kLanes = kChunk / 2;  // per row, 16 bytes each
+            constexpr uint32_t kLanes = kChunk / 2;  // per segment, 16 bytes each
             const uint32_t slot = slots_addr + (c % kReduceSlots) * Slot::kBytes;
             const uint32_t w = c * kChunk + 2 * (lane % kLanes);
-            if (w < prm.dots_stride) {
-                const uint32_t to = slot + (lane % kLanes) * 16;
-                const uint64_t* from = d0 + w;
 #pragma unroll 8
-                for (uint32_t i = 0; i < kLanes; ++i) {
-                    const uint32_t r = i * (32 / kLanes) + lane / kLanes;
-                    if (r < rows) cp_async_16(to + r * kPitch, from + size_t(r) * prm.dots_stride);
-                }
+            for (uint32_t i = 0; i < kLanes; ++i) {
+                const uint32_t r = i * (32 / kLanes) + lane / kLanes, at = (r % kSegments) * span + w;
+                if (r / kSegments < rows && at < prm.dots_stride)
+                    cp_async_16(slot + r * kPitch + (lane % kLanes) * 16, d0 + size_t(r / kSegments) * prm.dots_stride + at);
             }
-            if (lane < kChunk / 2) {  // q, then R: kChunk / 4 pieces of 16 bytes each
-                const uint32_t piece = lane % (kChunk / 4);
-                cp_async_16(slot + 32 * kPitch + lane * 16,
-                            (lane < kChunk / 4 ? prm.q : prm.minus_p) + c * kChunk + piece * 4);
+            constexpr uint32_t kPieces = kChunk / 2;  // of a segment's tables: q, then R
+            for (uint32_t i = lane; i < kSegments * kPieces; i += 32) {
+                const uint32_t g = i / kPieces, piece = i % kPieces, at = g * span + c * kChunk + piece % (kPieces / 2) * 4;
+                if (at < reduce_table_words(limbs))
+                    cp_async_16(slot + 32 * kPitch + g * Slot::kTablePitch + piece * 16,
+                                (piece < kPieces / 2 ? prm.q : prm.minus_p) + at);
             }
         }
         cp_async_commit();
     };
     for (uint32_t c = 0; c < kReduceSlots; ++c) fetch(c);
 
-    const uint64_t* d = d0 + size_t(min(lane, rows - 1)) * prm.dots_stride;
+    const uint64_t* d = d0 + size_t(min(own_row, rows - 1)) * prm.dots_stride;
     const uint64_t x[3] = {d[limbs + 2], d[limbs + 3], d[limbs + 4]};
     uint64_t window[kWindow];
 #pragma unroll
@@ -685,23 +693,26 @@ __global__ void reduce_kernel(ReduceParams prm) {
     }
     const RowQuotient f = row_quotient(x, window, prm);
     RowState st;
+    uint64_t above = 0;  // what the segment adds to the words from L up (in units of word L)
+    if (kSegments > 1 && own_segment > 0 && own_segment * span <= limbs) st.start(f, prm.q[own_segment * span - 1]);
     for (uint32_t c = 0; c < chunks; ++c) {
         cp_async_wait<kReduceSlots - 1>();
         __syncwarp();
         uint8_t* slot = slots + (c % kReduceSlots) * Slot::kBytes;
         uint8_t* own = slot + lane * kPitch;
-        const uint4* q4 = reinterpret_cast<const uint4*>(slot + 32 * kPitch);  // the same for every lane
+        const uint4* q4 = reinterpret_cast<const uint4*>(slot + 32 * kPitch + own_segment * Slot::kTablePitch);
         const uint4* r4 = q4 + kChunk / 4;
-        const uint32_t base = c * kChunk;
+        const uint32_t base = own_segment * span + c * kChunk;
 #pragma unroll 1
         for (uint32_t part = 0; part < kChunk; part += 16) {  // 16 words at a time through registers
-            if (base + part >= tlen) break;
+            if (kSegments == 1 && base + part >= tlen) break;
             uint64_t sums[16];
             uint4 q[4], r[4];
+            const bool table = base + part < tlen;  // past a row's end there is nothing (and nothing was fetched)
 #pragma unroll
             for (uint32_t g = 0; g < 4; ++g) {
-                q[g] = q4[part / 4 + g];
-                r[g] = r4[part / 4 + g];
+                q[g] = table ? q4[part / 4 + g] : make_uint4(0, 0, 0, 0);
+                r[g] = table ? r4[part / 4 + g] : make_uint4(0, 0, 0, 0);
             }
 #pragma unroll
             for (uint32_t g = 0; g < 8; ++g) {
@@ -715,20 +726,27 @@ __global__ void reduce_kernel(ReduceParams prm) {
             for (uint32_t g = 0; g < 4; ++g)  // over words that this thread has already read
                 *reinterpret_cast<uint4*>(own + part * 4 + g * 16) =
                     make_uint4(o[4 * g], o[4 * g + 1], o[4 * g + 2], o[4 * g + 3]);
+            if (kSegments > 1 && base + part + 16 > limbs) {
+#pragma unroll
+                for (uint32_t i = 0; i < 16; ++i) {
+                    if (base + part + i == limbs) above += o[i];
+                    if (base + part + i == limbs + 1) above += uint64_t(o[i]) << 32;
+                }
+            }
         }
         __syncwarp();
         if constexpr (kChunk == 16) {
-            // two rows per instruction (r and r + 4: their slots' banks do not meet), 64 bytes each
-            if (base + lane % 16 < limbs) {
-                uint32_t* out = prm.out + size_t(row0) * limbs + base + lane % 16;
+            // two lanes' words per instruction (r and r + 4: their banks do not meet), 64 bytes each
 #pragma unroll
-                for (uint32_t i = 0; i < 16; ++i) {
-                    const uint32_t r = (i / 4) * 8 + i % 4 + (lane / 16) * 4;
-                    if (r < rows)
-                        out[size_t(r) * limbs] = reinterpret_cast<const uint32_t*>(slot + r * kPitch)[lane % 16];
-                }
+            for (uint32_t i = 0; i < 16; ++i) {
+                const uint32_t r = (i / 4) * 8 + i % 4 + (lane / 16) * 4;
+                const uint32_t w = (r % kSegments) * span + c * kChunk + lane % 16;
+                if (r / kSegments < rows && w < limbs)
+                    prm.out[size_t(row0 + r / kSegments) * limbs + w] =
+                        reinterpret_cast<const uint32_t*>(slot + r * kPitch)[lane % 16];
             }
         } else {
+            static_assert(kChunk == 16 || kSegments == 1, "wide chunks go with whole rows");
 #pragma unroll
             for (uint32_t part = 0; part < kChunk; part += 32) {
                 if (base + part + lane >= limbs) continue;
@@ -741,7 +759,37 @@ __global__ void reduce_kernel(ReduceParams prm) {
         __syncwarp();
         fetch(c + kReduceSlots);
     }
-    if (lane < rows) st.finish(prm.out + size_t(row0 + lane) * limbs, prm);
+    uint32_t* row = prm.out + size_t(row0 + min(own_row, rows - 1)) * limbs;
+    if constexpr (kSegments == 1) {
+        if (lane < rows) st.finish(row, prm);
+    } else {
+        // carries between segments; above word L they are summed up instead
+        const uint32_t start = own_segment * span, end = start + span;
+        int64_t up = own_row < rows ? st.carry : 0;
+        if (end >= limbs) {
+            if (end < limbs + 2) above += uint64_t(up) << (32 * (end - limbs));
+            up = 0;
+        }
+        while (__any_sync(0xffffffffu, up != 0)) {
+            int64_t carry = __shfl_up_sync(0xffffffffu, up, 1, kSegments);
+            if (own_segment == 0) carry = 0;
+            up = 0;
+            uint32_t w = start;
+            for (; carry != 0 && w < min(end, limbs); ++w) {
+                const int64_t t = int64_t(row[w]) + carry;
+                row[w] = uint32_t(t);
+                carry = t >> 32;
+            }
+            if (w < limbs)
+                up = carry;
+            else
+                above += uint64_t(carry);
+        }
+#pragma unroll
+        for (uint32_t i = 1; i < kSegments; i *= 2) above += __shfl_xor_sync(0xffffffffu, above, i, kSegments);
+        __syncwarp();
+        if (own_segment == 0 && own_row < rows) RowState::finish_in_memory(row, uint32_t(above), prm);
+    }
 }
 
 uint32_t log2_u32(uint32_t x) { return x ? 31 - __builtin_clz(x) : 0; }
@@ -879,24 +927,38 @@ void launch_transpose(const uint32_t* residues, uint32_t* crt_in, uint32_t r, ui
                    j_count);
 }
 
-template <uint32_t kChunk>
+template <uint32_t kChunk, uint32_t kSegments>
 static void launch_reduce_chunks(const ReduceParams& params, uint32_t warps, cudaStream_t stream) {
-    const size_t smem = size_t(warps) * kReduceSlots * ReduceSlot<kChunk>::kBytes;
+    const size_t smem = size_t(warps) * kReduceSlots * ReduceSlot<kChunk, kSegments>::kBytes;
     if (smem > 48 * 1024)  // per device; cheap enough to repeat
-        cudaFuncSetAttribute(reduce_kernel<kChunk>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-    const uint32_t groups = (params.n + 31) / 32;  // of 32 rows, a warp each
-    launch_chained(reduce_kernel<kChunk>, (groups + warps - 1) / warps, warps * 32, smem, stream, params);
+        cudaFuncSetAttribute(reduce_kernel<kChunk, kSegments>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    const uint32_t rows = 32 / kSegments, groups = (params.n + rows - 1) / rows;  // of `rows` rows, a warp each
+    launch_chained(reduce_kernel<kChunk, kSegments>, (groups + warps - 1) / warps, warps * 32, smem, stream, params);
 }
 
 void launch_reduce(const ReduceParams& params, cudaStream_t stream) {
+    // Segments for fewer rows than a warp of them on every other SM: as many as leave 16 words each.
+    // Product, us, whole rows / segments: 186.8 / 131.3 (N = 256, L = 1747), 358.5 / 324.7 (N = 1024),
+    // 44.3 / 36.4 (N = 256, L = 313); from 4096 rows on they lose: 45.8 / 48.0 (L = 94), 893 / 909
+    // (N = 16384, L = 625).
+    uint32_t segments = 1;
+    if (params.n < 16 * 148)
+        while (segments < 16 && params.limbs / (2 * segments) >= 16) segments *= 2;
+    switch (segments) {
+        case 2: launch_reduce_chunks<16, 2>(params, 1, stream); return;
+        case 4: launch_reduce_chunks<16, 4>(params, 1, stream); return;
+        case 8: launch_reduce_chunks<16, 8>(params, 1, stream); return;
+        case 16: launch_reduce_chunks<16, 16>(params, 1, stream); return;
+        default: break;
+    }
     // Chunks of 64 words (512-byte runs per row) read DRAM better than chunks of 16 (128-byte runs
     // of rows 14 KB apart): 362 against 432 us at N = 65536, L = 1747, 22.5 against 30.4 at N = 16384,
     // L = 301. A row of up to 64 words is better read in four steps, with more warps per SM: 20.5
     // against 24.6 us at N = 65536, L = 55. (us of the stage between events, about 5 of them launch.)
     if (params.limbs + 2 <= 64)
-        launch_reduce_chunks<16>(params, params.n > 32 * 148 * 2 ? 2 : 1, stream);
+        launch_reduce_chunks<16, 1>(params, params.n > 32 * 148 * 2 ? 2 : 1, stream);
     else
-        launch_reduce_chunks<64>(params, 1, stream);
+        launch_reduce_chunks<64, 1>(params, 1, stream);
 }
 
 }  // namespace negacyclic

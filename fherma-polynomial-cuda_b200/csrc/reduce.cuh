@@ -84,11 +84,17 @@ static __device__ __noinline__ bool correct_row(uint32_t* row, uint32_t over, co
 }
 
 // Running state of one row's pass.
+// (A row may be cut into segments that start with no carry; they start with start().)
 struct RowState {
     int64_t carry = 0;   // signed carry into the next word
     uint64_t below = 0;  // hi(ql q[w-1]) + qh q[w-1], subtracted at word w
     // of the result: words at and above q's (or-ed), and the two below
     uint32_t over = 0, top1 = 0, top0 = 0;
+
+    // Before a first word above word 0: `q_below` is the word of q under it.
+    __device__ __forceinline__ void start(const RowQuotient& f, uint32_t q_below) {
+        below = ((uint64_t(f.low) * q_below) >> 32) + uint64_t(f.high) * q_below;
+    }
 
     // Word w of T' - quotient q: d + K R - lo(ql q) - below + carry. d < 2^56, K R < 2^46 and
     // below < 2^49, so the sum stays within int64.
@@ -127,6 +133,15 @@ struct RowState {
                 if (w >= prm.q_words) over |= o[i];
             }
         }
+    }
+
+    // The same for a row whose words are only in global memory, `above` standing over them.
+    static __device__ __forceinline__ void finish_in_memory(uint32_t* row, uint32_t above, const ReduceParams& prm) {
+        RowState st;
+        st.over = above | (prm.q_words < prm.limbs ? row[prm.q_words] : 0u);
+        st.top1 = row[prm.q_words - 1];
+        st.top0 = prm.q_words >= 2 ? row[prm.q_words - 2] : 0u;
+        st.finish(row, prm);
     }
 
     // After the row is in global memory: a result whose top two words are below q's is canonical; the

@@ -93,3 +93,20 @@ def test_host_chunks_below_a_gathered_tile(fpc, inputs, oracle):
     q, a, b = inputs.instance(n, limbs, 8, 0)
     with fpc.Plan(n, 32 * limbs, limbs, q, split=16) as plan:
         assert np.array_equal(plan.run(a, b), oracle.kronecker(q, a, b))
+
+
+# rows in 2 to 16 segments of a reduction, with carries that run through whole segments: with
+# q = 2^(32 L) - 1 and its neighbours, products of q - 1 and of limbs of ones leave long runs of equal words
+@pytest.mark.parametrize("limbs", [31, 32, 33, 63, 64, 127, 128, 254, 255, 256, 270, 300, 511, 520])
+@pytest.mark.parametrize("n", [1, 4, 128])
+def test_segmented_reduction(n, limbs, fpc, inputs, oracle, torch):
+    top = 1 << (32 * limbs)
+    for qv in (top - 1, top // 2 + 1, (top >> 33) - 1, top - (top >> 40) + 1):
+        q = inputs.from_int(qv, limbs)
+        rng = np.random.Generator(np.random.PCG64(limbs))
+        words = np.flatnonzero(q)[-1] + 1
+        pairs = [tuple(np.pad(inputs.random_operand(rng, n, q[:words]), ((0, 0), (0, limbs - words)))
+                       for _ in range(2))]
+        pairs += [(inputs.edge_operand(n, q, x), inputs.edge_operand(n, q, y)) for x, y in inputs.EDGE_PAIRS]
+        for a, b in pairs:
+            assert np.array_equal(device_product(fpc, torch, q, a, b), oracle.kronecker(q, a, b))
