@@ -377,13 +377,13 @@ __device__ __forceinline__ void gs_stages(uint32_t (&x)[1 << R], uint32_t group_
 // One pass of R stages over all of this thread's groups (transform length 2^kLog). src/dst are shared (swizzled index) or global (plain index);
 // kScale multiplies the values stored to global by (f, f_q).
 template <int R, bool kForward, bool kFromGlobal, bool kToGlobal, bool kScale, uint32_t kLogTMin, uint32_t kLog>
-__device__ __forceinline__ void ntt_pass(const uint32_t* src, uint32_t* dst, const uint2* __restrict__ table,
-                                         uint32_t p, uint32_t f, uint32_t f_q) {
+__device__ __forceinline__ void ntt_pass(uint32_t tid, const uint32_t* src, uint32_t* dst,
+                                         const uint2* __restrict__ table, uint32_t p, uint32_t f, uint32_t f_q) {
     constexpr int G = per_thread(kLog) >> R;  // groups per thread
     constexpr uint32_t kThreads = (1u << kLog) / per_thread(kLog);
 #pragma unroll
     for (int g = 0; g < G; ++g) {
-        const uint32_t group = threadIdx.x + g * kThreads;
+        const uint32_t group = tid + g * kThreads;
         const uint32_t off = group & ((1u << kLogTMin) - 1);
         const uint32_t base = ((group >> kLogTMin) << (kLogTMin + R)) + off;
         const uint32_t placed = swizzle<kLog>(base);  // shared-memory place of the group's first word
@@ -427,10 +427,10 @@ __device__ __forceinline__ void ntt_pass(const uint32_t* src, uint32_t* dst, con
         }
         if constexpr (kToGlobal && kPair) {
             *reinterpret_cast<uint2*>(dst + base) = make_uint2(x[0], x[1]);
-        } else if constexpr (kToGlobal && kVector && R == 4) {
+        } else if constexpr (kToGlobal && kVector && R == 4 && kThreads >= 32) {
             // neighbouring lanes trade quarters of their 16 words, so that the two of them fill
             // whole 32-byte sectors with each store
-            const bool odd = threadIdx.x & 1;
+            const bool odd = tid & 1;
             uint32_t* to = dst + base - (odd ? 16 - 4 : 0);
 #pragma unroll
             for (int q = 0; q < 16; q += 8) {
@@ -467,20 +467,24 @@ __device__ __forceinline__ void ntt_pass(const uint32_t* src, uint32_t* dst, con
 // inverse (small -> large, which also scales its output). Length 8192 takes five stages at the
 // large-stride end instead (its global accesses there are whole 128-byte lines), and four at the
 // unit-stride end, where lanes trade words so that their stores fill sectors.
+constexpr int ntt_pass_stages(bool forward, uint32_t log, uint32_t done) {
+    if (log == 13) return (forward ? done == 0 : done == 8) ? 5 : 4;
+    if (!forward && done == 0 && log % 4 != 0) return int(log % 4);
+    return log - done < 4 ? int(log - done) : 4;
+}
+
+// `tid`: the thread's number among the transform's.
 template <bool kForward, uint32_t kLog, uint32_t kDone>
-__device__ __forceinline__ void ntt_passes(uint32_t* data, uint32_t* xs, const uint2* __restrict__ table, uint32_t p,
-                                           uint32_t f, uint32_t f_q) {
-    constexpr int R = kLog == 13 ? (kForward ? (kDone == 0 ? 5 : 4) : (kDone == 8 ? 5 : 4))
-                      : (!kForward && kDone == 0 && kLog % 4 != 0) ? int(kLog % 4)
-                      : (kLog - kDone) < 4                       ? int(kLog - kDone)
-                                                                  : 4;
+__device__ __forceinline__ void ntt_passes(uint32_t tid, uint32_t* data, uint32_t* xs, const uint2* __restrict__ table,
+                                           uint32_t p, uint32_t f, uint32_t f_q) {
+    constexpr int R = ntt_pass_stages(kForward, kLog, kDone);
     constexpr uint32_t kLogTMin = kForward ? kLog - kDone - R : kDone;
     constexpr bool kFirst = kDone == 0, kLast = kDone + R == kLog;
-    ntt_pass<R, kForward, kFirst, kLast, kLast && !kForward, kLogTMin, kLog>(kFirst ? data : xs, kLast ? data : xs,
+    ntt_pass<R, kForward, kFirst, kLast, kLast && !kForward, kLogTMin, kLog>(tid, kFirst ? data : xs, kLast ? data : xs,
                                                                               table, p, f, f_q);
     if constexpr (!kLast) {
         __syncthreads();
-        ntt_passes<kForward, kLog, kDone + R>(data, xs, table, p, f, f_q);
+        ntt_passes<kForward, kLog, kDone + R>(tid, data, xs, table, p, f, f_q);
     }
 }
 
@@ -496,7 +500,7 @@ __global__ void __launch_bounds__((1u << kLog) / per_thread(kLog), 4) ntt_forwar
     const uint32_t local_op = blockIdx.x / t_count, op = op_first + local_op;
     const uint32_t t_index = t_first + blockIdx.x - local_op * t_count, k = blockIdx.y;
     uint32_t* data = residues + (size_t(op) * r + k) * n + size_t(t_index) * kN;
-    ntt_passes<true, kLog, 0>(data, xs, fwd + size_t(k) * kN, primes[k].p, 0, 0);
+    ntt_passes<true, kLog, 0>(threadIdx.x, data, xs, fwd + size_t(k) * kN, primes[k].p, 0, 0);
 }
 
 template <uint32_t kLog>
@@ -509,7 +513,84 @@ __global__ void __launch_bounds__((1u << kLog) / per_thread(kLog), 4) ntt_invers
     const uint32_t v_index = v_first + blockIdx.x, k = blockIdx.y;
     const DevicePrime f = primes[k];
     uint32_t* data = residues + size_t(k) * n + size_t(v_index) * kN;
-    ntt_passes<false, kLog, 0>(data, xs, inv + size_t(k) * kN, f.p, f.finish, f.finish_q);
+    ntt_passes<false, kLog, 0>(threadIdx.x, data, xs, inv + size_t(k) * kN, f.p, f.finish, f.finish_q);
+}
+
+// Unsplit rings (s = 1): both operands' forward transforms, their product and its inverse in one CTA
+// per prime; only the inputs are read and only the result is written (over operand a's residues).
+// One half of the block transforms a, the other b. The forward's last pass and the inverse's first
+// work on the same groups of consecutive values, so a's are still in registers when b's come
+// through shared memory, are multiplied, and enter the inverse, which the first half finishes.
+// Two launches and two round trips through L2 less. Product, us, three kernels / one: 17.7 / 12.4 at
+// N = 256, L = 2; 17.5 / 14.5 at N = 2048, L = 13; 38.5 / 34.8 at N = 4096, L = 64; 85.6 / 74.0 at
+// N = 8192, L = 128; 791 / 721 at N = 8192, L = 868 (33.0 / 33.6 at N = 2048, L = 94: 197 CTAs).
+template <uint32_t kLog, uint32_t kDone>
+__device__ __forceinline__ void forward_to_middle(uint32_t tid, uint32_t* data, uint32_t* xs,
+                                                  const uint2* __restrict__ table, uint32_t p) {
+    constexpr int R = ntt_pass_stages(true, kLog, kDone);
+    if constexpr (kDone + R < kLog) {
+        ntt_pass<R, true, kDone == 0, false, false, kLog - kDone - R, kLog>(tid, kDone == 0 ? data : xs, xs, table, p, 0, 0);
+        __syncthreads();
+        forward_to_middle<kLog, kDone + R>(tid, data, xs, table, p);
+    }
+}
+
+template <uint32_t kLog, uint32_t kDone>
+__device__ __forceinline__ void inverse_from_middle(bool active, uint32_t tid, uint32_t* data, uint32_t* xs,
+                                                    const uint2* __restrict__ table, uint32_t p, uint32_t f,
+                                                    uint32_t f_q) {
+    if constexpr (kDone < kLog) {
+        constexpr int R = ntt_pass_stages(false, kLog, kDone);
+        constexpr bool kLast = kDone + R == kLog;
+        __syncthreads();
+        if (active) ntt_pass<R, false, false, kLast, kLast, kDone, kLog>(tid, xs, kLast ? data : xs, table, p, f, f_q);
+        inverse_from_middle<kLog, kDone + R>(active, tid, data, xs, table, p, f, f_q);
+    }
+}
+
+template <uint32_t kLog>
+__global__ void __launch_bounds__(2 * (1u << kLog) / per_thread(kLog), (kLog >= 12 ? 2 : 4))
+    ntt_product_kernel(uint32_t* residues, const DevicePrime* __restrict__ primes, const uint2* __restrict__ fwd,
+                       const uint2* __restrict__ inv, uint32_t r) {
+    chain_enter();
+    extern __shared__ uint32_t xs[];
+    constexpr uint32_t kN = 1u << kLog, kThreads = kN / per_thread(kLog);
+    constexpr int R = kLog % 4 && kLog != 13 ? int(kLog % 4) : 4;  // of the forward's last and the inverse's first pass
+    constexpr int G = per_thread(kLog) >> R;
+    const uint32_t k = blockIdx.x, op = threadIdx.x / kThreads, tid = threadIdx.x % kThreads;
+    const DevicePrime f = primes[k];
+    uint32_t* data = residues + (size_t(op) * r + k) * kN;
+    uint32_t* own = xs + op * kN;
+    const uint2 *forward = fwd + size_t(k) * kN, *inverse = inv + size_t(k) * kN;
+    forward_to_middle<kLog, 0>(tid, data, own, forward, f.p);
+    constexpr bool kPaired = kLog == 13;
+    uint32_t x[G][1 << R];
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+        const uint32_t group = tid + g * kThreads, placed = swizzle<kLog>(group << R);
+#pragma unroll
+        for (int i = 0; i < (1 << R); ++i) x[g][i] = own[placed ^ swizzle<kLog>(uint32_t(i))];
+        ct_stages<R, kPaired>(x[g], group, 0, kLog, forward, f.p);
+#pragma unroll
+        for (int i = 0; i < (1 << R); ++i) {
+            x[g][i] = reduce_once(x[g][i], f.p);
+            if (op == 1) own[placed ^ swizzle<kLog>(uint32_t(i))] = x[g][i];
+        }
+    }
+    __syncthreads();
+    if (op == 0) {
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+            const uint32_t group = tid + g * kThreads, placed = swizzle<kLog>(group << R);
+#pragma unroll
+            for (int i = 0; i < (1 << R); ++i)
+                x[g][i] = mont(x[g][i], xs[kN + (placed ^ swizzle<kLog>(uint32_t(i)))], f.p, f.pinv);
+            gs_stages<R, kPaired>(x[g], group, 0, kLog, inverse, f.p);
+#pragma unroll
+            for (int i = 0; i < (1 << R); ++i) xs[placed ^ swizzle<kLog>(uint32_t(i))] = x[g][i];
+        }
+    }
+    inverse_from_middle<kLog, R>(op == 0, tid, data, xs, inverse, f.p, f.finish, f.finish_q);
 }
 
 // C_v = sum_{t+u=v} A_t B_u + zeta * sum_{t+u=v+s} A_t B_u at every evaluation point,
@@ -891,6 +972,29 @@ void launch_ntt_inverse(uint32_t* residues, const DevicePrime* primes, const uin
     dim3 grid(v_count, r);
     launch_chained(ntt_inverse_kernel, grid, ntt_threads(n_sub), n_sub * sizeof(uint32_t), stream, residues, primes, inv, r,
                    n, n_sub, v_first);
+}
+
+template <uint32_t kLog>
+static void launch_product(uint32_t* residues, const DevicePrime* primes, const uint2* fwd, const uint2* inv, uint32_t r,
+                           cudaStream_t stream) {
+    constexpr uint32_t kN = 1u << kLog;
+    constexpr int kSmem = 2 * kN * sizeof(uint32_t);
+    if (kSmem > 48 * 1024)  // per device; cheap enough to repeat
+        cudaFuncSetAttribute(ntt_product_kernel<kLog>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+    launch_chained(ntt_product_kernel<kLog>, r, 2 * kN / per_thread(kLog), kSmem, stream, residues, primes, fwd, inv, r);
+}
+
+bool launch_ntt_product(uint32_t* residues, const DevicePrime* primes, const uint2* fwd, const uint2* inv, uint32_t r,
+                        uint32_t n, cudaStream_t stream) {
+    switch (n) {
+        case 256: launch_product<8>(residues, primes, fwd, inv, r, stream); return true;
+        case 512: launch_product<9>(residues, primes, fwd, inv, r, stream); return true;
+        case 1024: launch_product<10>(residues, primes, fwd, inv, r, stream); return true;
+        case 2048: launch_product<11>(residues, primes, fwd, inv, r, stream); return true;
+        case 4096: launch_product<12>(residues, primes, fwd, inv, r, stream); return true;
+        case 8192: launch_product<13>(residues, primes, fwd, inv, r, stream); return true;
+        default: return false;
+    }
 }
 
 void launch_pointwise(uint32_t* residues, const DevicePrime* primes, const uint2* zeta, uint32_t r, uint32_t n,

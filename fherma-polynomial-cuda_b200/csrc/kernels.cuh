@@ -123,6 +123,10 @@ void launch_gemm_simt(const uint8_t* a, uint64_t a_pitch, RowMap rows, uint32_t 
 void launch_ntt_forward(uint32_t* residues, const DevicePrime* primes, const uint2* fwd, uint32_t r,
                         uint32_t n, uint32_t n_sub, uint32_t t_first, uint32_t t_count, cudaStream_t stream,
                         uint32_t op_first = 0, uint32_t op_count = 2);
+// forward NTTs of both operands, pointwise products and inverse NTTs of an unsplit ring (n = N'), every
+// prime, in one kernel; false (nothing launched) for lengths it does not take
+bool launch_ntt_product(uint32_t* residues, const DevicePrime* primes, const uint2* fwd, const uint2* inv, uint32_t r,
+                        uint32_t n, cudaStream_t stream);
 void launch_pointwise(uint32_t* residues, const DevicePrime* primes, const uint2* zeta, uint32_t r,
                       uint32_t n, uint32_t n_sub, uint32_t split, cudaStream_t stream);
 // inverse NTTs of transforms [v_first, v_first + v_count), every prime

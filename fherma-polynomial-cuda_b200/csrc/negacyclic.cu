@@ -175,12 +175,16 @@ void enqueue_middle(negacyclic_plan& s, cudaStream_t stream, cudaEvent_t* marks)
         if (marks) check(cudaEventRecord(marks[stage], stream), "cudaEventRecord");
         ++stage;
     };
-    launch_ntt_forward(s.residues, s.primes, s.fwd, s.r, n, h.n_sub, 0, h.split, stream);
-    mark();
-    launch_pointwise(s.residues, s.primes, s.zeta, s.r, n, h.n_sub, h.split, stream);
-    mark();
-    launch_ntt_inverse(s.residues, s.primes, s.inv, s.r, n, h.n_sub, 0, h.split, stream);
-    mark();
+    if (s.ntt_fused() && launch_ntt_product(s.residues, s.primes, s.fwd, s.inv, s.r, n, stream)) {
+        for (int i = 0; i < 3; ++i) mark();
+    } else {
+        launch_ntt_forward(s.residues, s.primes, s.fwd, s.r, n, h.n_sub, 0, h.split, stream);
+        mark();
+        launch_pointwise(s.residues, s.primes, s.zeta, s.r, n, h.n_sub, h.split, stream);
+        mark();
+        launch_ntt_inverse(s.residues, s.primes, s.inv, s.r, n, h.n_sub, 0, h.split, stream);
+        mark();
+    }
     if (!s.crt_gather.ready) launch_transpose(s.residues, s.crt_in, s.r, s.padded_r, n, h.split, 0, h.n_sub, stream);
     mark();
 }
@@ -638,6 +642,7 @@ void host_begin(negacyclic_plan& s, const uint32_t* a, const uint32_t* b, uint32
     std::vector<OutChunk> out;
     const bool ordered = transform_ordered_input(chunk_shape(s));
     stream_chunks(chunk_shape(s), ordered, in, out);
+    const bool fuse_ntt = s.ntt_fused() && in.size() == 1;  // in pieces, a's transforms run while b is on the link
     uint32_t pieces[negacyclic_plan::kMaxChunks] = {};  // pack pieces per input chunk
     if (!a_locked || !b_locked) {
         // One pack job over pieces of about kPieceBytes of the pageable operands, claimed in chunk
@@ -737,12 +742,14 @@ void host_begin(negacyclic_plan& s, const uint32_t* a, const uint32_t* b, uint32
             // coefficients [first, first + count): j in [first / s, (first + count) / s) of every transform
             enqueue_convert(s, staged, staged + words, 0, split, uint32_t(first / split), uint32_t(count / split), st,
                             op_first, op_count);
-            if (k + 1 == in.size() || in[k + 1].op != in[k].op)  // these operands are complete
+            if (!fuse_ntt && (k + 1 == in.size() || in[k + 1].op != in[k].op))  // these operands are complete
                 launch_ntt_forward(s.residues, s.primes, s.fwd, s.r, h.n, n_sub, 0, split, st, op_first, op_count);
         }
     }
-    launch_pointwise(s.residues, s.primes, s.zeta, s.r, h.n, n_sub, split, st);
-    launch_ntt_inverse(s.residues, s.primes, s.inv, s.r, h.n, n_sub, 0, split, st);
+    if (!fuse_ntt || !launch_ntt_product(s.residues, s.primes, s.fwd, s.inv, s.r, h.n, st)) {
+        launch_pointwise(s.residues, s.primes, s.zeta, s.r, h.n, n_sub, split, st);
+        launch_ntt_inverse(s.residues, s.primes, s.inv, s.r, h.n, n_sub, 0, split, st);
+    }
     // outputs: CRT GEMM and reduction per chunk, each chunk's copy-out overlapping the next
     // chunk's work. With wide rows the transpose also goes chunk by chunk, so only the first
     // chunk's share sits between the inverse NTT and the first copy-out.

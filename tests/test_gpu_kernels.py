@@ -110,3 +110,14 @@ def test_segmented_reduction(n, limbs, fpc, inputs, oracle, torch):
         pairs += [(inputs.edge_operand(n, q, x), inputs.edge_operand(n, q, y)) for x, y in inputs.EDGE_PAIRS]
         for a, b in pairs:
             assert np.array_equal(device_product(fpc, torch, q, a, b), oracle.kronecker(q, a, b))
+
+
+# every length of the fused transforms, with as few primes as possible and with more than one per SM
+@pytest.mark.parametrize("n", [256, 512, 1024, 2048, 4096, 8192])
+@pytest.mark.parametrize("limbs", [1, 75, 150])
+def test_fused_transforms(n, limbs, fpc, inputs, oracle, torch):
+    q, a, b = inputs.instance(n, limbs, 60 + limbs, 0)
+    want = oracle.kronecker(q, a, b)
+    assert np.array_equal(device_product(fpc, torch, q, a, b), want)
+    with fpc.Plan(n, 32 * limbs, limbs, q) as plan:
+        assert np.array_equal(plan.run(a, b), want)
