@@ -181,8 +181,19 @@ __device__ __forceinline__ void tmem_load4(uint32_t taddr, uint32_t (&v)[4]) {
 
 __device__ __forceinline__ void tmem_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
+__device__ __forceinline__ uint64_t mad_wide(uint32_t a, uint32_t b, uint64_t c) {
+    uint64_t d;
+    asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(d) : "r"(a), "r"(b), "l"(c));
+    return d;
+}
+
+// sum_d v_d 256^d of four byte dots. With K <= 256 bytes a dot is at most 256 * 255^2, and
+// v_0 + 256 v_1 <= 257 * 256 * 255^2 < 2^32: two of the three steps are 32-bit. The epilogue is
+// bound by the integer pipes (two warps per scheduler, 16 lanes wide), so each step counts.
+template <bool kShort>
 __device__ __forceinline__ uint64_t word_sum(uint32_t v0, uint32_t v1, uint32_t v2, uint32_t v3) {
-    return uint64_t(v0) + (uint64_t(v1) << 8) + (uint64_t(v2) << 16) + (uint64_t(v3) << 24);
+    if (kShort) return mad_wide(v2 + v3 * 256u, 65536u, v0 + v1 * 256u);
+    return mad_wide(v3, 1u << 24, mad_wide(v2, 65536u, mad_wide(v1, 256u, v0)));
 }
 
 __device__ __forceinline__ void cp_async_4(uint32_t smem, const void* global, uint32_t bytes) {  // 0: zero fill
@@ -229,8 +240,7 @@ __device__ __forceinline__ void epilogue_chunk(const Epilogue& epi, const uint32
     uint64_t sum[8];
 #pragma unroll
     for (int g = 0; g < 8; ++g)
-        sum[g] = uint64_t(v[4 * g]) + (uint64_t(v[4 * g + 1]) << 8) + (uint64_t(v[4 * g + 2]) << 16) +
-                 (uint64_t(v[4 * g + 3]) << 24);
+        sum[g] = word_sum<false>(v[4 * g], v[4 * g + 1], v[4 * g + 2], v[4 * g + 3]);
     // the lane's 8 words are consecutive in its row: two whole 32-byte sectors (the work space is
     // 256-byte aligned, rows are a multiple of 8 words, the chunk starts at a multiple of 8 words)
     const uint32_t g0 = c_base / 4;
@@ -258,12 +268,14 @@ __device__ __forceinline__ void epilogue_chunk(const Epilogue& epi, const uint32
 // What bounds it: with few K steps per tile the epilogue is the tile's longest part, and a warp by
 // itself leaves its scheduler idle four cycles out of five (2140 instructions in 10.5k cycles per
 // 256 x 256 tile with one warp per quarter). Two warps per quarter share the tile.
+template <bool kShort>
 __device__ __forceinline__ void epilogue_rows(const Epilogue& epi, uint32_t t_base, uint32_t col0, uint32_t columns,
                                               uint32_t chunks, bool row_ok, uint64_t out_row, uint32_t op,
                                               uint32_t column) {
     if (epi.mode == kEpilogueConvert) {
         const uint32_t k0 = col0 / 4;
-        uint32_t* out = epi.residues + (size_t(op) * epi.r + k0) * epi.n + column;  // + g * N for prime k0 + g
+        // byte offset of prime k0's value in the residues (2 r N words, below 4 GB), then + 4 N per prime
+        uint32_t at = ((op * epi.r + k0) * epi.n + column) * 4u;
 #pragma unroll 1
         for (uint32_t chunk = 0; chunk < chunks; ++chunk) {
             if (k0 + chunk * 8 >= epi.r) break;  // warp-uniform
@@ -275,12 +287,15 @@ __device__ __forceinline__ void epilogue_rows(const Epilogue& epi, uint32_t t_ba
             }
             uint32_t v[32];
             tmem_load32(t_base + chunk * 32, v);
+            const bool whole = k0 + chunk * 8 + 8 <= epi.r;
 #pragma unroll
             for (uint32_t g = 0; g < 8; ++g) {
-                const uint64_t s = uint64_t(v[4 * g]) + (uint64_t(v[4 * g + 1]) << 8) +
-                                   (uint64_t(v[4 * g + 2]) << 16) + (uint64_t(v[4 * g + 3]) << 24);
-                if (row_ok && k0 + chunk * 8 + g < epi.r) *out = redc(s, prime[g].x, prime[g].y);
-                out += epi.n;
+                const uint64_t s = word_sum<kShort>(v[4 * g], v[4 * g + 1], v[4 * g + 2], v[4 * g + 3]);
+                const uint32_t m = uint32_t(s) * prime[g].y;
+                const uint32_t u = reduce_once(uint32_t(mad_wide(m, prime[g].x, s) >> 32), prime[g].x);
+                if (row_ok && (whole || k0 + chunk * 8 + g < epi.r))
+                    *reinterpret_cast<uint32_t*>(reinterpret_cast<uint8_t*>(epi.residues) + at) = u;
+                at += 4u * epi.n;
             }
         }
         return;
@@ -313,9 +328,9 @@ __device__ __forceinline__ void reduce_rows(const ReduceParams& prm, uint32_t t_
     tmem_wait();
     uint64_t x[3], window[kWindow];
 #pragma unroll
-    for (int i = 0; i < 3; ++i) x[i] = word_sum(vx[i][0], vx[i][1], vx[i][2], vx[i][3]);
+    for (int i = 0; i < 3; ++i) x[i] = word_sum<false>(vx[i][0], vx[i][1], vx[i][2], vx[i][3]);
 #pragma unroll
-    for (int j = 0; j < kWindow; ++j) window[j] = word_sum(vw[j][0], vw[j][1], vw[j][2], vw[j][3]);
+    for (int j = 0; j < kWindow; ++j) window[j] = word_sum<false>(vw[j][0], vw[j][1], vw[j][2], vw[j][3]);
     const RowQuotient f = row_quotient(x, window, prm);
     RowState st;
     uint32_t* out = prm.out + size_t(first) * limbs;
@@ -333,7 +348,7 @@ __device__ __forceinline__ void reduce_rows(const ReduceParams& prm, uint32_t t_
             uint32_t v[32];
             tmem_load32(t_base + 4 * base + 32 * h, v);
 #pragma unroll
-            for (uint32_t i = 0; i < 8; ++i) d[8 * h + i] = word_sum(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+            for (uint32_t i = 0; i < 8; ++i) d[8 * h + i] = word_sum<false>(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
         }
         if (base + 16 >= tlen) {  // the accumulator's last columns are in registers
             fence_before();
@@ -417,7 +432,10 @@ __global__ void __launch_bounds__(kSource == kSourceTma ? kThreads : kGatherThre
     __syncthreads();
     fence_after();
     const uint32_t tmem = *tmem_slot;
-    chain_enter();
+    // With gathered A only the loaders wait for the kernel before this one: B tiles and every other
+    // table are constant, so the producer fetches B ahead of it, and the MMAs and the epilogue follow
+    // the loaders' stages.
+    if (kSource == kSourceTma) chain_enter();
 
     if (warp == 0) {
         if (lane == 0) {
@@ -498,6 +516,7 @@ __global__ void __launch_bounds__(kSource == kSourceTma ? kThreads : kGatherThre
         }
     } else if (kSource != kSourceTma && warp >= 2 + kEpilogueWarps) {
         // ---------------- A loaders
+        chain_enter();
         const uint32_t part = warp - (2 + kEpilogueWarps);  // rows 32 part .. 32 part + 31 of the tile
         const uint32_t a_addr = smem_u32(a_smem) + part * 32 * kBlockK;
         uint32_t step = 0, published = 0;
@@ -605,7 +624,7 @@ __global__ void __launch_bounds__(kSource == kSourceTma ? kThreads : kGatherThre
                     out_row = kSource == kSourceResidues ? shape.rows.coefficient(row) : shape.rows.row(row);
             }
             const uint32_t t_base = tmem + acc * kAccColumns + half * (shape.block_n / 2) + ((quarter * 32) << 16);
-            epilogue_rows(epi, t_base, col0 + half * (shape.block_n / 2), shape.columns, shape.block_n / 64, row_ok,
+            epilogue_rows<kSource == kSourceRows>(epi, t_base, col0 + half * (shape.block_n / 2), shape.columns, shape.block_n / 64, row_ok,
                           out_row, op, column);
             // every tcgen05.ld of this warp has completed (tmem_load32 waits): release the accumulator
             fence_before();
@@ -937,7 +956,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                     out_row = shape.rows.row(row);
             }
             const uint32_t t_base = tmem + acc * kAccColumns + half * (kBlockN / 2) + ((quarter * 32) << 16);
-            epilogue_rows(epi, t_base, col0 + half * (kBlockN / 2), shape.columns, kBlockN / 64, row_ok,
+            epilogue_rows<false>(epi, t_base, col0 + half * (kBlockN / 2), shape.columns, kBlockN / 64, row_ok,
                           out_row, op, column);
             fence_before();
             __syncwarp();

@@ -552,9 +552,15 @@ template <uint32_t kLog>
 __global__ void __launch_bounds__(2 * (1u << kLog) / per_thread(kLog), (kLog >= 12 ? 2 : 4))
     ntt_product_kernel(uint32_t* residues, const DevicePrime* __restrict__ primes, const uint2* __restrict__ fwd,
                        const uint2* __restrict__ inv, uint32_t r) {
-    chain_enter();
     extern __shared__ uint32_t xs[];
     constexpr uint32_t kN = 1u << kLog, kThreads = kN / per_thread(kLog);
+    // the prime's twiddles into L1 while the conversion finishes: one load per 128-byte line
+    for (uint32_t i = threadIdx.x * 16; i < 2 * kN; i += 2 * kThreads * 16) {
+        const uint2* line = (i < kN ? fwd : inv) + size_t(blockIdx.x) * kN + i % kN;
+        uint32_t unused;
+        asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(unused) : "l"(line));
+    }
+    chain_enter();
     constexpr int R = kLog % 4 && kLog != 13 ? int(kLog % 4) : 4;  // of the forward's last and the inverse's first pass
     constexpr int G = per_thread(kLog) >> R;
     const uint32_t k = blockIdx.x, op = threadIdx.x / kThreads, tid = threadIdx.x % kThreads;

@@ -5,8 +5,8 @@
 // finishes.
 //
 // Rules that keep this equal to plain stream order:
-//  * every kernel of the chain calls chain_wait() in every thread before it touches memory that a
-//    kernel writes (chain_wait returns once the kernel before it has completed and its writes are
+//  * every kernel of the chain calls chain_wait() in every block, and in every thread that touches
+//    memory that a kernel writes or follows one that waited, before that (chain_wait returns once the kernel before it has completed and its writes are
 //    visible). Since that kernel waited likewise, everything earlier on the stream has completed too;
 //  * chain_release(), which lets the next kernel's blocks be placed, comes after chain_wait(), so at
 //    most two kernels of a stream are resident, and two CTA-pair GEMMs never are: another kernel
