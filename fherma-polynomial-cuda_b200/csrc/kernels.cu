@@ -278,13 +278,14 @@ constexpr uint32_t per_thread(uint32_t log) { return log == 13 ? 32 : 16; }  // 
 // swizzle of base (once per group) XOR a compile-time constant.
 template <uint32_t kLog>
 __host__ __device__ constexpr uint32_t swizzle_column(int b) {
+    constexpr uint32_t c6[] = {1}, c7[] = {1, 2};  // short transforms share a warp; any column does
     constexpr uint32_t c8[] = {30, 1, 4};
     constexpr uint32_t c9[] = {7, 9, 27, 13};
     constexpr uint32_t c10[] = {27, 13, 8, 26, 8};
     constexpr uint32_t c11[] = {11, 1, 14, 20, 24, 27};
     constexpr uint32_t c12[] = {17, 26, 2, 21, 24, 25, 27};
     constexpr uint32_t c13[] = {1, 2, 4, 24, 0, 0, 0, 0};
-    return kLog == 8 ? c8[b] : kLog == 9 ? c9[b] : kLog == 10 ? c10[b] : kLog == 11 ? c11[b] : kLog == 12 ? c12[b] : c13[b];
+    return kLog == 6 ? c6[b] : kLog == 7 ? c7[b] : kLog == 8 ? c8[b] : kLog == 9 ? c9[b] : kLog == 10 ? c10[b] : kLog == 11 ? c11[b] : kLog == 12 ? c12[b] : c13[b];
 }
 
 template <uint32_t kLog>
@@ -524,14 +525,16 @@ __global__ void __launch_bounds__((1u << kLog) / per_thread(kLog), 4) ntt_invers
 // Two launches and two round trips through L2 less. Product, us, three kernels / one: 17.7 / 12.4 at
 // N = 256, L = 2; 17.5 / 14.5 at N = 2048, L = 13; 38.5 / 34.8 at N = 4096, L = 64; 85.6 / 74.0 at
 // N = 8192, L = 128; 791 / 721 at N = 8192, L = 868 (33.0 / 33.6 at N = 2048, L = 94: 197 CTAs).
-template <uint32_t kLog, uint32_t kDone>
-__device__ __forceinline__ void forward_to_middle(uint32_t tid, uint32_t* data, uint32_t* xs,
+template <uint32_t kLog, uint32_t kDone, bool kGlobalInput>
+__device__ __forceinline__ void forward_to_middle(bool active, uint32_t tid, uint32_t* data, uint32_t* xs,
                                                   const uint2* __restrict__ table, uint32_t p) {
     constexpr int R = ntt_pass_stages(true, kLog, kDone);
+    constexpr bool kGlobal = kGlobalInput && kDone == 0;
     if constexpr (kDone + R < kLog) {
-        ntt_pass<R, true, kDone == 0, false, false, kLog - kDone - R, kLog>(tid, kDone == 0 ? data : xs, xs, table, p, 0, 0);
+        if (active)
+            ntt_pass<R, true, kGlobal, false, false, kLog - kDone - R, kLog>(tid, kGlobal ? data : xs, xs, table, p, 0, 0);
         __syncthreads();
-        forward_to_middle<kLog, kDone + R>(tid, data, xs, table, p);
+        forward_to_middle<kLog, kDone + R, kGlobalInput>(active, tid, data, xs, table, p);
     }
 }
 
@@ -568,7 +571,7 @@ __global__ void __launch_bounds__(2 * (1u << kLog) / per_thread(kLog), (kLog >= 
     uint32_t* data = residues + (size_t(op) * r + k) * kN;
     uint32_t* own = xs + op * kN;
     const uint2 *forward = fwd + size_t(k) * kN, *inverse = inv + size_t(k) * kN;
-    forward_to_middle<kLog, 0>(tid, data, own, forward, f.p);
+    forward_to_middle<kLog, 0, true>(true, tid, data, own, forward, f.p);
     constexpr bool kPaired = kLog == 13;
     uint32_t x[G][1 << R];
 #pragma unroll
@@ -597,6 +600,151 @@ __global__ void __launch_bounds__(2 * (1u << kLog) / per_thread(kLog), (kLog >= 
         }
     }
     inverse_from_middle<kLog, R>(op == 0, tid, data, xs, inverse, f.p, f.finish, f.finish_q);
+}
+
+// ntt_product_kernel's middle, from the forward transforms' last pass through the products to the
+// inverse's first, for a block of several primes' transforms (as one function for both, the kernel
+// above spills and takes 4 % longer). `a` and b are
+// the operands' transforms in shared memory, b's b_offset words after a's, of which this thread works
+// on number `op`.
+template <uint32_t kLog>
+__device__ __forceinline__ void middle_passes(bool active, uint32_t tid, uint32_t op, uint32_t* a, uint32_t b_offset,
+                                              const uint2* __restrict__ forward, const uint2* __restrict__ inverse,
+                                              const DevicePrime& f) {
+    uint32_t* own = a + op * b_offset;
+    constexpr uint32_t kThreads = (1u << kLog) / per_thread(kLog);
+    constexpr int R = ntt_pass_stages(false, kLog, 0);  // of the forward's last and the inverse's first pass
+    constexpr int G = per_thread(kLog) >> R;
+    constexpr bool kPaired = kLog == 13;
+    uint32_t x[G][1 << R];
+    if (active) {
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+            const uint32_t group = tid + g * kThreads, placed = swizzle<kLog>(group << R);
+#pragma unroll
+            for (int i = 0; i < (1 << R); ++i) x[g][i] = own[placed ^ swizzle<kLog>(uint32_t(i))];
+            ct_stages<R, kPaired>(x[g], group, 0, kLog, forward, f.p);
+#pragma unroll
+            for (int i = 0; i < (1 << R); ++i) {
+                x[g][i] = reduce_once(x[g][i], f.p);
+                if (op == 1) own[placed ^ swizzle<kLog>(uint32_t(i))] = x[g][i];
+            }
+        }
+    }
+    __syncthreads();
+    if (active && op == 0) {
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+            const uint32_t group = tid + g * kThreads, placed = swizzle<kLog>(group << R);
+#pragma unroll
+            for (int i = 0; i < (1 << R); ++i)
+                x[g][i] = mont(x[g][i], a[b_offset + (placed ^ swizzle<kLog>(uint32_t(i)))], f.p, f.pinv);
+            gs_stages<R, kPaired>(x[g], group, 0, kLog, inverse, f.p);
+#pragma unroll
+            for (int i = 0; i < (1 << R); ++i) a[placed ^ swizzle<kLog>(uint32_t(i))] = x[g][i];
+        }
+    }
+}
+
+// A whole product of a small unsplit ring in one CTA: conversion, transforms, CRT and reduction. Such a
+// product is bound by its launches (three cost the host 9 to 13 us, more than the device needs), so all
+// of it is one. The conversion and the CRT are plain sums here: residue = sum_j REDC(limb_j c_j) with
+// c_j = 2^(32j) mod p, and the words of sum_k v_k W_k by a 96-bit accumulator per coefficient.
+// N = 256, L = 2: 12.0 -> 9.7 us; N = 64, L = 2: 19.7 -> 7.5 us.
+constexpr uint32_t kSmallPrimes = 64;
+template <uint32_t kLog>
+__global__ void __launch_bounds__(512) small_product_kernel(SmallProduct prm) {
+    extern __shared__ uint32_t xs[];
+    constexpr uint32_t kN = 1u << kLog, kThreads = kN / per_thread(kLog);
+    const uint32_t r = prm.r, limbs = prm.reduce.limbs, words = limbs + 5;
+    uint32_t* const v = xs + r * kN;             // operand b's transforms, later the residues v_k
+    uint32_t* const rows = v + r * kN;           // [2][N][limbs] operands
+    uint32_t* const digits = rows;               // [words][N] of the CRT sum, later
+    uint32_t* const c = rows + max(2 * limbs, words) * kN;  // [r][limbs]
+    uint32_t* const crt = c + r * limbs;                    // [r][words]
+    uint32_t* const tables = crt + r * words;               // q, then -P mod q: limbs + 2 words each
+    __shared__ DevicePrime primes[kSmallPrimes];
+    // constants first: the kernel before may still be running
+    for (uint32_t i = threadIdx.x; i < r * limbs; i += blockDim.x) {
+        const uint8_t* w = prm.convert_weights + size_t(4 * (i / limbs)) * prm.k_bytes + 4 * (i % limbs);
+        c[i] = w[0] | uint32_t(w[prm.k_bytes]) << 8 | uint32_t(w[2 * prm.k_bytes]) << 16 | uint32_t(w[3 * prm.k_bytes]) << 24;
+    }
+    for (uint32_t i = threadIdx.x; i < r * words; i += blockDim.x) crt[i] = prm.crt_words[i];
+    for (uint32_t i = threadIdx.x; i < limbs + 2; i += blockDim.x) {
+        tables[i] = prm.reduce.q[i];
+        tables[limbs + 2 + i] = prm.reduce.minus_p[i];
+    }
+    if (threadIdx.x < r) primes[threadIdx.x] = prm.primes[threadIdx.x];
+    for (uint32_t i = threadIdx.x * 16; i < 2 * r * kN; i += blockDim.x * 16) {  // twiddles into L1
+        const uint2* line = i < r * kN ? prm.fwd + i : prm.inv + (i - r * kN);
+        uint32_t unused;
+        asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(unused) : "l"(line));
+    }
+    chain_enter();
+    for (uint32_t i = threadIdx.x; i < kN * limbs; i += blockDim.x) {
+        rows[i] = prm.a[i];
+        rows[kN * limbs + i] = prm.b[i];
+    }
+    __syncthreads();
+#pragma unroll 4
+    for (uint32_t i = threadIdx.x; i < 2 * r * kN; i += blockDim.x) {
+        const uint32_t row = i / kN, op = row >= r ? 1 : 0, k = row - op * r;
+        const uint32_t p = primes[k].p, pinv = primes[k].pinv;
+        const uint32_t* x = rows + (op * kN + i % kN) * limbs;
+        uint32_t sum = 0;
+        for (uint32_t j = 0; j < limbs; ++j) sum = add_mod(sum, redc(uint64_t(x[j]) * c[k * limbs + j], p, pinv), p);
+        xs[row * kN + swizzle<kLog>(i % kN)] = sum;
+    }
+    __syncthreads();
+    {
+        const uint32_t team = threadIdx.x / (2 * kThreads), op = threadIdx.x / kThreads % 2, tid = threadIdx.x % kThreads;
+        const bool active = team < r;
+        const uint32_t k = active ? team : 0;
+        const DevicePrime f = primes[k];
+        const uint2 *forward = prm.fwd + k * kN, *inverse = prm.inv + k * kN;
+        uint32_t *a = xs + k * kN, *b = v + k * kN;
+        forward_to_middle<kLog, 0, false>(active, tid, nullptr, op ? b : a, forward, f.p);
+        middle_passes<kLog>(active, tid, op, a, r * kN, forward, inverse, f);
+        // the last pass writes v_k in plain order over b's transform
+        inverse_from_middle<kLog, ntt_pass_stages(false, kLog, 0)>(active && op == 0, tid, b, a, inverse, f.p, f.finish,
+                                                                    f.finish_q);
+    }
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < r * kN; i += blockDim.x) prm.residues[i] = v[i];
+    ReduceParams red = prm.reduce;
+    red.q = tables;
+    red.minus_p = tables + limbs + 2;
+    for (uint32_t i = threadIdx.x; i < kN; i += blockDim.x) {
+        uint64_t low = 0;  // the running sum from word w up: 96 bits
+        uint32_t high = 0;
+        for (uint32_t w = 0; w < words; ++w) {
+#pragma unroll 4
+            for (uint32_t k = 0; k < r; ++k) {
+                const uint64_t product = uint64_t(v[k * kN + i]) * crt[k * words + w];
+                low += product;
+                high += low < product ? 1 : 0;
+            }
+            digits[w * kN + i] = uint32_t(low);
+            low = (low >> 32) | (uint64_t(high) << 32);
+            high = 0;
+        }
+        const uint64_t x[3] = {digits[(limbs + 2) * kN + i], digits[(limbs + 3) * kN + i], digits[(limbs + 4) * kN + i]};
+        uint64_t window[kWindow];
+#pragma unroll
+        for (int j = 0; j < kWindow; ++j) {
+            uint32_t w;
+            window[j] = window_word(red, j, w) ? digits[w * kN + i] : 0;
+        }
+        const RowQuotient f = row_quotient(x, window, red);
+        RowState st;
+        uint32_t* out = red.out + i * limbs;
+        for (uint32_t w = 0; w < limbs + 2; ++w) {
+            const uint32_t o = st.word(f, digits[w * kN + i], red.minus_p[w], red.q[w]);
+            st.note(o, w, red);
+            if (w < limbs) out[w] = o;
+        }
+        st.finish(out, red);
+    }
 }
 
 // C_v = sum_{t+u=v} A_t B_u + zeta * sum_{t+u=v+s} A_t B_u at every evaluation point,
@@ -990,9 +1138,44 @@ static void launch_product(uint32_t* residues, const DevicePrime* primes, const 
     launch_chained(ntt_product_kernel<kLog>, r, 2 * kN / per_thread(kLog), kSmem, stream, residues, primes, fwd, inv, r);
 }
 
+static uint32_t small_threads(uint32_t n, uint32_t r) { return std::max(256u, (n / 8 * r + 31) / 32 * 32); }
+
+static size_t small_smem(uint32_t n, uint32_t r, uint32_t limbs) {
+    return (size_t(n) * (2 * r + std::max(2 * limbs, limbs + 5)) + size_t(r) * (2 * limbs + 5) + 2 * (limbs + 2)) *
+           sizeof(uint32_t);
+}
+
+// The line lies where the three kernels catch up. Product, us, one kernel / three, at N r L of:
+// 2560 (N=256, L=2) 9.7 / 12.0, 4608 (N=128, L=4) 9.0 / 12.3, 9216 (N=256, L=4) 14.1 / 12.0, 16384 (N=128,
+// L=8) 15.5 / 12.3, 5120 (N=512, L=2) 16.0 / 12.0. At N=64 the tensor GEMMs do not apply: 6272 (L=7) 11.3 /
+// 19.8, 16896 (L=11) 18.1 / 20.
+bool small_product_takes(uint32_t n, uint32_t r, uint32_t limbs) {
+    return n >= 64 && n <= 256 && r <= kSmallPrimes && small_threads(n, r) <= 512 &&
+           uint64_t(n) * r * limbs <= (n == 64 ? 12288 : 5000);
+}
+
+template <uint32_t kLog>
+static void launch_small(const SmallProduct& params, cudaStream_t stream) {
+    constexpr uint32_t kN = 1u << kLog;
+    const size_t smem = small_smem(kN, params.r, params.reduce.limbs);
+    if (smem > 48 * 1024)  // per device; cheap enough to repeat
+        cudaFuncSetAttribute(small_product_kernel<kLog>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    launch_chained(small_product_kernel<kLog>, 1, small_threads(kN, params.r), smem, stream, params);
+}
+
+void launch_small_product(const SmallProduct& params, cudaStream_t stream) {
+    switch (params.reduce.n) {
+        case 64: launch_small<6>(params, stream); break;
+        case 128: launch_small<7>(params, stream); break;
+        default: launch_small<8>(params, stream); break;
+    }
+}
+
 bool launch_ntt_product(uint32_t* residues, const DevicePrime* primes, const uint2* fwd, const uint2* inv, uint32_t r,
                         uint32_t n, cudaStream_t stream) {
     switch (n) {
+        case 64: launch_product<6>(residues, primes, fwd, inv, r, stream); return true;
+        case 128: launch_product<7>(residues, primes, fwd, inv, r, stream); return true;
         case 256: launch_product<8>(residues, primes, fwd, inv, r, stream); return true;
         case 512: launch_product<9>(residues, primes, fwd, inv, r, stream); return true;
         case 1024: launch_product<10>(residues, primes, fwd, inv, r, stream); return true;

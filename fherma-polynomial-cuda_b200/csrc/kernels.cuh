@@ -137,6 +137,20 @@ void launch_ntt_inverse(uint32_t* residues, const DevicePrime* primes, const uin
 void launch_transpose(const uint32_t* residues, uint32_t* crt_in, uint32_t r, uint32_t padded_r,
                       uint32_t n, uint32_t split, uint32_t j_first, uint32_t j_count, cudaStream_t stream);
 
+// A whole product in one kernel, where small_product_takes the ring, the primes and the limbs.
+struct SmallProduct {
+    const uint32_t *a, *b;           // [N][L]
+    const DevicePrime* primes;
+    const uint2 *fwd, *inv;          // [r][N]
+    const uint8_t* convert_weights;  // [4r'][k_bytes]
+    uint32_t k_bytes, r;
+    const uint32_t* crt_words;       // [r][L+5]: W_k
+    uint32_t* residues;              // receives v_k, [r][N]
+    ReduceParams reduce;             // n = N; dots not used
+};
+bool small_product_takes(uint32_t n, uint32_t r, uint32_t limbs);
+void launch_small_product(const SmallProduct& params, cudaStream_t stream);
+
 // Words the tables of launch_reduce hold: whole chunks of 64 covering L + 2 words.
 constexpr uint32_t reduce_table_words(uint32_t limbs) { return (limbs + 2 + 63) / 64 * 64; }
 void launch_reduce(const ReduceParams& params, cudaStream_t stream);

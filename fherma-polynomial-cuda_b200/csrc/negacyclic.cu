@@ -189,6 +189,24 @@ void enqueue_middle(negacyclic_plan& s, cudaStream_t stream, cudaEvent_t* marks)
     mark();
 }
 
+// The whole product of a small ring.
+void enqueue_small(negacyclic_plan& s, const uint32_t* a, const uint32_t* b, uint32_t* d_c, cudaStream_t stream) {
+    SmallProduct small{};
+    small.a = a;
+    small.b = b;
+    small.primes = s.primes;
+    small.fwd = s.fwd;
+    small.inv = s.inv;
+    small.convert_weights = s.convert_weights;
+    small.k_bytes = s.k_convert;
+    small.r = s.r;
+    small.crt_words = s.crt_words;
+    small.residues = s.residues;
+    small.reduce = reduce_params(s, 0, s.host.n, d_c);
+    launch_small_product(small, stream);
+    check(cudaGetLastError(), "product kernel");
+}
+
 // Pads the operands on `stream`, where the conversion reads them padded.
 void enqueue_pad(negacyclic_plan& s, const uint32_t* d_a, const uint32_t* d_b, cudaStream_t stream) {
     if (s.convert_rows.ready) return;
@@ -303,6 +321,10 @@ std::string bind_work(negacyclic_plan& s, void* arena) {
 
 void enqueue_device_product(negacyclic_plan& s, const uint32_t* d_a, const uint32_t* d_b, uint32_t* d_c,
                             cudaStream_t stream) {
+    if (s.small) {
+        enqueue_small(s, d_a, d_b, d_c, stream);
+        return;
+    }
     enqueue_pad(s, d_a, d_b, stream);
     enqueue_product(s, d_a, d_b, d_c, stream);
 }
@@ -410,7 +432,7 @@ int negacyclic_init(uint32_t n, uint32_t w, uint32_t limbs, const uint32_t* q, c
         device_alloc(s.minus_p, table_words, tables);
         device_alloc(s.own_status, 64, tables);
         s.status = s.own_status;
-        device_alloc(s.crt_words, size_t(s.r) * h.words, work);  // freed once the CRT weights are built
+        device_alloc(s.crt_words, size_t(s.r) * h.words, work);  // freed once the CRT weights are built, unless small
         work = 0;
         s.work_bytes = work_layout(s).total;
         if (!o.external_work) {
@@ -439,8 +461,11 @@ int negacyclic_init(uint32_t n, uint32_t w, uint32_t limbs, const uint32_t* q, c
         launch_crt_weights(s.crt_words, s.r, s.padded_r, h.words, s.crt_columns, s.crt_weights, st);
         check(cudaGetLastError(), "table kernels");
         check(cudaStreamSynchronize(st), "plan tables");
-        cudaFree(s.crt_words);
-        s.crt_words = nullptr;
+        s.small = o.gemm == NEGACYCLIC_GEMM_AUTO && h.split == 1 && small_product_takes(h.n, s.r, limbs);
+        if (!s.small) {
+            cudaFree(s.crt_words);
+            s.crt_words = nullptr;
+        }
 
         s.gemm_tensor_wanted = o.gemm != NEGACYCLIC_GEMM_SIMT;
         s.gemm_tensor_required = o.gemm == NEGACYCLIC_GEMM_TENSOR || o.gemm == NEGACYCLIC_GEMM_TENSOR_SINGLE;
@@ -519,7 +544,7 @@ int negacyclic_get_info(const negacyclic_plan* s, negacyclic_info* info) {
     info->split = h.split;
     info->n_sub = h.n_sub;
     info->words = h.words;
-    info->gemm = (s->convert_engine == NEGACYCLIC_GEMM_TENSOR || s->convert_rows.ready ? 1u : 0u) |
+    info->gemm = s->small ? 0u : (s->convert_engine == NEGACYCLIC_GEMM_TENSOR || s->convert_rows.ready ? 1u : 0u) |
                  (s->crt_engine == NEGACYCLIC_GEMM_TENSOR || s->crt_gather.ready ? 2u : 0u);
     info->q_bits = h.q_bits;
     info->device_bytes = s->device_bytes;
@@ -553,9 +578,14 @@ int negacyclic_run_device_timed(negacyclic_plan* s, const uint32_t* d_a, const u
     try {
         for (auto& e : events) check(cudaEventCreate(&e), "cudaEventCreate");
         check(cudaEventRecord(events[0], stream), "cudaEventRecord");
-        enqueue_pad(*s, d_a, d_b, stream);
-        check(cudaEventRecord(events[1], stream), "cudaEventRecord");
-        enqueue_product(*s, d_a, d_b, d_c, stream, events + 2);
+        if (s->small) {  // all of it in the first stage
+            enqueue_small(*s, d_a, d_b, d_c, stream);
+            for (uint32_t i = 1; i <= kStages + 1; ++i) check(cudaEventRecord(events[i], stream), "cudaEventRecord");
+        } else {
+            enqueue_pad(*s, d_a, d_b, stream);
+            check(cudaEventRecord(events[1], stream), "cudaEventRecord");
+            enqueue_product(*s, d_a, d_b, d_c, stream, events + 2);
+        }
         check(cudaEventSynchronize(events[kStages + 1]), "product");
         for (uint32_t i = 0; i <= kStages; ++i)
             check(cudaEventElapsedTime(&stage_ms[i], events[i], events[i + 1]), "cudaEventElapsedTime");
@@ -642,6 +672,7 @@ void host_begin(negacyclic_plan& s, const uint32_t* a, const uint32_t* b, uint32
     std::vector<OutChunk> out;
     const bool ordered = transform_ordered_input(chunk_shape(s));
     stream_chunks(chunk_shape(s), ordered, in, out);
+    const uint32_t* small_rows = nullptr;  // where the operands of a small product land
     const bool fuse_ntt = s.ntt_fused() && in.size() == 1;  // in pieces, a's transforms run while b is on the link
     uint32_t pieces[negacyclic_plan::kMaxChunks] = {};  // pack pieces per input chunk
     if (!a_locked || !b_locked) {
@@ -722,6 +753,7 @@ void host_begin(negacyclic_plan& s, const uint32_t* a, const uint32_t* b, uint32
     } else {
         const bool direct = s.padded_limbs == h.limbs && split == 1;
         uint32_t* staged = direct ? s.operands : reinterpret_cast<uint32_t*>(s.dots);
+        small_rows = staged;
         for (uint32_t k = 0; k < in.size(); ++k) {
             const size_t first = in[k].j0, count = in[k].span, bytes = count * row;  // coefficient range
             const uint32_t op_first = in[k].op == InChunk::kBothOperands ? 0u : in[k].op;
@@ -736,6 +768,7 @@ void host_begin(negacyclic_plan& s, const uint32_t* a, const uint32_t* b, uint32
             }
             check(cudaEventRecord(s.in_ready[k], s.copy_in), "cudaEventRecord");
             check(cudaStreamWaitEvent(st, s.in_ready[k], 0), "cudaStreamWaitEvent");
+            if (s.small) continue;  // one piece; the whole product follows
             if (!direct && !s.convert_rows.ready)
                 launch_pad_rows(staged, s.operands, h.n, h.limbs, s.padded_limbs, split, uint32_t(first),
                                 uint32_t(count), st, op_first, op_count);
@@ -746,7 +779,9 @@ void host_begin(negacyclic_plan& s, const uint32_t* a, const uint32_t* b, uint32
                 launch_ntt_forward(s.residues, s.primes, s.fwd, s.r, h.n, n_sub, 0, split, st, op_first, op_count);
         }
     }
-    if (!fuse_ntt || !launch_ntt_product(s.residues, s.primes, s.fwd, s.inv, s.r, h.n, st)) {
+    if (s.small)
+        enqueue_small(s, small_rows, small_rows + words, s.result, st);
+    else if (!fuse_ntt || !launch_ntt_product(s.residues, s.primes, s.fwd, s.inv, s.r, h.n, st)) {
         launch_pointwise(s.residues, s.primes, s.zeta, s.r, h.n, n_sub, split, st);
         launch_ntt_inverse(s.residues, s.primes, s.inv, s.r, h.n, n_sub, 0, split, st);
     }
@@ -754,8 +789,8 @@ void host_begin(negacyclic_plan& s, const uint32_t* a, const uint32_t* b, uint32
     // chunk's work. With wide rows the transpose also goes chunk by chunk, so only the first
     // chunk's share sits between the inverse NTT and the first copy-out.
     uint32_t* dst = s.outputs_staged ? s.stage_out : c;
-    bool gather = s.crt_gather.ready;
-    for (const OutChunk& ch : out) gather = gather && gather_span(s, ch.first, ch.count);
+    bool gather = s.crt_gather.ready || s.small;
+    for (const OutChunk& ch : out) gather = gather && (s.small || gather_span(s, ch.first, ch.count));
     const bool transpose_per_chunk = wide_rows(chunk_shape(s)) && !gather;
     if (!transpose_per_chunk && !gather)
         launch_transpose(s.residues, s.crt_in, s.r, s.padded_r, h.n, split, 0, n_sub, st);
@@ -764,7 +799,7 @@ void host_begin(negacyclic_plan& s, const uint32_t* a, const uint32_t* b, uint32
             if (transpose_per_chunk)  // chunk coefficients are whole multiples of s
                 launch_transpose(s.residues, s.crt_in, s.r, s.padded_r, h.n, split, out[k].first / split,
                                  out[k].count / split, st);
-            enqueue_output(s, out[k].first, out[k].count, s.result, st, gather);
+            if (!s.small) enqueue_output(s, out[k].first, out[k].count, s.result, st, gather);
             check(cudaEventRecord(s.out_ready[k], st), "cudaEventRecord");
         }
         if (k >= 1) {
@@ -913,7 +948,7 @@ int negacyclic_debug_read(negacyclic_plan* s, int which, void* host, size_t* byt
     }
     if (*bytes < size) return fail(NEGACYCLIC_EINVAL, "host buffer too small");
     DeviceGuard guard(s->device);
-    if (which >= 1 && s->crt_gather.ready) {  // the product kept neither buffer: make them from its residues
+    if (which >= 1 && (s->crt_gather.ready || s->small)) {  // the product kept neither buffer: make them from its residues
         launch_transpose(s->residues, s->crt_in, s->r, s->padded_r, h.n, h.split, 0, h.n_sub, s->stream);
         if (which == 2) enqueue_crt_sums(*s, 0, h.n, s->stream, false);
         if (cudaStreamSynchronize(s->stream) != cudaSuccess)

@@ -61,9 +61,11 @@ struct negacyclic_plan {
     // where a row's word sums fit one tile (crt_reduces) the CRT GEMM also reduces mod q.
     negacyclic::TensorGemmPlan convert_rows, crt_gather;
     bool crt_reduces = false;
-    // Unsplit rings of 256 to 8192 coefficients: forward, pointwise and inverse in one kernel.
-    bool ntt_fused() const { return host.split == 1 && host.n >= 256 && host.n <= 8192; }
+    // Unsplit rings of 64 to 8192 coefficients: forward, pointwise and inverse in one kernel.
+    bool ntt_fused() const { return host.split == 1 && host.n >= 64 && host.n <= 8192; }
+    bool small = false;  // the whole product in one kernel (crt_words is kept for it)
     uint32_t kernels_per_product() const {
+        if (small) return 1;
         return 8 - (ntt_fused() ? 2 : 0) - (convert_rows.ready ? 1 : 0) - (crt_gather.ready ? 1 : 0) - (crt_reduces ? 1 : 0);
     }
 

@@ -126,13 +126,15 @@ struct RowState {
         }
         if (base + 16 + 2 > prm.q_words) {  // some of the top words
 #pragma unroll
-            for (uint32_t i = 0; i < 16; ++i) {
-                const uint32_t w = base + i;
-                if (w + 2 == prm.q_words) top0 = o[i];
-                if (w + 1 == prm.q_words) top1 = o[i];
-                if (w >= prm.q_words) over |= o[i];
-            }
+            for (uint32_t i = 0; i < 16; ++i) note(o[i], base + i, prm);
         }
+    }
+
+    // Keeps what finish() needs of word w of the result.
+    __device__ __forceinline__ void note(uint32_t o, uint32_t w, const ReduceParams& prm) {
+        if (w + 2 == prm.q_words) top0 = o;
+        if (w + 1 == prm.q_words) top1 = o;
+        if (w >= prm.q_words) over |= o;
     }
 
     // The same for a row whose words are only in global memory, `above` standing over them.

@@ -121,3 +121,35 @@ def test_fused_transforms(n, limbs, fpc, inputs, oracle, torch):
     assert np.array_equal(device_product(fpc, torch, q, a, b), want)
     with fpc.Plan(n, 32 * limbs, limbs, q) as plan:
         assert np.array_equal(plan.run(a, b), want)
+
+
+# rings that run as one kernel (N r L up to 5000, 12288 at N = 64) and their neighbours that do not
+@pytest.mark.parametrize("n,limbs", [(64, 1), (64, 2), (64, 8), (64, 9), (64, 10), (128, 1), (128, 3), (128, 4),
+                                     (128, 5), (256, 1), (256, 2), (256, 3), (512, 1), (32, 2), (2048, 1)])
+def test_small_products(n, limbs, fpc, inputs, oracle, torch):
+    top = 1 << (32 * limbs)
+    for qv in (inputs.to_int(inputs.random_modulus(limbs, n)), top - 1, top // 2 + 1, 3, (top >> 31) + 1):
+        q = inputs.from_int(qv, limbs)
+        rng = np.random.Generator(np.random.PCG64(limbs))
+        words = np.flatnonzero(q)[-1] + 1
+        pairs = [tuple(np.pad(inputs.random_operand(rng, n, q[:words]), ((0, 0), (0, limbs - words)))
+                       for _ in range(2))]
+        pairs += [(inputs.edge_operand(n, q, x), inputs.edge_operand(n, q, y)) for x, y in inputs.EDGE_PAIRS]
+        for a, b in pairs:
+            want = oracle.kronecker(q, a, b)
+            assert np.array_equal(device_product(fpc, torch, q, a, b), want)
+        with fpc.Plan(n, 32 * limbs, limbs, q) as plan:  # the last pair once more through the host path
+            assert np.array_equal(plan.run(a, b), want)
+
+
+def test_small_product_stages_match_the_general_path(fpc, inputs):
+    """The stage buffers of a one-kernel product are those of the same product in stages."""
+    n, limbs = 256, 3
+    q, a, b = inputs.instance(n, limbs, 6, 0)
+    dumps = []
+    for gemm in (fpc.GEMM_AUTO, fpc.GEMM_SIMT):
+        with fpc.Plan(n, 32 * limbs, limbs, q, gemm=gemm) as plan:
+            c = plan.run(a, b)
+            r = plan.info()["primes"]
+            dumps.append((c.tobytes(), plan.debug_read(0)[:r * n * 4], plan.debug_read(1), plan.debug_read(2)))
+    assert dumps[0] == dumps[1]
