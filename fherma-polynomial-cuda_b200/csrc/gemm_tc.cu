@@ -69,14 +69,16 @@ __device__ __forceinline__ uint32_t smem_u32(const void* ptr) {
 // UMMA shared-memory descriptor for a K-major tile in the canonical 128B-swizzle
 // layout: rows of 128 bytes, 8-row core groups 1024 bytes apart (SBO), tile base
 // 1024-byte aligned (base offset 0), descriptor version 1.
+// The fields above the address are constants, and the 14-bit address field never overflows into them
+// (shared-memory addresses end below 256 KB), so a descriptor is one 32-bit addition to a constant: the
+// issuing thread shares its scheduler with the epilogue, and with few K steps its own instructions
+// set the pace of a tile (64-bit field assembly per MMA: 1050 cycles a step against 611 of MMA time).
 __device__ __forceinline__ uint64_t smem_descriptor(uint32_t addr) {
-    uint64_t d = 0;
-    d |= uint64_t((addr & 0x3FFFFu) >> 4);
-    d |= uint64_t(1) << 16;           // leading byte offset (unused for swizzled K-major)
-    d |= uint64_t(1024 >> 4) << 32;   // stride byte offset
-    d |= uint64_t(1) << 46;           // version
-    d |= uint64_t(2) << 61;           // SWIZZLE_128B
-    return d;
+    constexpr uint32_t kLow = 1u << 16;          // leading byte offset (unused for swizzled K-major)
+    constexpr uint32_t kHigh = (1024u >> 4)      // stride byte offset
+                               | (1u << 14)      // version
+                               | (2u << 29);     // SWIZZLE_128B
+    return (uint64_t(kHigh) << 32) | (kLow + (addr >> 4));
 }
 
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
@@ -212,12 +214,18 @@ struct TileShape {
     long long limit;         // cycles any one pipeline wait may take
     uint32_t withheld;       // diagnostics: CTA (pair) 0's producer stops before this pipeline step
     uint32_t block_n;        // columns per tile: 256, or 128 (single-CTA kernel)
+    bool resident;           // gathered A: each CTA keeps its column tile of B (n fastest, grid % n_tiles = 0)
 };
 
 // Tile index -> (m tile, n tile) in groups of group_m m-tiles, m fastest, so the
 // CTAs running at the same time share B tiles (and their A tiles stay in L2).
 __device__ __forceinline__ void tile_coords(uint32_t tile, const TileShape& shape, uint32_t& m_tile,
                                             uint32_t& n_tile) {
+    if (shape.resident) {
+        m_tile = tile / shape.n_tiles;
+        n_tile = tile - m_tile * shape.n_tiles;
+        return;
+    }
     const uint32_t span = shape.group_m * shape.n_tiles;
     const uint32_t group = tile / span, within = tile - group * span;
     const uint32_t first_m = group * shape.group_m;
@@ -403,7 +411,8 @@ __global__ void __launch_bounds__(kSource == kSourceTma ? kThreads : kGatherThre
     uint64_t* acc_full = empty + kStages;  // [2] MMA -> epilogue
     uint64_t* acc_empty = acc_full + 2;    // [2] epilogue -> MMA
     uint64_t* drain = acc_empty + 2;       // MMA warp's final completion
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 1);
+    uint64_t* b_full = drain + 1;          // resident B has landed
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(b_full + 1);
     volatile uint32_t* abort_flag = tmem_slot + 1;
 
     const uint32_t warp = threadIdx.x / 32, lane = threadIdx.x % 32;
@@ -411,7 +420,7 @@ __global__ void __launch_bounds__(kSource == kSourceTma ? kThreads : kGatherThre
 
     if (threadIdx.x == 0) {
         for (uint32_t s = 0; s < kStages; ++s) {
-            mbar_init(&full[s], kSource == kSourceTma ? 1 : 1 + kLoaderWarps);
+            mbar_init(&full[s], kSource == kSourceTma ? 1 : (shape.resident ? 0 : 1) + kLoaderWarps);
             mbar_init(&empty[s], 1);
         }
         for (uint32_t a = 0; a < 2; ++a) {
@@ -419,6 +428,7 @@ __global__ void __launch_bounds__(kSource == kSourceTma ? kThreads : kGatherThre
             mbar_init(&acc_empty[a], kReduce ? kEpilogueWarps / 2 : kEpilogueWarps);
         }
         mbar_init(drain, 1);
+        mbar_init(b_full, 1);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -442,7 +452,20 @@ __global__ void __launch_bounds__(kSource == kSourceTma ? kThreads : kGatherThre
             // ---------------- TMA producer
             uint32_t step = 0, issued = 0;
             bool ok = true, withheld = false;
-            for (uint32_t tile = blockIdx.x; tile < tiles && ok && !withheld; tile += gridDim.x) {
+            const bool resident = kSource != kSourceTma && shape.resident;
+            if (resident) {  // this CTA's column tile, once
+                uint32_t m_tile, n_tile;
+                tile_coords(blockIdx.x, shape, m_tile, n_tile);
+                mbar_expect_tx(b_full, shape.k_tiles * shape.block_n * kBlockK);
+                for (uint32_t ks = 0; ks < shape.k_tiles; ++ks)
+                    tma_load_2d(b_smem + ks * shape.block_n * kBlockK, &b_map, b_full, int(ks * kBlockK),
+                                int(n_tile * shape.block_n));
+                if (!mbar_wait(b_full, 0, shape.limit)) {  // it has to land before the CTA can exit
+                    *abort_flag = 1;
+                    record_error(shape.status, 1u);
+                }
+            }
+            for (uint32_t tile = blockIdx.x; !resident && tile < tiles && ok && !withheld; tile += gridDim.x) {
                 uint32_t m_tile, n_tile;
                 tile_coords(tile, shape, m_tile, n_tile);
                 const uint32_t row0 = m_tile * kBlockM, col0 = n_tile * shape.block_n;
@@ -481,7 +504,8 @@ __global__ void __launch_bounds__(kSource == kSourceTma ? kThreads : kGatherThre
             // ---------------- MMA issuer
             uint32_t step = 0, local = 0;
             const uint32_t instr = instr_desc(shape.block_n);
-            bool ok = true;
+            const bool resident = kSource != kSourceTma && shape.resident;
+            bool ok = !resident || mbar_wait(b_full, 0, shape.limit, abort_flag);
             for (uint32_t tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x, ++local) {
                 const uint32_t acc = local & 1, use = local >> 1;
                 if (*abort_flag || !mbar_wait(&acc_empty[acc], (use & 1) ^ 1, shape.limit, abort_flag)) {
@@ -492,13 +516,13 @@ __global__ void __launch_bounds__(kSource == kSourceTma ? kThreads : kGatherThre
                 const uint32_t d_tmem = tmem + acc * kAccColumns;
                 for (uint32_t ks = 0; ks < shape.k_tiles; ++ks, ++step) {
                     const uint32_t s = step % kStages, round = step / kStages;
-                    if (*abort_flag || !mbar_wait(&full[s], round & 1, shape.limit, abort_flag)) {
+                    if (!mbar_wait(&full[s], round & 1, shape.limit, abort_flag)) {
                         ok = false;
                         break;
                     }
                     fence_after();
                     const uint32_t a_addr = smem_u32(a_smem + s * kATileBytes);
-                    const uint32_t b_addr = smem_u32(b_smem + s * kBTileBytes);
+                    const uint32_t b_addr = smem_u32(b_smem) + (resident ? ks * shape.block_n * kBlockK : s * kBTileBytes);
 #pragma unroll
                     for (uint32_t kk = 0; kk < kBlockK / 32; ++kk)
                         mma_i8(d_tmem, smem_descriptor(a_addr + kk * 32), smem_descriptor(b_addr + kk * 32), instr,
@@ -901,7 +925,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                 const uint32_t d_tmem = tmem + acc * kAccColumns;
                 for (uint32_t ks = 0; ks < shape.k_tiles; ++ks, ++step) {
                     const uint32_t s = step % kPairStages, round = step / kPairStages;
-                    if (*abort_flag || !mbar_wait(&full[s], round & 1, limit, abort_flag)) {
+                    if (!mbar_wait(&full[s], round & 1, limit, abort_flag)) {
                         ok = false;
                         break;
                     }
@@ -1131,7 +1155,7 @@ void launch_gemm_tensor(const TensorGemmPlan& plan, const Epilogue& epilogue, cu
     TileShape shape{m,      plan.columns,       plan.k_tiles,
                     m_tiles, plan.n_tiles,      uint32_t(group),
                     rows,    plan.tile_counter, epilogue.status,
-                    options.limit_cycles > 0 ? options.limit_cycles : kDefaultLimitCycles, options.withheld, kBlockN};
+                    options.limit_cycles > 0 ? options.limit_cycles : kDefaultLimitCycles, options.withheld, kBlockN, false};
     const uint32_t tiles = m_tiles * plan.n_tiles;
     if (pairs) {
         const uint32_t max_pairs = plan.sm_count / 2;
@@ -1199,9 +1223,13 @@ void launch_gemm_gather(const TensorGemmPlan& plan, const GatherSource& source, 
     const uint32_t n_tiles = (plan.columns + block_n - 1) / block_n, tiles = m_tiles * n_tiles;
     uint64_t group = (48ull << 20) / plan.a_tile_bytes;
     group = group < 4 ? 4 : (group > 64 ? 64 : group);
+    // B stays in shared memory where a column tile's K steps fit the ring's B stages
+    const bool resident = plan.k_tiles * block_n * kBlockK <= kStages * kBTileBytes && n_tiles <= plan.sm_count;
     const TileShape shape{m,    plan.columns, plan.k_tiles,    m_tiles,             n_tiles,         uint32_t(group),
-                          rows, nullptr,      epilogue.status, kDefaultLimitCycles, kNoWithheldStep, block_n};
-    const uint32_t grid = tiles < plan.sm_count ? tiles : plan.sm_count;
+                          rows, nullptr,      epilogue.status, kDefaultLimitCycles, kNoWithheldStep, block_n,
+                          resident};
+    const uint32_t slots = resident ? plan.sm_count / n_tiles * n_tiles : plan.sm_count;
+    const uint32_t grid = tiles < slots ? tiles : slots;
     const CUtensorMap& b_map = block_n == 128 ? plan.b_map_half : plan.b_map;
     if (source.kind == kSourceRows)
         launch_chained(gemm_tc_kernel<kSourceRows, false>, grid, kGatherThreads, kSmemBytes, stream, b_map, b_map, shape,
