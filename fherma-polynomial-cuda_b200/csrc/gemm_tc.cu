@@ -106,6 +106,7 @@ __device__ __forceinline__ bool mbar_try(uint64_t* bar, uint32_t parity) {
 // (when `abort` is given) as soon as another role has raised the abort flag.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, long long limit,
                                           const volatile uint32_t* abort = nullptr) {
+    if (mbar_try(bar, parity)) return true;  // the usual case costs no clock read
     const long long start = clock64();
     for (uint32_t i = 0;; ++i) {
         if (mbar_try(bar, parity)) return true;
@@ -502,7 +503,7 @@ __global__ void __launch_bounds__(kSource == kSourceTma ? kThreads : kGatherThre
     } else if (warp == 1) {
         if (lane == 0) {
             // ---------------- MMA issuer
-            uint32_t step = 0, local = 0;
+            uint32_t s = 0, parity = 0, local = 0;  // ring stage, and its pass's parity
             const uint32_t instr = instr_desc(shape.block_n);
             const bool resident = kSource != kSourceTma && shape.resident;
             bool ok = !resident || mbar_wait(b_full, 0, shape.limit, abort_flag);
@@ -514,9 +515,8 @@ __global__ void __launch_bounds__(kSource == kSourceTma ? kThreads : kGatherThre
                 }
                 fence_after();
                 const uint32_t d_tmem = tmem + acc * kAccColumns;
-                for (uint32_t ks = 0; ks < shape.k_tiles; ++ks, ++step) {
-                    const uint32_t s = step % kStages, round = step / kStages;
-                    if (!mbar_wait(&full[s], round & 1, shape.limit, abort_flag)) {
+                for (uint32_t ks = 0; ks < shape.k_tiles; ++ks) {
+                    if (!mbar_wait(&full[s], parity, shape.limit, abort_flag)) {
                         ok = false;
                         break;
                     }
@@ -528,6 +528,10 @@ __global__ void __launch_bounds__(kSource == kSourceTma ? kThreads : kGatherThre
                         mma_i8(d_tmem, smem_descriptor(a_addr + kk * 32), smem_descriptor(b_addr + kk * 32), instr,
                                (ks | kk) != 0 ? 1u : 0u);
                     mma_commit(&empty[s]);  // frees the stage once these MMAs have read it
+                    if (++s == kStages) {
+                        s = 0;
+                        parity ^= 1;
+                    }
                 }
                 if (ok) mma_commit(&acc_full[acc]);  // accumulator complete
             }
@@ -910,7 +914,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     } else if (warp == 1) {
         if (lane == 0 && leader) {
             // ---------------- MMA issuer (leader only)
-            uint32_t step = 0, local = 0;
+            uint32_t s = 0, parity = 0, local = 0;
             bool ok = true;
             for (uint32_t i = 0; ok; ++i, ++local) {
                 const uint32_t tile = read_ring(i, true);
@@ -923,9 +927,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                 }
                 fence_after();
                 const uint32_t d_tmem = tmem + acc * kAccColumns;
-                for (uint32_t ks = 0; ks < shape.k_tiles; ++ks, ++step) {
-                    const uint32_t s = step % kPairStages, round = step / kPairStages;
-                    if (!mbar_wait(&full[s], round & 1, limit, abort_flag)) {
+                for (uint32_t ks = 0; ks < shape.k_tiles; ++ks) {
+                    if (!mbar_wait(&full[s], parity, limit, abort_flag)) {
                         ok = false;
                         break;
                     }
@@ -937,6 +940,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                         mma_i8_pair(d_tmem, smem_descriptor(a_addr + kk * 32), smem_descriptor(b_addr + kk * 32),
                                     (ks | kk) != 0 ? 1u : 0u);
                     mma_commit_pair(&empty[s]);  // frees stage s in both CTAs
+                    if (++s == kPairStages) {
+                        s = 0;
+                        parity ^= 1;
+                    }
                 }
                 if (ok) mma_commit_pair(&acc_full[acc]);
             }
