@@ -156,7 +156,9 @@ double estimate_ms(const negacyclic_plan& plan) {
 
 // Automatic lanes: instances under kSmallMs of device time share the GPU on kSmallLanes streams.
 constexpr double kSmallMs = 1.0;
-constexpr uint32_t kSmallLanes = 4;
+// Device time of a batch, us, 4 / 6 / 8 lanes: 938 / 912 / 958 (24 products, N 2048..16384, L 18..147), 158 / 125 /
+// 121 (20, N 256..2048, L 11..94), 65 / 52 / 44 (20, N 64..512, L 2..7), 364 / 355 / 364 (6, N 2048..16384).
+constexpr uint32_t kSmallLanes = 6;
 
 struct negacyclic_batch {
     int device = 0;

@@ -264,7 +264,7 @@ int negacyclic_gemm_u8(const uint8_t* d_a, const uint8_t* d_b, int32_t* d_d, uin
  * src/main.cpp:164-204). Instances are planned individually (an autotuner picks
  * each shape's ring split and GEMM kernel by timing them, cached in a text file)
  * and captured into a single CUDA graph. By default the graph has two phases:
- * instances under about 1 ms of device time share the GPU on up to four compute
+ * instances under about 1 ms of device time share the GPU on up to six compute
  * lanes (single-CTA tensor GEMMs), then the larger ones run one after another on
  * lane 0 with CTA-pair GEMMs. lanes > 0 instead spreads every instance over that
  * many lanes. Each lane shares one work arena among its instances.
