@@ -22,6 +22,7 @@
 // copies it issued land, frees TMEM and returns.
 #include <cuda.h>
 
+#include <algorithm>
 #include <cstdio>
 #include <cstdlib>
 
@@ -112,6 +113,10 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, long l
         if (mbar_try(bar, parity)) return true;
         if ((i & 63u) == 63u && ((abort && *abort) || clock64() - start > limit)) return false;
     }
+}
+
+__device__ __forceinline__ void mbar_arrive_local(uint64_t* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
 __device__ __forceinline__ uint64_t global_ns() {
@@ -215,6 +220,7 @@ struct TileShape {
     long long limit;         // cycles any one pipeline wait may take
     uint32_t withheld;       // diagnostics: CTA (pair) 0's producer stops before this pipeline step
     uint32_t block_n;        // columns per tile: 256, or 128 (single-CTA kernel)
+    bool paired;             // reduction of two column tiles: a CTA takes both of a row tile, one after the other
     bool resident;           // gathered A: each CTA keeps its column tile of B (n fastest, grid % n_tiles = 0)
 };
 
@@ -222,7 +228,7 @@ struct TileShape {
 // CTAs running at the same time share B tiles (and their A tiles stay in L2).
 __device__ __forceinline__ void tile_coords(uint32_t tile, const TileShape& shape, uint32_t& m_tile,
                                             uint32_t& n_tile) {
-    if (shape.resident) {
+    if (shape.resident || shape.paired) {
         m_tile = tile / shape.n_tiles;
         n_tile = tile - m_tile * shape.n_tiles;
         return;
@@ -233,6 +239,12 @@ __device__ __forceinline__ void tile_coords(uint32_t tile, const TileShape& shap
     const uint32_t rows_in_group = min(shape.group_m, shape.m_tiles - first_m);
     m_tile = first_m + within % rows_in_group;
     n_tile = within / rows_in_group;
+}
+
+// The i-th tile of a CTA of the single-CTA kernel (at or past the tile count: none).
+__device__ __forceinline__ uint32_t tile_at(uint32_t i, const TileShape& shape) {
+    if (shape.paired) return 2 * (blockIdx.x + (i >> 1) * gridDim.x) + (i & 1);
+    return blockIdx.x + i * gridDim.x;
 }
 
 // Applies the epilogue to 32 accumulator columns (c_base .. c_base+31) of one row.
@@ -324,7 +336,7 @@ __device__ __forceinline__ void epilogue_rows(const Epilogue& epi, uint32_t t_ba
 // kStagingPitch bytes), so that global stores are 64-byte runs. The accumulator is released once
 // its last column is read.
 __device__ __forceinline__ void reduce_rows(const ReduceParams& prm, uint32_t t_base, uint32_t* staging, uint32_t first,
-                                            uint32_t step, uint64_t* release, uint32_t lane) {
+                                            uint32_t step, uint64_t* release, bool paired, uint32_t lane) {
     const uint32_t limbs = prm.limbs, tlen = limbs + 2;
     uint32_t vx[3][4], vw[kWindow][4] = {};
 #pragma unroll
@@ -359,10 +371,13 @@ __device__ __forceinline__ void reduce_rows(const ReduceParams& prm, uint32_t t_
 #pragma unroll
             for (uint32_t i = 0; i < 8; ++i) d[8 * h + i] = word_sum<false>(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
         }
-        if (base + 16 >= tlen) {  // the accumulator's last columns are in registers
+        const bool last = base + 16 >= tlen;
+        if (last || (paired && base == 48)) {  // an accumulator's last columns are in registers
             fence_before();
             __syncwarp();
-            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(release)) : "memory");
+            // (L + 2 = 62..64: the second accumulator holds only words of D, read above)
+            if (lane == 0 && paired && base == 48) mbar_arrive_local(&release[0]);
+            if (lane == 0 && last) mbar_arrive_local(&release[paired ? 1 : 0]);
         }
         uint32_t o[16];
         st.words16(f, d, q, r, base, prm, o);
@@ -396,7 +411,8 @@ __device__ __forceinline__ void reduce_rows(const ReduceParams& prm, uint32_t t_
 //                        sectors and writes all 32 banks. This replaces the pad and transpose
 //                        kernels, each a pass over the data and a link in the chain of launches;
 //                        it pays while the K steps are few, since every column tile gathers again.
-// kReduce: all of a row's columns are in one tile, and a warp of the epilogue takes whole rows, one
+// kReduce: all of a row's columns are in one tile, or in the two accumulators (paired: a CTA computes both
+// column tiles of a row tile, one after the other), and a warp of the epilogue takes whole rows, one
 // per lane, through the reduction mod q straight from TMEM (csrc/reduce.cuh); the two sets of four
 // warps take alternate tiles, so that two tiles' carry chains run side by side.
 template <int kSource, bool kReduce>
@@ -466,7 +482,7 @@ __global__ void __launch_bounds__(kSource == kSourceTma ? kThreads : kGatherThre
                     record_error(shape.status, 1u);
                 }
             }
-            for (uint32_t tile = blockIdx.x; !resident && tile < tiles && ok && !withheld; tile += gridDim.x) {
+            for (uint32_t i = 0, tile; !resident && ok && !withheld && (tile = tile_at(i, shape)) < tiles; ++i) {
                 uint32_t m_tile, n_tile;
                 tile_coords(tile, shape, m_tile, n_tile);
                 const uint32_t row0 = m_tile * kBlockM, col0 = n_tile * shape.block_n;
@@ -507,7 +523,7 @@ __global__ void __launch_bounds__(kSource == kSourceTma ? kThreads : kGatherThre
             const uint32_t instr = instr_desc(shape.block_n);
             const bool resident = kSource != kSourceTma && shape.resident;
             bool ok = !resident || mbar_wait(b_full, 0, shape.limit, abort_flag);
-            for (uint32_t tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x, ++local) {
+            for (; ok && tile_at(local, shape) < tiles; ++local) {
                 const uint32_t acc = local & 1, use = local >> 1;
                 if (*abort_flag || !mbar_wait(&acc_empty[acc], (use & 1) ^ 1, shape.limit, abort_flag)) {
                     ok = false;
@@ -533,7 +549,12 @@ __global__ void __launch_bounds__(kSource == kSourceTma ? kThreads : kGatherThre
                         parity ^= 1;
                     }
                 }
-                if (ok) mma_commit(&acc_full[acc]);  // accumulator complete
+                // accumulator complete; paired: row tile `use` is, and its set of warps has the barrier to
+                // itself (a set that skipped phases of a shared one could take an old phase for its own)
+                if (ok && !(kReduce && shape.paired))
+                    mma_commit(&acc_full[acc]);
+                else if (ok && acc == 1)
+                    mma_commit(&acc_full[use & 1]);
             }
             if (!ok) {
                 *abort_flag = 1;
@@ -557,7 +578,7 @@ __global__ void __launch_bounds__(kSource == kSourceTma ? kThreads : kGatherThre
                              : "memory");
             ++published;
         };
-        for (uint32_t tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
+        for (uint32_t i = 0, tile; ok && (tile = tile_at(i, shape)) < tiles; ++i) {
             uint32_t m_tile, n_tile, op, t, j;
             tile_coords(tile, shape, m_tile, n_tile);
             shape.rows.decompose(m_tile * kBlockM, op, t, j);  // 128 consecutive j of one (op, t)
@@ -617,14 +638,16 @@ __global__ void __launch_bounds__(kSource == kSourceTma ? kThreads : kGatherThre
         // ---------------- epilogue: warp w reads TMEM lanes 32*(w%4).. (rows of the tile),
         // columns 128*((w-2)/4)..
         const uint32_t quarter = warp & 3, half = (warp - 2) >> 2;
-        uint32_t local = 0;
-        for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++local) {
+        for (uint32_t local = 0, tile; (tile = tile_at(local, shape)) < tiles; ++local) {
             const uint32_t acc = local & 1, use = local >> 1;
-            if (kReduce && acc != half) continue;
+            // reductions: the two sets of four warps take alternate row tiles, whole
+            if (kReduce && (shape.paired ? acc != 0 || (use & 1) != half : acc != half)) continue;
             uint32_t m_tile, n_tile;
             tile_coords(tile, shape, m_tile, n_tile);
             const uint32_t row0 = m_tile * kBlockM, col0 = n_tile * shape.block_n;
-            bool have = !*abort_flag && mbar_wait(&acc_full[acc], use & 1, shape.limit, abort_flag);
+            const bool row_tile = kReduce && shape.paired;
+            bool have = !*abort_flag && mbar_wait(&acc_full[row_tile ? half : acc], (row_tile ? use >> 1 : use) & 1,
+                                                  shape.limit, abort_flag);
             have = __all_sync(0xffffffffu, have);
             if (!have) {
                 if (lane == 0) {
@@ -639,7 +662,7 @@ __global__ void __launch_bounds__(kSource == kSourceTma ? kThreads : kGatherThre
                 uint32_t* staging = reinterpret_cast<uint32_t*>(
                     reinterpret_cast<uint8_t*>(full) + 256 + (warp - 2) * kStagingBytes);
                 reduce_rows(epi.reduce, tmem + acc * kAccColumns + ((quarter * 32) << 16), staging,
-                            shape.rows.coefficient(row - lane), shape.rows.split, &acc_empty[acc], lane);
+                            shape.rows.coefficient(row - lane), shape.rows.split, &acc_empty[acc], shape.paired, lane);
                 continue;
             }
             const bool row_ok = row < shape.m;
@@ -741,10 +764,6 @@ __device__ __forceinline__ void mma_commit_pair_local(uint64_t* bar) {
 
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar_cluster) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster) : "memory");
-}
-
-__device__ __forceinline__ void mbar_arrive_local(uint64_t* bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
 // Bounded wait with cluster-scope acquire: data written by the other CTA of the pair before its
@@ -1162,7 +1181,7 @@ void launch_gemm_tensor(const TensorGemmPlan& plan, const Epilogue& epilogue, cu
     TileShape shape{m,      plan.columns,       plan.k_tiles,
                     m_tiles, plan.n_tiles,      uint32_t(group),
                     rows,    plan.tile_counter, epilogue.status,
-                    options.limit_cycles > 0 ? options.limit_cycles : kDefaultLimitCycles, options.withheld, kBlockN, false};
+                    options.limit_cycles > 0 ? options.limit_cycles : kDefaultLimitCycles, options.withheld, kBlockN, false, false};
     const uint32_t tiles = m_tiles * plan.n_tiles;
     if (pairs) {
         const uint32_t max_pairs = plan.sm_count / 2;
@@ -1231,12 +1250,13 @@ void launch_gemm_gather(const TensorGemmPlan& plan, const GatherSource& source, 
     uint64_t group = (48ull << 20) / plan.a_tile_bytes;
     group = group < 4 ? 4 : (group > 64 ? 64 : group);
     // B stays in shared memory where a column tile's K steps fit the ring's B stages
-    const bool resident = plan.k_tiles * block_n * kBlockK <= kStages * kBTileBytes && n_tiles <= plan.sm_count;
+    const bool paired = reduce && n_tiles == 2;
+    const bool resident = !paired && plan.k_tiles * block_n * kBlockK <= kStages * kBTileBytes && n_tiles <= plan.sm_count;
     const TileShape shape{m,    plan.columns, plan.k_tiles,    m_tiles,             n_tiles,         uint32_t(group),
                           rows, nullptr,      epilogue.status, kDefaultLimitCycles, kNoWithheldStep, block_n,
-                          resident};
+                          paired, resident};
     const uint32_t slots = resident ? plan.sm_count / n_tiles * n_tiles : plan.sm_count;
-    const uint32_t grid = tiles < slots ? tiles : slots;
+    const uint32_t grid = std::min(paired ? m_tiles : tiles, slots);
     const CUtensorMap& b_map = block_n == 128 ? plan.b_map_half : plan.b_map;
     if (source.kind == kSourceRows)
         launch_chained(gemm_tc_kernel<kSourceRows, false>, grid, kGatherThreads, kSmemBytes, stream, b_map, b_map, shape,

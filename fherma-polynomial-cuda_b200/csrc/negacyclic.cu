@@ -272,7 +272,10 @@ void prepare_gather(negacyclic_plan& s) {
         prepare_gemm_gather(s.convert_rows, both, 2 * h.n, s.convert_weights, 4 * s.r, s.k_convert, why);
     if (s.k_crt <= kGatherResidueSteps * 128)
         prepare_gemm_gather(s.crt_gather, both, h.n, s.crt_weights, 4 * h.words, s.k_crt, why);
-    s.crt_reduces = s.crt_gather.ready && 4 * h.words <= 256;
+    // Two column tiles of a row tile in turn pay once the row tiles nearly fill the GPU. Product, us, two
+    // tiles reduced / word sums and the reduce kernel: 63.1 / 70.7 (N=16384, L=64), 160.8 / 179.5 (N=32768,
+    // L=94), 384 / 406 (N=65536, L=122); 66.9 / 64.8 (N=8192, L=122), 43.1 / 39.3 (N=4096, L=94).
+    s.crt_reduces = s.crt_gather.ready && 4 * h.words <= (h.n >= 16384 ? 512u : 256u);
 }
 
 constexpr char kFewColumns[] = "fewer than 256 output columns";

@@ -153,3 +153,15 @@ def test_small_product_stages_match_the_general_path(fpc, inputs):
             r = plan.info()["primes"]
             dumps.append((c.tobytes(), plan.debug_read(0)[:r * n * 4], plan.debug_read(1), plan.debug_read(2)))
     assert dumps[0] == dumps[1]
+
+
+# the reduction over two column tiles, at one to four row tiles per CTA: L = 60..62 (the second tile
+# holds words of the quotient only), the ends of the second tile, and word sums again past it
+@pytest.mark.parametrize("n,limbs", [(8192, 60), (16384, 60), (16384, 61), (16384, 62), (16384, 63), (16384, 75),
+                                     (16384, 123), (16384, 124), (32768, 62), (32768, 91), (65536, 60), (65536, 63), (65536, 123)])
+def test_reduction_over_two_column_tiles(n, limbs, fpc, inputs, torch):
+    q, a, b = inputs.instance(n, limbs, 300 + limbs, 0)
+    top = inputs.edge_operand(n, q, "max")
+    for x, y in ((a, b), (top, a), (top, top)):
+        assert np.array_equal(device_product(fpc, torch, q, x, y),
+                              device_product(fpc, torch, q, x, y, gemm=fpc.GEMM_SIMT))
