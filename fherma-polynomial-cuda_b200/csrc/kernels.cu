@@ -650,7 +650,8 @@ __device__ __forceinline__ void middle_passes(bool active, uint32_t tid, uint32_
 // product is bound by its launches (three cost the host 9 to 13 us, more than the device needs), so all
 // of it is one. The conversion and the CRT are plain sums here: residue = sum_j REDC(limb_j c_j) with
 // c_j = 2^(32j) mod p, and the words of sum_k v_k W_k by a 96-bit accumulator per coefficient.
-// N = 256, L = 2: 12.0 -> 9.7 us; N = 64, L = 2: 19.7 -> 7.5 us.
+// N = 256, L = 2: 12.0 -> 8.9 us; N = 64, L = 2: 19.7 -> 7.4 us. At least 512 threads, for the conversion
+// (256: 9.6 us).
 constexpr uint32_t kSmallPrimes = 64;
 template <uint32_t kLog>
 __global__ void __launch_bounds__(512) small_product_kernel(SmallProduct prm) {
@@ -1138,7 +1139,7 @@ static void launch_product(uint32_t* residues, const DevicePrime* primes, const 
     launch_chained(ntt_product_kernel<kLog>, r, 2 * kN / per_thread(kLog), kSmem, stream, residues, primes, fwd, inv, r);
 }
 
-static uint32_t small_threads(uint32_t n, uint32_t r) { return std::max(256u, (n / 8 * r + 31) / 32 * 32); }
+static uint32_t small_threads(uint32_t n, uint32_t r) { return std::max(512u, (n / 8 * r + 31) / 32 * 32); }
 
 static size_t small_smem(uint32_t n, uint32_t r, uint32_t limbs) {
     return (size_t(n) * (2 * r + std::max(2 * limbs, limbs + 5)) + size_t(r) * (2 * limbs + 5) + 2 * (limbs + 2)) *
@@ -1146,7 +1147,7 @@ static size_t small_smem(uint32_t n, uint32_t r, uint32_t limbs) {
 }
 
 // The line lies where the three kernels catch up. Product, us, one kernel / three, at N r L of:
-// 2560 (N=256, L=2) 9.7 / 12.0, 4608 (N=128, L=4) 9.0 / 12.3, 9216 (N=256, L=4) 14.1 / 12.0, 16384 (N=128,
+// 2560 (N=256, L=2) 8.9 / 12.0, 4608 (N=128, L=4) 8.5 / 12.3, 9216 (N=256, L=4) 14.1 / 12.0, 16384 (N=128,
 // L=8) 15.5 / 12.3, 5120 (N=512, L=2) 16.0 / 12.0. At N=64 the tensor GEMMs do not apply: 6272 (L=7) 11.3 /
 // 19.8, 16896 (L=11) 18.1 / 20.
 bool small_product_takes(uint32_t n, uint32_t r, uint32_t limbs) {
