@@ -9,6 +9,9 @@
 //   transpose  -> coefficient-major CRT inputs            [transpose_residues, src/solve.cu:244-253]
 //   crt        byte-sliced u8 GEMM -> u64 word sums       [tensor_product<false>, src/solve.cu:603]
 //   reduce     carry, CRT quotient, mod q                 [reconstruct*, src/solve.cu:323-500]
+// Where it is faster, one kernel does several: the conversion reads unpadded operands and the CRT GEMM
+// the residues, and reduces (prepare_gather); unsplit rings run forward, pointwise and inverse in one
+// kernel (negacyclic_plan::ntt_fused); the smallest products are one kernel (negacyclic_plan::small).
 #include <cuda_runtime.h>
 
 #include <algorithm>

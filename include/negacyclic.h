@@ -150,7 +150,9 @@ int negacyclic_run_device(negacyclic_plan* plan, const uint32_t* d_a, const uint
 /*
  * negacyclic_run_device, synchronously, with CUDA events recorded on `stream`
  * between stages. stage_ms[8] receives the milliseconds of: pad, convert,
- * forward NTT, pointwise, inverse NTT, transpose, CRT GEMM, reduce.
+ * forward NTT, pointwise, inverse NTT, transpose, CRT GEMM, reduce. Where one kernel
+ * does several of these (small and narrow points), its time is that of the first of
+ * them it does and the others are about zero.
  */
 int negacyclic_run_device_timed(negacyclic_plan* plan, const uint32_t* d_a, const uint32_t* d_b,
                                 uint32_t* d_c, void* stream, float* stage_ms);
@@ -246,7 +248,8 @@ int negacyclic_host_plan(uint32_t n, uint32_t limbs, const uint32_t* q, uint32_t
  * Copies one internal stage buffer of the last product to host memory, for
  * stage-by-stage checks at small sizes. which: 0 residues [2][r][N] u32 (after
  * the last stage that wrote them), 1 CRT inputs [N][padded_primes] u32,
- * 2 CRT word sums [N][words] u64. Returns the byte size in *bytes when host is NULL.
+ * 2 CRT word sums [N][words] u64 (made from the residues where the product's kernels
+ * kept neither). Returns the byte size in *bytes when host is NULL.
  */
 int negacyclic_debug_read(negacyclic_plan* plan, int which, void* host, size_t* bytes);
 
