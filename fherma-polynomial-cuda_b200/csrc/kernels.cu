@@ -353,10 +353,21 @@ __device__ __forceinline__ void ct_stages(uint32_t (&x)[1 << R], uint32_t group_
 // Gentleman-Sande stages with half-sizes t_min .. t_min*2^(R-1) (inverse). Stage r's butterflies
 // (k, k + 2^r) in block b = k >> (r + 1) share twiddle h + group_hi * 2^(R-1-r) + b.
 // Values between stages are in [0, 2p), as in ct_stages.
-template <int R, bool kPaired, int r = 0>
+// kScale: the pass ends the transform, and its last stage scales (Finish) to canonical values.
+template <int R, bool kPaired, bool kScale = false, int r = 0>
 __device__ __forceinline__ void gs_stages(uint32_t (&x)[1 << R], uint32_t group_hi, uint32_t log_t_min,
-                                          uint32_t log_n, const uint2* __restrict__ table, uint32_t p) {
+                                          uint32_t log_n, const uint2* __restrict__ table, uint32_t p,
+                                          const Finish& finish = Finish{}) {
     constexpr int half = 1 << r;
+    if constexpr (kScale && r == R - 1) {
+#pragma unroll
+        for (int k = 0; k < half; ++k) {
+            const uint32_t u = reduce_once(x[k], p), v = reduce_once(x[k + half], p);
+            x[k] = shoup(u + v, finish.f, finish.f_q, p);
+            x[k + half] = shoup(u - v + p, finish.w, finish.w_q, p);
+        }
+        return;
+    }
     const uint32_t log_t = log_t_min + r;
     const uint32_t h = 1u << (log_n - 1 - log_t);
     constexpr int blocks = 1 << (R - 1 - r);
@@ -372,14 +383,15 @@ __device__ __forceinline__ void gs_stages(uint32_t (&x)[1 << R], uint32_t group_
             x[k + half] = shoup_lazy(u - v + p, w.x, w.y, p);
         }
     }
-    if constexpr (r + 1 < R) gs_stages<R, kPaired, r + 1>(x, group_hi, log_t_min, log_n, table, p);
+    if constexpr (r + 1 < R) gs_stages<R, kPaired, kScale, r + 1>(x, group_hi, log_t_min, log_n, table, p, finish);
 }
 
 // One pass of R stages over all of this thread's groups (transform length 2^kLog). src/dst are shared (swizzled index) or global (plain index);
-// kScale multiplies the values stored to global by (f, f_q).
+// kScale: the last inverse pass, whose last stage scales.
 template <int R, bool kForward, bool kFromGlobal, bool kToGlobal, bool kScale, uint32_t kLogTMin, uint32_t kLog>
 __device__ __forceinline__ void ntt_pass(uint32_t tid, const uint32_t* src, uint32_t* dst,
-                                         const uint2* __restrict__ table, uint32_t p, uint32_t f, uint32_t f_q) {
+                                         const uint2* __restrict__ table, uint32_t p,
+                                         const Finish& finish = Finish{}) {
     constexpr int G = per_thread(kLog) >> R;  // groups per thread
     constexpr uint32_t kThreads = (1u << kLog) / per_thread(kLog);
 #pragma unroll
@@ -418,13 +430,10 @@ __device__ __forceinline__ void ntt_pass(uint32_t tid, const uint32_t* src, uint
         if (kForward)
             ct_stages<R, kPaired>(x, group >> kLogTMin, kLogTMin, kLog, table, p);
         else
-            gs_stages<R, kPaired>(x, group >> kLogTMin, kLogTMin, kLog, table, p);
+            gs_stages<R, kPaired, kScale>(x, group >> kLogTMin, kLogTMin, kLog, table, p, finish);
+        if constexpr (kToGlobal && !kScale) {
 #pragma unroll
-        for (int k = 0; k < (1 << R); ++k) {
-            if (kScale)
-                x[k] = shoup(x[k], f, f_q, p);  // canonical: shoup takes any 32-bit value
-            else if (kToGlobal)
-                x[k] = reduce_once(x[k], p);    // [0, 2p) -> canonical
+            for (int k = 0; k < (1 << R); ++k) x[k] = reduce_once(x[k], p);  // [0, 2p) -> canonical
         }
         if constexpr (kToGlobal && kPair) {
             *reinterpret_cast<uint2*>(dst + base) = make_uint2(x[0], x[1]);
@@ -477,15 +486,15 @@ constexpr int ntt_pass_stages(bool forward, uint32_t log, uint32_t done) {
 // `tid`: the thread's number among the transform's.
 template <bool kForward, uint32_t kLog, uint32_t kDone>
 __device__ __forceinline__ void ntt_passes(uint32_t tid, uint32_t* data, uint32_t* xs, const uint2* __restrict__ table,
-                                           uint32_t p, uint32_t f, uint32_t f_q) {
+                                           uint32_t p, const Finish& finish = Finish{}) {
     constexpr int R = ntt_pass_stages(kForward, kLog, kDone);
     constexpr uint32_t kLogTMin = kForward ? kLog - kDone - R : kDone;
     constexpr bool kFirst = kDone == 0, kLast = kDone + R == kLog;
     ntt_pass<R, kForward, kFirst, kLast, kLast && !kForward, kLogTMin, kLog>(tid, kFirst ? data : xs, kLast ? data : xs,
-                                                                              table, p, f, f_q);
+                                                                              table, p, finish);
     if constexpr (!kLast) {
         __syncthreads();
-        ntt_passes<kForward, kLog, kDone + R>(tid, data, xs, table, p, f, f_q);
+        ntt_passes<kForward, kLog, kDone + R>(tid, data, xs, table, p, finish);
     }
 }
 
@@ -501,7 +510,7 @@ __global__ void __launch_bounds__((1u << kLog) / per_thread(kLog), 4) ntt_forwar
     const uint32_t local_op = blockIdx.x / t_count, op = op_first + local_op;
     const uint32_t t_index = t_first + blockIdx.x - local_op * t_count, k = blockIdx.y;
     uint32_t* data = residues + (size_t(op) * r + k) * n + size_t(t_index) * kN;
-    ntt_passes<true, kLog, 0>(threadIdx.x, data, xs, fwd + size_t(k) * kN, primes[k].p, 0, 0);
+    ntt_passes<true, kLog, 0>(threadIdx.x, data, xs, fwd + size_t(k) * kN, primes[k].p);
 }
 
 template <uint32_t kLog>
@@ -514,7 +523,7 @@ __global__ void __launch_bounds__((1u << kLog) / per_thread(kLog), 4) ntt_invers
     const uint32_t v_index = v_first + blockIdx.x, k = blockIdx.y;
     const DevicePrime f = primes[k];
     uint32_t* data = residues + size_t(k) * n + size_t(v_index) * kN;
-    ntt_passes<false, kLog, 0>(threadIdx.x, data, xs, inv + size_t(k) * kN, f.p, f.finish, f.finish_q);
+    ntt_passes<false, kLog, 0>(threadIdx.x, data, xs, inv + size_t(k) * kN, f.p, finish_of(f));
 }
 
 // Unsplit rings (s = 1): both operands' forward transforms, their product and its inverse in one CTA
@@ -532,7 +541,7 @@ __device__ __forceinline__ void forward_to_middle(bool active, uint32_t tid, uin
     constexpr bool kGlobal = kGlobalInput && kDone == 0;
     if constexpr (kDone + R < kLog) {
         if (active)
-            ntt_pass<R, true, kGlobal, false, false, kLog - kDone - R, kLog>(tid, kGlobal ? data : xs, xs, table, p, 0, 0);
+            ntt_pass<R, true, kGlobal, false, false, kLog - kDone - R, kLog>(tid, kGlobal ? data : xs, xs, table, p);
         __syncthreads();
         forward_to_middle<kLog, kDone + R, kGlobalInput>(active, tid, data, xs, table, p);
     }
@@ -540,14 +549,14 @@ __device__ __forceinline__ void forward_to_middle(bool active, uint32_t tid, uin
 
 template <uint32_t kLog, uint32_t kDone>
 __device__ __forceinline__ void inverse_from_middle(bool active, uint32_t tid, uint32_t* data, uint32_t* xs,
-                                                    const uint2* __restrict__ table, uint32_t p, uint32_t f,
-                                                    uint32_t f_q) {
+                                                    const uint2* __restrict__ table, uint32_t p,
+                                                    const Finish& finish) {
     if constexpr (kDone < kLog) {
         constexpr int R = ntt_pass_stages(false, kLog, kDone);
         constexpr bool kLast = kDone + R == kLog;
         __syncthreads();
-        if (active) ntt_pass<R, false, false, kLast, kLast, kDone, kLog>(tid, xs, kLast ? data : xs, table, p, f, f_q);
-        inverse_from_middle<kLog, kDone + R>(active, tid, data, xs, table, p, f, f_q);
+        if (active) ntt_pass<R, false, false, kLast, kLast, kDone, kLog>(tid, xs, kLast ? data : xs, table, p, finish);
+        inverse_from_middle<kLog, kDone + R>(active, tid, data, xs, table, p, finish);
     }
 }
 
@@ -599,7 +608,7 @@ __global__ void __launch_bounds__(2 * (1u << kLog) / per_thread(kLog), (kLog >= 
             for (int i = 0; i < (1 << R); ++i) xs[placed ^ swizzle<kLog>(uint32_t(i))] = x[g][i];
         }
     }
-    inverse_from_middle<kLog, R>(op == 0, tid, data, xs, inverse, f.p, f.finish, f.finish_q);
+    inverse_from_middle<kLog, R>(op == 0, tid, data, xs, inverse, f.p, finish_of(f));
 }
 
 // ntt_product_kernel's middle, from the forward transforms' last pass through the products to the
@@ -707,8 +716,8 @@ __global__ void __launch_bounds__(512) small_product_kernel(SmallProduct prm) {
         forward_to_middle<kLog, 0, false>(active, tid, nullptr, op ? b : a, forward, f.p);
         middle_passes<kLog>(active, tid, op, a, r * kN, forward, inverse, f);
         // the last pass writes v_k in plain order over b's transform
-        inverse_from_middle<kLog, ntt_pass_stages(false, kLog, 0)>(active && op == 0, tid, b, a, inverse, f.p, f.finish,
-                                                                    f.finish_q);
+        inverse_from_middle<kLog, ntt_pass_stages(false, kLog, 0)>(active && op == 0, tid, b, a, inverse, f.p,
+                                                                    finish_of(f));
     }
     __syncthreads();
     for (uint32_t i = threadIdx.x; i < r * kN; i += blockDim.x) prm.residues[i] = v[i];

@@ -451,7 +451,13 @@ int negacyclic_init(uint32_t n, uint32_t w, uint32_t limbs, const uint32_t* q, c
         std::vector<DevicePrime> primes(s.r);
         for (uint32_t k = 0; k < s.r; ++k) {
             const PrimeInfo& p = h.primes[k];
-            primes[k] = DevicePrime{p.p, p.pinv, p.finish, p.finish_q, p.psi, p.r2};
+            // the inverse transform's last twiddle: psi^(2N' - N'/2) (no stages, and any value, at N' = 1)
+            uint64_t w = 1, base = p.psi;
+            for (uint32_t e = 2 * h.n_sub - h.n_sub / 2; e; e >>= 1, base = base * base % p.p)
+                if (e & 1) w = w * base % p.p;
+            const uint32_t finish_w = uint32_t(w * p.finish % p.p);
+            primes[k] = DevicePrime{p.p, p.pinv, p.finish, p.finish_q, p.psi, p.r2, finish_w,
+                                    uint32_t((uint64_t(finish_w) << 32) / p.p)};
         }
         cudaStream_t st = s.stream;
         check(cudaMemcpyAsync(s.primes, primes.data(), s.r * sizeof(DevicePrime), cudaMemcpyHostToDevice, st), "upload");
