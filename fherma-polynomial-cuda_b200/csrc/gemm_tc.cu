@@ -295,10 +295,9 @@ __device__ __forceinline__ void epilogue_rows(const Epilogue& epi, uint32_t t_ba
                                               uint32_t column) {
     if (epi.mode == kEpilogueConvert) {
         const uint32_t k0 = col0 / 4;
-        // byte offset of prime k0's value in the residues (2 r N words, below 4 GB), then + 4 N per prime
-        uint32_t at = ((op * epi.r + k0) * epi.n + column) * 4u;
+        uint32_t* out = epi.residues + residue_index(op, k0, column, epi.r, epi.n);  // + N per prime
 #pragma unroll 1
-        for (uint32_t chunk = 0; chunk < chunks; ++chunk) {
+        for (uint32_t chunk = 0; chunk < chunks; ++chunk, out += 8 * size_t(epi.n)) {
             if (k0 + chunk * 8 >= epi.r) break;  // warp-uniform
             uint2 prime[8];
 #pragma unroll
@@ -314,9 +313,7 @@ __device__ __forceinline__ void epilogue_rows(const Epilogue& epi, uint32_t t_ba
                 const uint64_t s = word_sum<kShort>(v[4 * g], v[4 * g + 1], v[4 * g + 2], v[4 * g + 3]);
                 const uint32_t m = uint32_t(s) * prime[g].y;
                 const uint32_t u = reduce_once(uint32_t(mad_wide(m, prime[g].x, s) >> 32), prime[g].x);
-                if (row_ok && (whole || k0 + chunk * 8 + g < epi.r))
-                    *reinterpret_cast<uint32_t*>(reinterpret_cast<uint8_t*>(epi.residues) + at) = u;
-                at += 4u * epi.n;
+                if (row_ok && (whole || k0 + chunk * 8 + g < epi.r)) out[g * size_t(epi.n)] = u;
             }
         }
         return;

@@ -190,7 +190,7 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(const uint8_t* __restric
             const DevicePrime f = epi.primes[group];
             uint32_t op, column;
             rows.residue(m, op, column);
-            epi.residues[(size_t(op) * epi.r + group) * epi.n + column] = redc(s, f.p, f.pinv);
+            epi.residues[residue_index(op, group, column, epi.r, epi.n)] = redc(s, f.p, f.pinv);
         } else {
             if (group < epi.words) epi.dots[rows.row(m) * epi.dots_stride + group] = s;
         }

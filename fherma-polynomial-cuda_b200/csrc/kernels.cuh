@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include "modarith.cuh"
+#include "residue_index.h"
 
 namespace negacyclic {
 
