@@ -184,3 +184,40 @@ def test_residues_past_four_gigabytes(fpc, inputs, oracle, torch):
             assert plan.status() == 0
         for i, row in want.items():
             assert np.array_equal(row, dc[i].cpu().numpy().view(np.uint32)), (gemm, i)
+
+
+# one-kernel products with few primes and many zero limbs above q: 44 to 51 KB of shared memory
+@pytest.mark.parametrize("limbs", range(85, 94))
+@pytest.mark.parametrize("qv", [2001, (1 << 24) - 3, (1 << 27) - 39])
+def test_small_products_around_the_shared_memory_default(limbs, qv, fpc, inputs, oracle, torch):
+    n, q = 64, inputs.from_int(qv, limbs)
+    rng = np.random.Generator(np.random.PCG64(limbs))
+    a, b = (np.pad(inputs.random_operand(rng, n, q[:1]), ((0, 0), (0, limbs - 1))) for _ in range(2))
+    want = oracle.kronecker(q, a, b)
+    assert np.array_equal(device_product(fpc, torch, q, a, b), want)
+    with fpc.Plan(n, 32 * limbs, limbs, q) as plan:
+        assert np.array_equal(plan.run(a, b), want)
+
+
+def test_small_products_of_several_sizes_on_threads(fpc, inputs, oracle):
+    """Launches of one-kernel products that need different amounts of shared memory."""
+    import threading
+    n, qv, failed = 64, 2001, []
+
+    def worker(limbs):
+        q = inputs.from_int(qv, limbs)
+        a = np.pad(inputs.random_operand(np.random.Generator(np.random.PCG64(1)), n, q[:1]), ((0, 0), (0, limbs - 1)))
+        want = oracle.kronecker(q, a, a)
+        try:
+            with fpc.Plan(n, 32 * limbs, limbs, q) as plan:
+                for _ in range(2000):
+                    assert np.array_equal(plan.run(a, a), want)
+        except Exception as e:
+            failed.append((limbs, repr(e)))
+
+    threads = [threading.Thread(target=worker, args=(limbs,)) for limbs in (100, 150, 192)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed
