@@ -12,6 +12,8 @@
 //
 // The team runs jobs in the order they are posted. Every worker takes part in every job (a
 // job is a function of the worker index), so a job splits its work into one slice per worker.
+// Several plans share a team (shared_host_team), so a long copy is posted in turns (Turns): a job
+// posted meanwhile by another thread waits for a few turns and not for the whole copy.
 // A job can publish finer-grained progress itself (per-chunk counters), which is how the
 // launcher thread learns that chunk k is packed while later chunks are still being copied.
 // Waits spin for a fixed time (kSpinTime) before they block, and the team keeps spinning between
@@ -156,21 +158,55 @@ public:
     // Whether job `ticket` has finished (no waiting).
     bool finished(uint64_t ticket) const { return finished_.load(std::memory_order_acquire) >= ticket; }
 
+    // One caller's way of posting long work: jobs ("turns") of about kTurnBytes, at most kAhead of them
+    // posted and unfinished at a time. A short call beside a wide one (see shared_host_team), ms, at 1 / 2 /
+    // 4 MB with three ahead: 0.88 / 0.98 / 1.3; with two ahead: 0.73 / 0.73 at 1 / 2 MB.
+    class Turns {
+    public:
+        static constexpr size_t kTurnBytes = 2 << 20;
+        static constexpr uint32_t kAhead = 2;  // the workers run one while the next is at hand
+
+        explicit Turns(HostTeam& team) : team_(team) {}
+        bool ready() const { return count_ < kAhead || team_.finished(tickets_[count_ % kAhead]); }
+        void post(Job job) {  // waits until there is room
+            if (!ready()) team_.wait(tickets_[count_ % kAhead]);
+            tickets_[count_++ % kAhead] = last_ = team_.post(std::move(job));
+        }
+        uint64_t last() const { return last_; }  // ticket of the last turn posted (0: none)
+
+    private:
+        HostTeam& team_;
+        uint64_t tickets_[kAhead] = {}, last_ = 0;
+        uint64_t count_ = 0;
+    };
+
+    // Posts part(begin, end) over slices that cover [0, bytes), in turns.
+    template <class Part>
+    static void post_range(Turns& turns, size_t bytes, const Part& part) {
+        for (size_t first = 0; first < bytes; first += Turns::kTurnBytes) {
+            const size_t size = std::min(bytes - first, Turns::kTurnBytes);
+            turns.post([=](unsigned w, unsigned n) {
+                const size_t b = slice_begin(size, w, n), e = slice_begin(size, w + 1, n);
+                if (e > b) part(first + b, first + e);
+            });
+        }
+    }
+
     // dst[0..bytes) = src[0..bytes), split over the workers; blocking.
     void copy(void* dst, const void* src, size_t bytes) {
-        wait(post([=](unsigned w, unsigned n) {
-            const size_t b = slice_begin(bytes, w, n), e = slice_begin(bytes, w + 1, n);
-            if (e > b) std::memcpy(static_cast<char*>(dst) + b, static_cast<const char*>(src) + b, e - b);
-        }));
+        Turns turns(*this);
+        post_range(turns, bytes, [=](size_t b, size_t e) {
+            std::memcpy(static_cast<char*>(dst) + b, static_cast<const char*>(src) + b, e - b);
+        });
+        wait(turns.last());
     }
 
     // Writes zeros over [ptr, ptr + bytes), split over the workers: the first touch of freshly
     // mapped pages (page faults and the kernel's own zeroing) runs on every worker at once.
     void touch(void* ptr, size_t bytes) {
-        wait(post([=](unsigned w, unsigned n) {
-            const size_t b = slice_begin(bytes, w, n), e = slice_begin(bytes, w + 1, n);
-            if (e > b) std::memset(static_cast<char*>(ptr) + b, 0, e - b);
-        }));
+        Turns turns(*this);
+        post_range(turns, bytes, [=](size_t b, size_t e) { std::memset(static_cast<char*>(ptr) + b, 0, e - b); });
+        wait(turns.last());
     }
 
     // Start of slice w of n over `total` units, in 64-unit steps (cache lines for bytes).
@@ -231,13 +267,54 @@ private:
     std::atomic<bool> stopping_{false};
 };
 
+// Pieces 0 .. total - 1 of a long job, run on the team in turns of `per_turn`. Workers claim pieces in
+// order, one at a time (a descheduled worker holds up at most the piece it has); the caller calls feed()
+// while it waits for them. Turns already posted may run on after this object is gone (last()).
+class PieceFeed {
+public:
+    PieceFeed(HostTeam& team, uint32_t total, uint32_t per_turn, std::function<void(uint32_t piece)> run)
+        : turns_(team), state_(std::make_shared<State>()), total_(total), per_turn_(std::max(1u, per_turn)) {
+        state_->run = std::move(run);
+    }
+
+    // Posts the turns there is room for.
+    void feed() {
+        while (fed_ < total_ && turns_.ready()) {
+            const uint32_t end = total_ - fed_ > per_turn_ ? fed_ + per_turn_ : total_;
+            turns_.post([state = state_, end](unsigned, unsigned) {
+                // a worker gets here once every piece before this turn is claimed
+                uint32_t piece = state->next.load(std::memory_order_relaxed);
+                while (piece < end)
+                    if (state->next.compare_exchange_weak(piece, piece + 1, std::memory_order_relaxed)) {
+                        state->run(piece);
+                        piece = state->next.load(std::memory_order_relaxed);
+                    }
+            });
+            fed_ = end;
+        }
+    }
+    uint64_t last() const { return turns_.last(); }
+
+private:
+    struct State {
+        std::atomic<uint32_t> next{0};
+        std::function<void(uint32_t)> run;
+    };
+    HostTeam::Turns turns_;
+    std::shared_ptr<State> state_;
+    uint32_t total_, per_turn_, fed_ = 0;
+};
+
 // The process's team of this size and spin time: made for the first plan that asks, shared by all
 // that hold it, and joined with the last of them. Jobs of several plans run in the order they are
-// posted; a job only copies host memory and never waits for another, so plans on different threads
-// do not block each other. One team instead of one per plan: host memory bandwidth is the limit
-// either way, and the spinning workers of an idle plan's team took the cores from the plan that was
-// running (three plans called in turn at N=32768, L=28 on a 16-vCPU host: 18 spinning threads, 5-15
-// ms per call against 0.37 with one team of six).
+// posted; a job only copies host memory and never waits for another, and a long copy is posted in
+// turns, so a plan's call waits for a few turns of another thread's call and not for its whole product.
+// One team instead of one per plan: host memory bandwidth is the limit either way, and the spinning
+// workers of an idle plan's team took the cores from the plan that was running (three plans called in
+// turn at N=32768, L=28 on a 16-vCPU host: 18 spinning threads, 5-15 ms per call against 0.37 with one
+// team of six). The price is paid beside a wide product of another thread: a call at N=32768, L=28 beside
+// one at N=65536, L=1747 (both pageable) took 0.73 ms in the middle against 0.42-0.50 with teams of their
+// own, and 3.8 against 3.5 ms at nine in ten; alone 0.36 against 0.41. Without turns it took 13 to 35 ms.
 inline std::shared_ptr<HostTeam> shared_host_team(unsigned workers, std::chrono::microseconds spin) {
     static std::mutex mu;
     static std::map<std::pair<unsigned, std::chrono::microseconds::rep>, std::weak_ptr<HostTeam>> teams;
@@ -249,17 +326,22 @@ inline std::shared_ptr<HostTeam> shared_host_team(unsigned workers, std::chrono:
     return team;
 }
 
-// Spins until `flag` reaches `value` (acquire): one thread's short waits (the launcher waiting
-// for the team to pack a chunk); yields its core after `spin`.
-inline void spin_until(const std::atomic<uint32_t>& flag, uint32_t value,
-                       std::chrono::microseconds spin = HostTeam::kSpinTime) {
+// Spins until `flag` reaches `value` (acquire), calling `poll` meanwhile: one thread's short waits (the
+// launcher waiting for the team to pack a chunk); yields its core after `spin`.
+template <class Poll>
+inline void spin_until(const std::atomic<uint32_t>& flag, uint32_t value, std::chrono::microseconds spin, Poll&& poll) {
     const auto until = std::chrono::steady_clock::now() + spin;
     for (uint32_t spins = 0; flag.load(std::memory_order_acquire) < value; ++spins) {
+        poll();
         if ((spins & 63u) != 63u || std::chrono::steady_clock::now() < until)
             NEGACYCLIC_PAUSE();
         else
             std::this_thread::yield();
     }
+}
+inline void spin_until(const std::atomic<uint32_t>& flag, uint32_t value,
+                       std::chrono::microseconds spin = HostTeam::kSpinTime) {
+    spin_until(flag, value, spin, [] {});
 }
 
 }  // namespace negacyclic

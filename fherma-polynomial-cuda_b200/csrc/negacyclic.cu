@@ -687,9 +687,9 @@ void host_begin(negacyclic_plan& s, const uint32_t* a, const uint32_t* b, uint32
     const uint32_t* small_rows = nullptr;  // where the operands of a small product land
     const bool fuse_ntt = s.ntt_fused() && in.size() == 1;  // in pieces, a's transforms run while b is on the link
     uint32_t pieces[negacyclic_plan::kMaxChunks] = {};  // pack pieces per input chunk
+    std::unique_ptr<PieceFeed> pack;
     if (!a_locked || !b_locked) {
-        // One pack job over pieces of about kPieceBytes of the pageable operands, claimed in chunk
-        // order from a shared counter (a descheduled worker holds up at most the piece it has).
+        // Pieces of about kPieceBytes of the pageable operands, packed by the team in chunk order.
         // Contiguous ranges (narrow rows) are copied with streaming stores: behind the reference's
         // harness, fherma_run took 0.465 against 0.517 ms at N=32768/L=28 and 1.330 against 1.396
         // ms at N=65536/L=55 (4 alternating runs of 20 cases). The row gather of wide rows keeps
@@ -706,44 +706,48 @@ void host_begin(negacyclic_plan& s, const uint32_t* a, const uint32_t* b, uint32
             first_piece[k + 1] = first_piece[k] + pieces[k];
             s.packed[k].store(0, std::memory_order_relaxed);
         }
-        s.next_piece.store(0, std::memory_order_relaxed);
         uint32_t* stage = s.stage_in;
         const uint32_t n = h.n, limbs = h.limbs, total = first_piece.back();
         std::atomic<uint32_t>* packed = s.packed;
-        std::atomic<uint32_t>* next = &s.next_piece;
-        s.pack_ticket = s.team->post([=](unsigned, unsigned) {
+        pack = std::make_unique<PieceFeed>(*s.team, total, uint32_t(HostTeam::Turns::kTurnBytes / kPieceBytes), [=](uint32_t piece) {
             uint32_t k = 0;
-            for (uint32_t piece = next->fetch_add(1, std::memory_order_relaxed); piece < total;
-                 piece = next->fetch_add(1, std::memory_order_relaxed)) {
-                while (piece >= first_piece[k + 1]) ++k;
-                const InChunk ch = in[k];
-                const uint32_t local = piece - first_piece[k], per_op = (ch.span + per_piece - 1) / per_piece;
-                const int op = ch.op != InChunk::kBothOperands ? int(ch.op)
-                               : operands == 2                 ? int(local / per_op)
-                                                               : (a_locked ? 1 : 0);
-                const size_t first = size_t(local % per_op) * per_piece;
-                const size_t last = std::min<size_t>(ch.span, first + per_piece);
-                if (ordered) {  // gather rows s*j + t to their split-major places t*N' + j
-                    const size_t host_row0 = size_t(split) * ch.j0 + ch.t, buf_row0 = size_t(ch.t) * n_sub + ch.j0;
-                    const uint32_t* from = src[op] + host_row0 * limbs;
-                    uint32_t* to = stage + (op * size_t(n) + buf_row0) * limbs;
-                    for (size_t j = first; j < last; ++j) std::memcpy(to + j * limbs, from + j * split * limbs, row);
-                } else {  // a contiguous coefficient range, with streaming stores
-                    const size_t at = (size_t(ch.j0) + first) * limbs;
-                    stage_copy(stage + op * size_t(n) * limbs + at, src[op] + at, (last - first) * row);
-                }
-                store_fence();  // the streaming stores land before the piece is counted
-                packed[k].fetch_add(1, std::memory_order_release);
+            while (piece >= first_piece[k + 1]) ++k;
+            const InChunk ch = in[k];
+            const uint32_t local = piece - first_piece[k], per_op = (ch.span + per_piece - 1) / per_piece;
+            const int op = ch.op != InChunk::kBothOperands ? int(ch.op)
+                           : operands == 2                 ? int(local / per_op)
+                                                           : (a_locked ? 1 : 0);
+            const size_t first = size_t(local % per_op) * per_piece;
+            const size_t last = std::min<size_t>(ch.span, first + per_piece);
+            if (ordered) {  // gather rows s*j + t to their split-major places t*N' + j
+                const size_t host_row0 = size_t(split) * ch.j0 + ch.t, buf_row0 = size_t(ch.t) * n_sub + ch.j0;
+                const uint32_t* from = src[op] + host_row0 * limbs;
+                uint32_t* to = stage + (op * size_t(n) + buf_row0) * limbs;
+                for (size_t j = first; j < last; ++j) std::memcpy(to + j * limbs, from + j * split * limbs, row);
+            } else {  // a contiguous coefficient range, with streaming stores
+                const size_t at = (size_t(ch.j0) + first) * limbs;
+                stage_copy(stage + op * size_t(n) * limbs + at, src[op] + at, (last - first) * row);
             }
+            store_fence();  // the streaming stores land before the piece is counted
+            packed[k].fetch_add(1, std::memory_order_release);
         });
     }
+    auto feed = [&] {
+        if (!pack) return;
+        pack->feed();
+        s.pack_ticket = pack->last();
+    };
+    feed();
+    auto await_packed = [&](uint32_t k) {  // chunk k is in the staging
+        spin_until(s.packed[k], pieces[k], s.team ? s.team->spin_time() : HostTeam::kSpinTime, feed);
+    };
     if (ordered) {
         const bool direct = s.padded_limbs == h.limbs;
         uint32_t* staged = direct ? s.operands : reinterpret_cast<uint32_t*>(s.dots);
         for (uint32_t k = 0; k < in.size(); ++k) {
             const InChunk ch = in[k];
             const size_t host_row0 = size_t(split) * ch.j0 + ch.t, buf_row0 = size_t(ch.t) * n_sub + ch.j0;
-            spin_until(s.packed[k], pieces[k], s.team ? s.team->spin_time() : HostTeam::kSpinTime);
+            await_packed(k);
             for (int op = 0; op < 2; ++op) {
                 const uint32_t* from = src[op] + host_row0 * h.limbs;
                 size_t pitch = split * row;
@@ -770,7 +774,7 @@ void host_begin(negacyclic_plan& s, const uint32_t* a, const uint32_t* b, uint32
             const size_t first = in[k].j0, count = in[k].span, bytes = count * row;  // coefficient range
             const uint32_t op_first = in[k].op == InChunk::kBothOperands ? 0u : in[k].op;
             const uint32_t op_count = in[k].op == InChunk::kBothOperands ? 2u : 1u;
-            spin_until(s.packed[k], pieces[k], s.team ? s.team->spin_time() : HostTeam::kSpinTime);
+            await_packed(k);
             for (uint32_t op = op_first; op < op_first + op_count; ++op) {
                 const uint32_t* from = src[op] + first * h.limbs;
                 if (!locked[op]) from = s.stage_in + op * words + first * h.limbs;  // packed by the team
@@ -840,26 +844,25 @@ int host_finish(negacyclic_plan& s, uint32_t* c) {
         std::vector<InChunk> in;
         std::vector<OutChunk> out;
         stream_chunks(chunk_shape(s), false, in, out);  // the output chunks do not depend on the input order
-        // one unpack job per output chunk, posted as soon as its copy-out has completed: the
+        // each output chunk is unpacked, in turns, as soon as its copy-out has completed: the
         // workers copy their slices of it into c while later chunks are still on the way (and
         // sleep, instead of spinning, while the device computes)
         const uint32_t limbs = h.limbs;
         const uint32_t* stage = s.stage_out;
         std::string failed;
-        uint64_t ticket = 0;
+        HostTeam::Turns turns(*s.team);
         for (uint32_t k = 0; k < out.size(); ++k) {
             const cudaError_t e = cudaEventSynchronize(s.copied_out[k]);
             if (e != cudaSuccess) {
                 failed = cudaGetErrorString(e);
                 break;
             }
-            const size_t words = size_t(out[k].count) * limbs, at = size_t(out[k].first) * limbs;
-            ticket = s.team->post([=](unsigned w, unsigned workers) {
-                const size_t b = HostTeam::slice_begin(words, w, workers), e = HostTeam::slice_begin(words, w + 1, workers);
-                if (e > b) std::memcpy(c + at + b, stage + at + b, (e - b) * 4);
-            });
+            char* to = reinterpret_cast<char*>(c + size_t(out[k].first) * limbs);
+            const char* from = reinterpret_cast<const char*>(stage + size_t(out[k].first) * limbs);
+            HostTeam::post_range(turns, size_t(out[k].count) * limbs * 4,
+                                 [=](size_t b, size_t e) { std::memcpy(to + b, from + b, e - b); });
         }
-        if (ticket) s.team->wait(ticket);
+        s.team->wait(turns.last());
         if (!failed.empty()) return fail(NEGACYCLIC_ECUDA, "copy c: " + failed);
     }
     check(cudaStreamSynchronize(s.copy_out), "product");

@@ -51,8 +51,7 @@ struct negacyclic_plan {
     uint32_t* status_host = nullptr;
     std::shared_ptr<negacyclic::HostTeam> team;     // the process's, held while this plan lives
     std::atomic<uint32_t> packed[kMaxChunks] = {};  // pieces of input chunk k packed
-    std::atomic<uint32_t> next_piece{0};            // next unclaimed piece of the running pack job
-    uint64_t pack_ticket = 0;                       // the running call's pack job (0: none)
+    uint64_t pack_ticket = 0;                       // the running call's last pack turn (0: none)
     bool outputs_staged = false;    // the running host product copies c through stage_out
     size_t device_bytes = 0, table_bytes = 0;
     negacyclic::TensorGemmPlan convert_gemm, crt_gemm;
