@@ -963,7 +963,10 @@ int negacyclic_debug_read(negacyclic_plan* s, int which, void* host, size_t* byt
     }
     if (*bytes < size) return fail(NEGACYCLIC_EINVAL, "host buffer too small");
     DeviceGuard guard(s->device);
-    if (which >= 1 && (s->crt_gather.ready || s->small)) {  // the product kept neither buffer: make them from its residues
+    // what no kernel of the product kept is made from its residues
+    const bool kept_sums = !s->small && !(s->crt_gather.ready && s->crt_reduces);
+    const bool kept_inputs = !s->small && !s->crt_gather.ready;
+    if ((which == 1 && !kept_inputs) || (which == 2 && !kept_sums)) {
         launch_transpose(s->residues, s->crt_in, s->r, s->padded_r, h.n, h.split, 0, h.n_sub, s->stream);
         if (which == 2) enqueue_crt_sums(*s, 0, h.n, s->stream, false);
         if (cudaStreamSynchronize(s->stream) != cudaSuccess)

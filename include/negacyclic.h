@@ -247,9 +247,10 @@ int negacyclic_host_plan(uint32_t n, uint32_t limbs, const uint32_t* q, uint32_t
 /*
  * Copies one internal stage buffer of the last product to host memory, for
  * stage-by-stage checks at small sizes. which: 0 residues [2][r][N] u32 (after
- * the last stage that wrote them), 1 CRT inputs [N][padded_primes] u32,
- * 2 CRT word sums [N][words] u64 (made from the residues where the product's kernels
- * kept neither). Returns the byte size in *bytes when host is NULL.
+ * the last stage that wrote them; a product in one kernel writes the first [r][N]
+ * only), 1 CRT inputs [N][padded_primes] u32, 2 CRT word sums [N][words] u64. A
+ * buffer of 1 and 2 that the product's kernels did not write is made from the
+ * residues. Returns the byte size in *bytes when host is NULL.
  */
 int negacyclic_debug_read(negacyclic_plan* plan, int which, void* host, size_t* bytes);
 

@@ -221,3 +221,44 @@ def test_small_products_of_several_sizes_on_threads(fpc, inputs, oracle):
     for t in threads:
         t.join()
     assert not failed
+
+
+# the word sums that the gathering CRT GEMM leaves (L = 60 up, below N = 16384), from exact products
+@pytest.mark.parametrize("n,limbs,split", [(256, 60, 2), (512, 64, 1), (1024, 100, 4), (512, 123, 2)])
+def test_word_sums_of_gathered_tiles(n, limbs, split, fpc, inputs):
+    import model
+    q, a, b = inputs.instance(n, limbs, 77, 0)
+    setup = model.make_plan(n, limbs, inputs.to_int(q), split)
+    product, weights, _, _ = model.crt_constants(setup)
+    bits = 2 * 32 * limbs + n.bit_length()
+    x, y = (sum(v << (bits * i) for i, v in enumerate(inputs.poly_to_ints(p))) for p in (a, b))
+    z = x * y
+    at = [(z >> (bits * i)) & ((1 << bits) - 1) for i in range(2 * n)]
+    z = [at[i] - at[i + n] for i in range(n)]
+    v = np.array([[zi * pow(product // p, -1, p) % p for p in setup.primes] for zi in z], dtype=np.uint32)
+    words, r = limbs + 5, len(setup.primes)
+    w_bytes = np.frombuffer(b"".join(w.to_bytes(4 * words, "little") for w in weights), np.uint8).reshape(r, 4 * words)
+    columns = np.zeros((n, 4 * words), np.int64)
+    v_bytes = v.view(np.uint8).reshape(n, r, 4).astype(np.int64)
+    for d in range(4):  # column c takes byte c - d of W_k
+        columns[:, d:] += v_bytes[:, :, d] @ w_bytes[:, :4 * words - d].astype(np.int64)
+    sums = (columns.reshape(n, words, 4) << (8 * np.arange(4))).sum(axis=2)
+    with fpc.Plan(n, 32 * limbs, limbs, q, split=split) as plan:
+        assert inputs.poly_to_ints(plan.run(a, b)) == [zi % inputs.to_int(q) for zi in z]
+        # the sums first: reading the CRT inputs may make them from the residues
+        assert np.array_equal(np.frombuffer(plan.debug_read(2), np.int64).reshape(n, words), sums)
+        crt_in = np.frombuffer(plan.debug_read(1), np.uint32).reshape(n, plan.info()["padded_primes"])
+        assert np.array_equal(crt_in[:, :r], v) and not crt_in[:, r:].any()
+
+
+def test_reading_a_stage_buffer_leaves_it_as_it_is(fpc, inputs, torch):
+    """Word sums that the product keeps are read, not made again from the residues."""
+    n, limbs = 512, 64
+    q, a, b = inputs.instance(n, limbs, 77, 0)
+    with fpc.Plan(n, 32 * limbs, limbs, q, external_work=True) as plan:
+        work = torch.empty(plan.work_bytes(), dtype=torch.uint8, device="cuda")
+        plan.bind_work(work.data_ptr(), work.numel())
+        plan.run(a, b)
+        work.fill_(0xA5)
+        torch.cuda.synchronize()
+        assert set(plan.debug_read(2)) == {0xA5}
