@@ -22,7 +22,7 @@ namespace negacyclic {
 namespace {
 
 // One padded row: Lp words (16-byte aligned) from `limbs` words, zeros above.
-__device__ __forceinline__ void pad_row(const uint32_t* __restrict__ src, uint32_t* __restrict__ dst, uint32_t limbs,
+__device__ __forceinline__ void pad_row(const uint32_t* src, uint32_t* __restrict__ dst, uint32_t limbs,
                                         uint32_t padded, uint32_t lane) {
     uint4* out = reinterpret_cast<uint4*>(dst);
     for (uint32_t c = lane; c < padded / 4; c += 32) {
@@ -39,8 +39,7 @@ __device__ __forceinline__ void pad_row(const uint32_t* __restrict__ src, uint32
 // [N][L] a and b -> [2][N][Lp] split-major: output row op*N + t*N' + j holds coefficient
 // s*j + t of operand op. One warp per output row. Also clears the GEMMs' tile counters, so that no
 // memset node stands in the product's chain.
-__global__ void pad_operands_kernel(const uint32_t* __restrict__ a, const uint32_t* __restrict__ b,
-                                    uint32_t* __restrict__ out, uint32_t n, uint32_t limbs, uint32_t padded,
+__global__ void pad_operands_kernel(const uint32_t* a, const uint32_t* b, uint32_t* __restrict__ out, uint32_t n, uint32_t limbs, uint32_t padded,
                                     uint32_t log_split, uint32_t log_n_sub, uint32_t* tile_counters) {
     chain_enter();
     if (blockIdx.x == 0 && threadIdx.x < kTileCounters) tile_counters[threadIdx.x] = 0;
@@ -57,7 +56,7 @@ __global__ void pad_operands_kernel(const uint32_t* __restrict__ a, const uint32
 // from an unpadded [2][N][L] array into the padded split-major layout. Staged rows are either
 // already split-major (log_split = 0: row = position) or in coefficient order (row i goes to
 // t*N' + j, i = s*j + t). One warp per row.
-__global__ void pad_rows_kernel(const uint32_t* __restrict__ staged, uint32_t* __restrict__ out, uint32_t n,
+__global__ void pad_rows_kernel(const uint32_t* staged, uint32_t* __restrict__ out, uint32_t n,
                                 uint32_t limbs, uint32_t padded, uint32_t log_split, uint32_t log_n_sub,
                                 uint32_t first, uint32_t count, uint32_t op_first, uint32_t op_count) {
     chain_enter();
@@ -127,9 +126,8 @@ __global__ void crt_weights_kernel(const uint32_t* __restrict__ weights, uint32_
 // 256 threads, each thread a 4-row x 4-column (one column group) micro-tile.
 constexpr int kTile = 64, kTileK = 64;
 
-__global__ void __launch_bounds__(256) gemm_simt_kernel(const uint8_t* __restrict__ a, uint64_t a_pitch,
-                                                        RowMap rows, uint32_t m_total,
-                                                        const uint8_t* __restrict__ b, uint32_t columns,
+__global__ void __launch_bounds__(256) gemm_simt_kernel(const uint8_t* a, uint64_t a_pitch, RowMap rows,
+                                                        uint32_t m_total, const uint8_t* b, uint32_t columns,
                                                         uint32_t k_bytes, Epilogue epi) {
     chain_enter();
     __shared__ uint32_t as[kTile][kTileK / 4 + 1];
@@ -824,7 +822,7 @@ __global__ void pointwise_kernel(uint32_t* residues, const DevicePrime* __restri
 // padded to 65 words, which keeps both the row-wise writes and the column-wise reads free of bank
 // conflicts. 256 threads: 16 loads in flight per thread.
 constexpr uint32_t kTransposeTile = 64;
-__global__ void __launch_bounds__(256) transpose_kernel(const uint32_t* __restrict__ residues,
+__global__ void __launch_bounds__(256) transpose_kernel(const uint32_t* residues,
                                                         uint32_t* __restrict__ crt_in, uint32_t r, uint32_t padded_r,
                                                         uint32_t n, uint32_t log_split, uint32_t log_n_sub,
                                                         uint32_t j_first, uint32_t j_count) {

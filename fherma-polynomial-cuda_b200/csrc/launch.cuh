@@ -5,12 +5,16 @@
 // finishes.
 //
 // Rules that keep this equal to plain stream order:
-//  * every kernel of the chain calls chain_wait() in every block, and in every thread that touches
-//    memory that a kernel writes or follows one that waited, before that (chain_wait returns once the kernel before it has completed and its writes are
-//    visible). Since that kernel waited likewise, everything earlier on the stream has completed too;
+//  * every block of every kernel of the chain calls chain_wait(), in each thread that touches memory
+//    that another kernel writes, or synchronises with one that called it, before it does. chain_wait()
+//    returns once the kernel before has completed and its writes are visible; since that kernel waited
+//    likewise, everything earlier on the stream has completed too;
 //  * chain_release(), which lets the next kernel's blocks be placed, comes after chain_wait(), so at
 //    most two kernels of a stream are resident, and two CTA-pair GEMMs never are: another kernel
-//    stands between them.
+//    stands between them;
+//  * memory that an earlier kernel of the stream writes (operands, residues, CRT inputs) is not read
+//    through a const __restrict__ pointer or __ldg: those promise data that is constant for the whole
+//    kernel, and a kernel may start before that data is there. A plan's tables may be.
 #pragma once
 #include <cuda_runtime.h>
 
