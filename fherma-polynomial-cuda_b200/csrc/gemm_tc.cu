@@ -195,7 +195,7 @@ __device__ __forceinline__ uint64_t mad_wide(uint32_t a, uint32_t b, uint64_t c)
     return d;
 }
 
-// sum_d v_d 256^d of four byte dots. With K <= 256 bytes a dot is at most 256 * 255^2, and
+// sum_d v_d 256^d of four byte dots. kShort (K <= kGatherRowBytes): a dot is at most 256 * 255^2, and
 // v_0 + 256 v_1 <= 257 * 256 * 255^2 < 2^32: two of the three steps are 32-bit. The epilogue is
 // bound by the integer pipes (two warps per scheduler, 16 lanes wide), so each step counts.
 template <bool kShort>
@@ -1193,7 +1193,7 @@ void launch_gemm_tensor(const TensorGemmPlan& plan, const Epilogue& epilogue, cu
                    GatherSource{}, epilogue);
 }
 
-bool prepare_gemm_gather(TensorGemmPlan& plan, RowMap rows, uint32_t m, const uint8_t* b, uint32_t columns,
+bool prepare_gemm_gather(TensorGemmPlan& plan, GemmSource source, RowMap rows, uint32_t m, const uint8_t* b, uint32_t columns,
                          uint32_t k_bytes, std::string& why) {
     plan.ready = false;
     EncodeTiled encode = encoder();
@@ -1203,6 +1203,10 @@ bool prepare_gemm_gather(TensorGemmPlan& plan, RowMap rows, uint32_t m, const ui
     }
     if (k_bytes < kBlockK || k_bytes % kBlockK || reinterpret_cast<uintptr_t>(b) % 16) {
         why = "K must be whole steps of 128 bytes";
+        return false;
+    }
+    if (source == kSourceTma || (source == kSourceRows && k_bytes > kGatherRowBytes)) {
+        why = "operand rows too long to gather";
         return false;
     }
     if (rows.mode != kRowsSplit || rows.n_sub % kBlockM) {
@@ -1229,6 +1233,7 @@ bool prepare_gemm_gather(TensorGemmPlan& plan, RowMap rows, uint32_t m, const ui
     plan.error_flag = tensor_gemm_error_flag();
     plan.sm_count = device_sm_count();
     plan.pairs = false;
+    plan.source = source;
     plan.ready = true;
     return true;
 }
@@ -1255,7 +1260,7 @@ void launch_gemm_gather(const TensorGemmPlan& plan, const GatherSource& source, 
     const uint32_t slots = resident ? plan.sm_count / n_tiles * n_tiles : plan.sm_count;
     const uint32_t grid = std::min(paired ? m_tiles : tiles, slots);
     const CUtensorMap& b_map = block_n == 128 ? plan.b_map_half : plan.b_map;
-    if (source.kind == kSourceRows)
+    if (plan.source == kSourceRows)
         launch_chained(gemm_tc_kernel<kSourceRows, false>, grid, kGatherThreads, kSmemBytes, stream, b_map, b_map, shape,
                        source, epilogue);
     else if (reduce)

@@ -23,6 +23,7 @@ struct TensorGemmPlan {
     uint64_t a_tile_bytes = 0;        // bytes of one 128-row A tile (raster group sizing)
     bool pairs = false;               // 2-CTA (cta_group::2) 256x256 tiles
     bool narrow = false;              // fewer columns than one tile: TMA fills the rest of B with zeros
+    int source = 0;                   // GemmSource of the A tiles
     bool ready = false;
 };
 
@@ -34,8 +35,12 @@ struct TensorGemmPlan {
 //                   (zeros above).
 enum GemmSource : int { kSourceTma = 0, kSourceRows = 1, kSourceResidues = 2 };
 
+// Longest K, in bytes, of a GEMM that gathers operand rows: its epilogue forms v_0 + 256 v_1 of two byte
+// dots in 32 bits, exact while 257 K 255^2 < 2^32.
+constexpr uint32_t kGatherRowBytes = 256;
+static_assert(257ull * kGatherRowBytes * 255 * 255 < 1ull << 32, "two byte dots in 32 bits");
+
 struct GatherSource {
-    GemmSource kind;
     const uint32_t* rows[2];
     uint32_t limbs;
     bool aligned;  // both operands start on 16 bytes and L is a multiple of 4
@@ -44,8 +49,9 @@ struct GatherSource {
 };
 
 // A GEMM whose A operand is gathered by warps (GatherSource) instead of read by TMA: `rows` is the
-// split row map of the whole shape, k_bytes a multiple of 128. False (with `why`) outside that.
-bool prepare_gemm_gather(TensorGemmPlan& plan, RowMap rows, uint32_t m, const uint8_t* b, uint32_t columns,
+// split row map of the whole shape, k_bytes a multiple of 128, and of operand rows at most
+// kGatherRowBytes. False (with `why`) outside that.
+bool prepare_gemm_gather(TensorGemmPlan& plan, GemmSource source, RowMap rows, uint32_t m, const uint8_t* b, uint32_t columns,
                          uint32_t k_bytes, std::string& why);
 void launch_gemm_gather(const TensorGemmPlan& plan, const GatherSource& source, const Epilogue& epilogue,
                         cudaStream_t stream, const RowMap& rows, uint32_t m);

@@ -85,7 +85,6 @@ void enqueue_convert(negacyclic_plan& s, const uint32_t* a, const uint32_t* b, u
     const uint32_t m = op_count * t_count * span;
     if (s.convert_rows.ready) {  // its callers pass whole tiles (gather_span)
         GatherSource source{};
-        source.kind = kSourceRows;
         source.rows[0] = a;
         source.rows[1] = b;
         source.limbs = h.limbs;
@@ -151,7 +150,6 @@ void enqueue_output(negacyclic_plan& s, uint32_t first, uint32_t count, uint32_t
     const HostPlan& h = s.host;
     if (gather) {
         GatherSource source{};
-        source.kind = kSourceResidues;
         source.residues = s.residues;
         source.r = s.r;
         source.n = h.n;
@@ -264,6 +262,7 @@ WorkLayout work_layout(const negacyclic_plan& s) {
 // L=94), 66.7 / 69.7 (N=8192), 324 / 322 (N=65536); 89.1 / 85.8 at nine (N=8192, L=128). With the
 // reduction in its epilogue: 59.1 / 70.0 (N=32768, L=28), 165.5 / 183.0 (N=65536, L=55).
 constexpr uint32_t kGatherRowSteps = 2, kGatherResidueSteps = 8;
+static_assert(kGatherRowSteps * 128 <= kGatherRowBytes, "the gathered conversion's short word sums");
 
 // The gathering GEMMs of a plan: they read tables only, so they do not depend on the work space.
 void prepare_gather(negacyclic_plan& s) {
@@ -272,9 +271,9 @@ void prepare_gather(negacyclic_plan& s) {
     const RowMap both = RowMap::split_rows(h.n, h.n_sub, h.split, 0, h.n_sub, 0, h.split);
     // (rows that the host path sends in transform order arrive permuted, and are padded)
     if (s.k_convert <= kGatherRowSteps * 128 && !wide_rows(ChunkShape{h.n, h.n_sub, h.split, h.limbs, s.chunks}))
-        prepare_gemm_gather(s.convert_rows, both, 2 * h.n, s.convert_weights, 4 * s.r, s.k_convert, why);
+        prepare_gemm_gather(s.convert_rows, kSourceRows, both, 2 * h.n, s.convert_weights, 4 * s.r, s.k_convert, why);
     if (s.k_crt <= kGatherResidueSteps * 128)
-        prepare_gemm_gather(s.crt_gather, both, h.n, s.crt_weights, 4 * h.words, s.k_crt, why);
+        prepare_gemm_gather(s.crt_gather, kSourceResidues, both, h.n, s.crt_weights, 4 * h.words, s.k_crt, why);
     // Two column tiles of a row tile in turn pay once the row tiles nearly fill the GPU. Product, us, two
     // tiles reduced / word sums and the reduce kernel: 63.1 / 70.7 (N=16384, L=64), 160.8 / 179.5 (N=32768,
     // L=94), 384 / 406 (N=65536, L=122); 66.9 / 64.8 (N=8192, L=122), 43.1 / 39.3 (N=4096, L=94).
