@@ -456,9 +456,9 @@ __global__ void __launch_bounds__(kSource == kSourceTma ? kThreads : kGatherThre
     __syncthreads();
     fence_after();
     const uint32_t tmem = *tmem_slot;
-    // With gathered A only the loaders wait for the kernel before this one: B tiles and every other
-    // table are constant, so the producer fetches B ahead of it, and the MMAs and the epilogue follow
-    // the loaders' stages.
+    // With gathered A the producer fetches B tiles, which are constant, ahead of the kernel before this one.
+    // Every role waits for that kernel before it waits on a barrier, so that those waits' limits count from
+    // its end, however early it let this one start.
     if (kSource == kSourceTma) chain_enter();
 
     if (warp == 0) {
@@ -474,6 +474,7 @@ __global__ void __launch_bounds__(kSource == kSourceTma ? kThreads : kGatherThre
                 for (uint32_t ks = 0; ks < shape.k_tiles; ++ks)
                     tma_load_2d(b_smem + ks * shape.block_n * kBlockK, &b_map, b_full, int(ks * kBlockK),
                                 int(n_tile * shape.block_n));
+                chain_wait();
                 if (!mbar_wait(b_full, 0, shape.limit)) {  // it has to land before the CTA can exit
                     *abort_flag = 1;
                     record_error(shape.status, 1u);
@@ -491,6 +492,7 @@ __global__ void __launch_bounds__(kSource == kSourceTma ? kThreads : kGatherThre
                         withheld = true;
                         break;
                     }
+                    if (kSource != kSourceTma && step == kStages) chain_wait();  // the ring's first round is free
                     if (*abort_flag || !mbar_wait(&empty[s], (round & 1) ^ 1, shape.limit, abort_flag)) {
                         ok = false;
                         break;
@@ -519,6 +521,7 @@ __global__ void __launch_bounds__(kSource == kSourceTma ? kThreads : kGatherThre
             uint32_t s = 0, parity = 0, local = 0;  // ring stage, and its pass's parity
             const uint32_t instr = instr_desc(shape.block_n);
             const bool resident = kSource != kSourceTma && shape.resident;
+            if (kSource != kSourceTma) chain_wait();
             bool ok = !resident || mbar_wait(b_full, 0, shape.limit, abort_flag);
             for (; ok && tile_at(local, shape) < tiles; ++local) {
                 const uint32_t acc = local & 1, use = local >> 1;
@@ -635,6 +638,7 @@ __global__ void __launch_bounds__(kSource == kSourceTma ? kThreads : kGatherThre
         // ---------------- epilogue: warp w reads TMEM lanes 32*(w%4).. (rows of the tile),
         // columns 128*((w-2)/4)..
         const uint32_t quarter = warp & 3, half = (warp - 2) >> 2;
+        if (kSource != kSourceTma) chain_wait();
         for (uint32_t local = 0, tile; (tile = tile_at(local, shape)) < tiles; ++local) {
             const uint32_t acc = local & 1, use = local >> 1;
             // reductions: the two sets of four warps take alternate row tiles, whole
