@@ -473,7 +473,11 @@ int negacyclic_init(uint32_t n, uint32_t w, uint32_t limbs, const uint32_t* q, c
         check(cudaGetLastError(), "table kernels");
         check(cudaStreamSynchronize(st), "plan tables");
         s.small = o.gemm == NEGACYCLIC_GEMM_AUTO && h.split == 1 && prepare_small_product(h.n, s.r, limbs);
-        if (!s.small) {
+        if (s.small) {
+            const size_t kept = size_t(s.r) * h.words * sizeof(uint32_t);
+            s.table_bytes += kept;
+            s.device_bytes += kept;
+        } else {
             cudaFree(s.crt_words);
             s.crt_words = nullptr;
         }

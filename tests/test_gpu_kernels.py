@@ -262,3 +262,18 @@ def test_reading_a_stage_buffer_leaves_it_as_it_is(fpc, inputs, torch):
         work.fill_(0xA5)
         torch.cuda.synchronize()
         assert set(plan.debug_read(2)) == {0xA5}
+
+
+def test_device_bytes_of_a_one_kernel_product(fpc, inputs):
+    """A one-kernel product keeps its CRT weights as words, [r][L+5], beside the general path's tables."""
+    n, limbs = 256, 2
+    q, _, _ = inputs.instance(n, limbs, 6, 0)
+    infos = []
+    for gemm in (fpc.GEMM_AUTO, fpc.GEMM_SIMT):
+        with fpc.Plan(n, 32 * limbs, limbs, q, gemm=gemm) as plan:
+            infos.append(plan.info())
+    small, general = infos
+    assert small["kernels_per_product"] == 1 < general["kernels_per_product"]
+    kept = 4 * small["primes"] * small["words"]
+    assert small["table_bytes"] - general["table_bytes"] == kept
+    assert small["device_bytes"] - general["device_bytes"] == kept
