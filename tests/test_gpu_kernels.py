@@ -277,3 +277,13 @@ def test_device_bytes_of_a_one_kernel_product(fpc, inputs):
     kept = 4 * small["primes"] * small["words"]
     assert small["table_bytes"] - general["table_bytes"] == kept
     assert small["device_bytes"] - general["device_bytes"] == kept
+
+
+# the reduction over two column tiles against exact products: L = 60 and 62 (the second tile holds words of
+# the quotient only), 63, and the last L that fits
+@pytest.mark.parametrize("n,limbs", [(16384, 60), (16384, 62), (16384, 63), (16384, 123), (32768, 91)])
+def test_reduction_over_two_column_tiles_matches_the_oracle(n, limbs, fpc, inputs, oracle, torch):
+    q, a, b = inputs.instance(n, limbs, 300 + limbs, 0)
+    top = inputs.edge_operand(n, q, "max")
+    for x, y in ((a, b), (top, a), (top, top)):
+        assert np.array_equal(device_product(fpc, torch, q, x, y), oracle.kronecker(q, x, y))
