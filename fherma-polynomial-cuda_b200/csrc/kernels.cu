@@ -1156,33 +1156,16 @@ static size_t small_smem(uint32_t n, uint32_t r, uint32_t limbs) {
 // The line lies where the three kernels catch up. Product, us, one kernel / three, at N r L of:
 // 2560 (N=256, L=2) 8.9 / 12.0, 4608 (N=128, L=4) 8.5 / 12.3, 9216 (N=256, L=4) 14.1 / 12.0, 16384 (N=128,
 // L=8) 15.5 / 12.3, 5120 (N=512, L=2) 16.0 / 12.0. At N=64 the tensor GEMMs do not apply: 6272 (L=7) 11.3 /
-// 19.8, 16896 (L=11) 18.1 / 20.
-static bool small_product_takes(uint32_t n, uint32_t r, uint32_t limbs) {
-    return n >= 64 && n <= 256 && r <= kSmallPrimes && small_threads(n, r) <= 512 &&
-           uint64_t(n) * r * limbs <= (n == 64 ? 12288 : 5000);
-}
-
-template <uint32_t kLog>
-static bool prepare_small(size_t smem) {
-    // The limit of a launch is on dynamic and static shared memory together, and belongs to the kernel and
-    // not to the plan: every plan sets the same one, the device's, so that plans on other threads agree.
-    int device = 0, most = 0;
-    cudaFuncAttributes attributes{};
-    if (cudaGetDevice(&device) != cudaSuccess ||
-        cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess ||
-        cudaFuncGetAttributes(&attributes, small_product_kernel<kLog>) != cudaSuccess ||
-        cudaFuncSetAttribute(small_product_kernel<kLog>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             most - int(attributes.sharedSizeBytes)) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
-    return smem + attributes.sharedSizeBytes <= size_t(most);
-}
-
-bool prepare_small_product(uint32_t n, uint32_t r, uint32_t limbs) {
-    if (!small_product_takes(n, r, limbs)) return false;
-    const size_t smem = small_smem(n, r, limbs);
-    return n == 64 ? prepare_small<6>(smem) : n == 128 ? prepare_small<7>(smem) : prepare_small<8>(smem);
+// 19.8, 16896 (L=11) 18.1 / 20. With few primes (q much shorter than its limbs) the L + 5 words that a thread
+// takes one after another count instead: N=64, one prime, 14.9 at L=48, 20.5 at 64, 46.9 at 160 and 55.6 at
+// 192 against 20 at 64, 27 at 160 and 29 at 192.
+// The launch stays within the 48 KB of static and dynamic shared memory that need no attribute (43 KB
+// at most under the other bounds): an attribute would belong to the kernel, not to the plan, and plans on
+// other threads set theirs.
+bool small_product_takes(uint32_t n, uint32_t r, uint32_t limbs) {
+    return n >= 64 && n <= 256 && r <= kSmallPrimes && small_threads(n, r) <= 512 && limbs <= 48 &&
+           uint64_t(n) * r * limbs <= (n == 64 ? 12288 : 5000) &&
+           small_smem(n, r, limbs) + kSmallPrimes * sizeof(DevicePrime) <= 48 * 1024;
 }
 
 template <uint32_t kLog>

@@ -138,7 +138,7 @@ void launch_ntt_inverse(uint32_t* residues, const DevicePrime* primes, const uin
 void launch_transpose(const uint32_t* residues, uint32_t* crt_in, uint32_t r, uint32_t padded_r,
                       uint32_t n, uint32_t split, uint32_t j_first, uint32_t j_count, cudaStream_t stream);
 
-// A whole product in one kernel.
+// A whole product in one kernel, where small_product_takes the ring, the primes and the limbs.
 struct SmallProduct {
     const uint32_t *a, *b;           // [N][L]
     const DevicePrime* primes;
@@ -149,8 +149,7 @@ struct SmallProduct {
     uint32_t* residues;              // receives v_k, [r][N]
     ReduceParams reduce;             // n = N; dots not used
 };
-// Whether it takes the ring, the primes and the limbs on the current device; launches only after this.
-bool prepare_small_product(uint32_t n, uint32_t r, uint32_t limbs);
+bool small_product_takes(uint32_t n, uint32_t r, uint32_t limbs);
 void launch_small_product(const SmallProduct& params, cudaStream_t stream);
 
 // Words the tables of launch_reduce hold: whole chunks of 64 covering L + 2 words.

@@ -472,7 +472,7 @@ int negacyclic_init(uint32_t n, uint32_t w, uint32_t limbs, const uint32_t* q, c
         launch_crt_weights(s.crt_words, s.r, s.padded_r, h.words, s.crt_columns, s.crt_weights, st);
         check(cudaGetLastError(), "table kernels");
         check(cudaStreamSynchronize(st), "plan tables");
-        s.small = o.gemm == NEGACYCLIC_GEMM_AUTO && h.split == 1 && prepare_small_product(h.n, s.r, limbs);
+        s.small = o.gemm == NEGACYCLIC_GEMM_AUTO && h.split == 1 && small_product_takes(h.n, s.r, limbs);
         if (s.small) {
             const size_t kept = size_t(s.r) * h.words * sizeof(uint32_t);
             s.table_bytes += kept;

@@ -186,10 +186,11 @@ def test_residues_past_four_gigabytes(fpc, inputs, oracle, torch):
             assert np.array_equal(row, dc[i].cpu().numpy().view(np.uint32)), (gemm, i)
 
 
-# one-kernel products with few primes and many zero limbs above q: 44 to 51 KB of shared memory
-@pytest.mark.parametrize("limbs", range(85, 94))
+# few primes and many zero limbs above q: the last one-kernel products (L = 48), and around 48 KB of their
+# shared memory
+@pytest.mark.parametrize("limbs", [47, 48, 49, *range(85, 94)])
 @pytest.mark.parametrize("qv", [2001, (1 << 24) - 3, (1 << 27) - 39])
-def test_small_products_around_the_shared_memory_default(limbs, qv, fpc, inputs, oracle, torch):
+def test_small_products_with_zero_limbs(limbs, qv, fpc, inputs, oracle, torch):
     n, q = 64, inputs.from_int(qv, limbs)
     rng = np.random.Generator(np.random.PCG64(limbs))
     a, b = (np.pad(inputs.random_operand(rng, n, q[:1]), ((0, 0), (0, limbs - 1))) for _ in range(2))
@@ -215,7 +216,7 @@ def test_small_products_of_several_sizes_on_threads(fpc, inputs, oracle):
         except Exception as e:
             failed.append((limbs, repr(e)))
 
-    threads = [threading.Thread(target=worker, args=(limbs,)) for limbs in (100, 150, 192)]
+    threads = [threading.Thread(target=worker, args=(limbs,)) for limbs in (20, 48, 100, 192)]
     for t in threads:
         t.start()
     for t in threads:
@@ -287,3 +288,10 @@ def test_reduction_over_two_column_tiles_matches_the_oracle(n, limbs, fpc, input
     top = inputs.edge_operand(n, q, "max")
     for x, y in ((a, b), (top, a), (top, top)):
         assert np.array_equal(device_product(fpc, torch, q, x, y), oracle.kronecker(q, x, y))
+
+
+def test_many_zero_limbs_do_not_run_as_one_kernel(fpc, inputs):
+    """N=64 with one prime: a thread's chain of L + 5 words made L = 192 slower in one kernel than in stages."""
+    for limbs, one in ((4, True), (48, True), (49, False), (192, False)):
+        with fpc.Plan(64, 32 * limbs, limbs, inputs.from_int(2001, limbs)) as plan:
+            assert (plan.info()["kernels_per_product"] == 1) == one, limbs
