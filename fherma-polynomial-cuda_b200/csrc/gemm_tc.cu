@@ -1142,7 +1142,6 @@ bool prepare_gemm_tensor(TensorGemmPlan& plan, const uint8_t* a, uint64_t a_pitc
     plan.k_tiles = (k_bytes + kBlockK - 1) / kBlockK;
     plan.rows = rows;
     plan.a_tile_bytes = uint64_t(kBlockM) * k_bytes;
-    plan.error_flag = tensor_gemm_error_flag();
     if (!plan.tile_counter) {  // callers that keep GEMMs of one plan on one stream may bind their own
         void* counter = nullptr;
         if (cudaGetSymbolAddress(&counter, g_tile_counter) != cudaSuccess) {
@@ -1234,7 +1233,6 @@ bool prepare_gemm_gather(TensorGemmPlan& plan, GemmSource source, RowMap rows, u
     plan.k_tiles = k_bytes / kBlockK;
     plan.rows = rows;
     plan.a_tile_bytes = uint64_t(kBlockM) * k_bytes;
-    plan.error_flag = tensor_gemm_error_flag();
     plan.sm_count = device_sm_count();
     plan.pairs = false;
     plan.source = source;

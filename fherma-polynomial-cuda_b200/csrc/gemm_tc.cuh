@@ -16,7 +16,6 @@ struct TensorGemmPlan {
     uint32_t m = 0, columns = 0, k_bytes = 0;
     uint32_t m_tiles = 0, n_tiles = 0, k_tiles = 0;
     RowMap rows{};
-    uint32_t* error_flag = nullptr;  // device word set when a pipeline wait times out
     uint32_t* tile_counter = nullptr;  // device word the CTA-pair kernel claims tiles from; GEMMs that
                                        // share one may not run at the same time
     uint32_t sm_count = 148;          // persistent grid size

@@ -43,7 +43,8 @@ inline uint32_t host_chunks(uint32_t n, uint32_t n_sub, uint32_t split) {
 
 // Rows of at least 1 KB: chunks carry enough work that finer chunks near the ends (and one
 // transpose per output chunk) pay for their extra launches. Narrower rows keep equal chunks.
-inline bool wide_rows(const ChunkShape& s) { return s.limbs >= 256; }
+constexpr uint32_t kWideRowLimbs = 256;
+inline bool wide_rows(const ChunkShape& s) { return s.limbs >= kWideRowLimbs; }
 
 // Transform order needs rows gathered with a stride of s rows, by the copy engine as a 2-D copy
 // or by the host team while it packs pageable operands. Both pay only for rows of 1 KB or more:

@@ -269,8 +269,9 @@ void prepare_gather(negacyclic_plan& s) {
     const HostPlan& h = s.host;
     std::string why;
     const RowMap both = RowMap::split_rows(h.n, h.n_sub, h.split, 0, h.n_sub, 0, h.split);
-    // (rows that the host path sends in transform order arrive permuted, and are padded)
-    if (s.k_convert <= kGatherRowSteps * 128 && !wide_rows(ChunkShape{h.n, h.n_sub, h.split, h.limbs, s.chunks}))
+    // (rows that the host path sends in transform order arrive permuted, and are padded: those are wide)
+    static_assert(kGatherRowSteps * 32 < kWideRowLimbs, "gathered rows arrive in coefficient order");
+    if (s.k_convert <= kGatherRowSteps * 128)
         prepare_gemm_gather(s.convert_rows, kSourceRows, both, 2 * h.n, s.convert_weights, 4 * s.r, s.k_convert, why);
     if (s.k_crt <= kGatherResidueSteps * 128)
         prepare_gemm_gather(s.crt_gather, kSourceResidues, both, h.n, s.crt_weights, 4 * h.words, s.k_crt, why);
