@@ -104,14 +104,21 @@ __device__ __forceinline__ bool mbar_try(uint64_t* bar, uint32_t parity) {
 }
 
 // Bounded wait for the phase with the given parity to complete: false after `limit` cycles, or
-// (when `abort` is given) as soon as another role has raised the abort flag.
+// (when `abort` is given) as soon as another role has raised the abort flag. The cycles count from when
+// `started` (when given) is set.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, long long limit,
-                                          const volatile uint32_t* abort = nullptr) {
+                                          const volatile uint32_t* abort = nullptr,
+                                          const volatile uint32_t* started = nullptr) {
     if (mbar_try(bar, parity)) return true;  // the usual case costs no clock read
-    const long long start = clock64();
+    long long start = clock64();
     for (uint32_t i = 0;; ++i) {
         if (mbar_try(bar, parity)) return true;
-        if ((i & 63u) == 63u && ((abort && *abort) || clock64() - start > limit)) return false;
+        if ((i & 63u) != 63u) continue;
+        if (abort && *abort) return false;
+        if (started && !*started)
+            start = clock64();
+        else if (clock64() - start > limit)
+            return false;
     }
 }
 
@@ -428,6 +435,10 @@ __global__ void __launch_bounds__(kSource == kSourceTma ? kThreads : kGatherThre
     uint64_t* b_full = drain + 1;          // resident B has landed
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(b_full + 1);
     volatile uint32_t* abort_flag = tmem_slot + 1;
+    // gathered A: set once the kernel before has ended. The other roles may be placed while it runs; their
+    // waits' limits count from here, however early it let this kernel start. (Waiting for that kernel in every
+    // role instead cost 0.4 us: 55.9 -> 56.3 at N=32768, L=28, 160.7 -> 161.1 at N=65536, L=55.)
+    volatile uint32_t* started = kSource == kSourceTma ? nullptr : tmem_slot + 2;
 
     const uint32_t warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     const uint32_t tiles = shape.m_tiles * shape.n_tiles;
@@ -444,6 +455,7 @@ __global__ void __launch_bounds__(kSource == kSourceTma ? kThreads : kGatherThre
         mbar_init(drain, 1);
         mbar_init(b_full, 1);
         *abort_flag = 0;
+        if (started) *started = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
@@ -456,9 +468,9 @@ __global__ void __launch_bounds__(kSource == kSourceTma ? kThreads : kGatherThre
     __syncthreads();
     fence_after();
     const uint32_t tmem = *tmem_slot;
-    // With gathered A the producer fetches B tiles, which are constant, ahead of the kernel before this one.
-    // Every role waits for that kernel before it waits on a barrier, so that those waits' limits count from
-    // its end, however early it let this one start.
+    // With gathered A only the loaders wait for the kernel before this one: B tiles and every other
+    // table are constant, so the producer fetches B ahead of it, and the MMAs and the epilogue follow
+    // the loaders' stages.
     if (kSource == kSourceTma) chain_enter();
 
     if (warp == 0) {
@@ -474,8 +486,7 @@ __global__ void __launch_bounds__(kSource == kSourceTma ? kThreads : kGatherThre
                 for (uint32_t ks = 0; ks < shape.k_tiles; ++ks)
                     tma_load_2d(b_smem + ks * shape.block_n * kBlockK, &b_map, b_full, int(ks * kBlockK),
                                 int(n_tile * shape.block_n));
-                chain_wait();
-                if (!mbar_wait(b_full, 0, shape.limit)) {  // it has to land before the CTA can exit
+                if (!mbar_wait(b_full, 0, shape.limit, nullptr, started)) {  // it has to land before the CTA can exit
                     *abort_flag = 1;
                     record_error(shape.status, 1u);
                 }
@@ -492,8 +503,7 @@ __global__ void __launch_bounds__(kSource == kSourceTma ? kThreads : kGatherThre
                         withheld = true;
                         break;
                     }
-                    if (kSource != kSourceTma && step == kStages) chain_wait();  // the ring's first round is free
-                    if (*abort_flag || !mbar_wait(&empty[s], (round & 1) ^ 1, shape.limit, abort_flag)) {
+                    if (*abort_flag || !mbar_wait(&empty[s], (round & 1) ^ 1, shape.limit, abort_flag, started)) {
                         ok = false;
                         break;
                     }
@@ -521,18 +531,17 @@ __global__ void __launch_bounds__(kSource == kSourceTma ? kThreads : kGatherThre
             uint32_t s = 0, parity = 0, local = 0;  // ring stage, and its pass's parity
             const uint32_t instr = instr_desc(shape.block_n);
             const bool resident = kSource != kSourceTma && shape.resident;
-            if (kSource != kSourceTma) chain_wait();
-            bool ok = !resident || mbar_wait(b_full, 0, shape.limit, abort_flag);
+            bool ok = !resident || mbar_wait(b_full, 0, shape.limit, abort_flag, started);
             for (; ok && tile_at(local, shape) < tiles; ++local) {
                 const uint32_t acc = local & 1, use = local >> 1;
-                if (*abort_flag || !mbar_wait(&acc_empty[acc], (use & 1) ^ 1, shape.limit, abort_flag)) {
+                if (*abort_flag || !mbar_wait(&acc_empty[acc], (use & 1) ^ 1, shape.limit, abort_flag, started)) {
                     ok = false;
                     break;
                 }
                 fence_after();
                 const uint32_t d_tmem = tmem + acc * kAccColumns;
                 for (uint32_t ks = 0; ks < shape.k_tiles; ++ks) {
-                    if (!mbar_wait(&full[s], parity, shape.limit, abort_flag)) {
+                    if (!mbar_wait(&full[s], parity, shape.limit, abort_flag, started)) {
                         ok = false;
                         break;
                     }
@@ -566,6 +575,7 @@ __global__ void __launch_bounds__(kSource == kSourceTma ? kThreads : kGatherThre
     } else if (kSource != kSourceTma && warp >= 2 + kEpilogueWarps) {
         // ---------------- A loaders
         chain_enter();
+        if (warp == 2 + kEpilogueWarps && lane == 0) *started = 1;
         const uint32_t part = warp - (2 + kEpilogueWarps);  // rows 32 part .. 32 part + 31 of the tile
         const uint32_t a_addr = smem_u32(a_smem) + part * 32 * kBlockK;
         uint32_t step = 0, published = 0;
@@ -638,7 +648,6 @@ __global__ void __launch_bounds__(kSource == kSourceTma ? kThreads : kGatherThre
         // ---------------- epilogue: warp w reads TMEM lanes 32*(w%4).. (rows of the tile),
         // columns 128*((w-2)/4)..
         const uint32_t quarter = warp & 3, half = (warp - 2) >> 2;
-        if (kSource != kSourceTma) chain_wait();
         for (uint32_t local = 0, tile; (tile = tile_at(local, shape)) < tiles; ++local) {
             const uint32_t acc = local & 1, use = local >> 1;
             // reductions: the two sets of four warps take alternate row tiles, whole
@@ -648,7 +657,7 @@ __global__ void __launch_bounds__(kSource == kSourceTma ? kThreads : kGatherThre
             const uint32_t row0 = m_tile * kBlockM, col0 = n_tile * shape.block_n;
             const bool row_tile = kReduce && shape.paired;
             bool have = !*abort_flag && mbar_wait(&acc_full[row_tile ? half : acc], (row_tile ? use >> 1 : use) & 1,
-                                                  shape.limit, abort_flag);
+                                                  shape.limit, abort_flag, started);
             have = __all_sync(0xffffffffu, have);
             if (!have) {
                 if (lane == 0) {
