@@ -65,14 +65,14 @@ CPU_SAMPLE_N = N // 16  # bounded CPU sample: 4096 coefficients of the same widt
 # profiles/cpu_baseline_gmp_N65536_L1747.md); without it the linear factor N / CPU_SAMPLE_N is used
 CPU_FULL_OVER_SAMPLE = 19.35  # 77.74 s against 4.01 s (median of 3), 16-core Xeon host of a B200 box
 # DRAM bytes (read + write) of one conversion-GEMM launch on this workload, from a one-pass ncu
-# capture (dram__bytes_read.sum 4.32 GB + dram__bytes_write.sum 1.90 GB) of
+# capture (dram__bytes_read.sum 4.35 GB + dram__bytes_write.sum 1.90 GB) of
 #   python bench.py --workload 65536,1747 --steps 1 --warmup 1 --device-only
-CONVERT_DRAM_BYTES = 6.22e9
+CONVERT_DRAM_BYTES = 6.25e9
 # sm__pipe_tensor_cycles_active of the conversion GEMM alone, from the single-kernel capture
 #   ncu --set full --clock-control none -k regex:gemm_tc -c 2 \
 #       python bench.py --workload 16384,1747 --steps 1 --warmup 1 --device-only
 # (profiles/gemm_tc_N16384_L1747.md): the clock-free fraction of the int8 tensor pipe's peak
-CONVERT_TENSOR_PIPE_ACTIVE = 0.836
+CONVERT_TENSOR_PIPE_ACTIVE = 0.903
 
 
 def _load(name, path, package_dir=None):
@@ -687,7 +687,7 @@ def run_batch(args):
                          "plain_products_per_s": len(instances) / (host_plain_ms / 1000),
                          "batched_over_plain": host_plain_ms / host_batched_ms,
                          "bytes_per_batch": int(sum(3 * a.nbytes for _, _, _, a, _ in instances))},
-            "lanes": args.lanes or "two phases (concurrent small instances on up to 4 lanes, then large ones alone)",
+            "lanes": args.lanes or "two phases (concurrent small instances on up to 6 lanes, then large ones alone)",
             "concurrent_phase": small,
             "tuned": bool(args.tune), "setup_s": setup_s,
             "steps": args.steps, "warmup": args.warmup, "data": "synthetic (seed 100)"}

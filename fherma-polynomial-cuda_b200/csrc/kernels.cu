@@ -249,7 +249,7 @@ __global__ void __launch_bounds__(512) ntt_inverse_kernel(uint32_t* residues, co
 }
 
 // ---------------------------------------------------------------------------
-// Register-blocked NTT for N' >= 256: 16 values per thread (32 at N' = 8192), up to four (five)
+// Register-blocked NTT for N' >= 256 (from 64 in the kernels that do whole products): 16 values per thread (32 at N' = 8192), up to four (five)
 // butterfly stages per pass between shared-memory exchanges.
 // A pass of R stages on group g (2^R values spaced t_min apart, t_min = the
 // smallest half-size in the pass) covers indices base + k*t_min, k < 2^R, with
@@ -260,8 +260,8 @@ __global__ void __launch_bounds__(512) ntt_inverse_kernel(uint32_t* residues, co
 // three passes, one exchange fewer than 4 + 4 + 4 + 1, in four CTAs of 256 threads per SM instead of
 // two of 512, so that one CTA's loads and barriers fall into another's arithmetic; twiddles are loaded in
 // pairs, and those of the unit-stride pass from a table laid out for it. 16450 warp instructions per
-// transform instead of 18600. Forward 2010 -> 1840 us and inverse 1226 -> 961 us at N = 65536,
-// L = 1747 (58176 and 29088 transforms; 2.1 TB/s). Keeping the next transform's input on its way into
+// transform instead of 18600. Forward 2010 -> 1810 us and inverse 1226 -> 890 us (961 before its scaling
+// went into the last stage) at N = 65536, L = 1747 (58176 and 29088 transforms; 2.1 TB/s). Keeping the next transform's input on its way into
 // shared memory (persistent CTAs), or 16 values per thread with three CTAs of 512, were slower.
 
 constexpr uint32_t per_thread(uint32_t log) { return log == 13 ? 32 : 16; }  // values per thread
@@ -869,7 +869,6 @@ __global__ void __launch_bounds__(256) transpose_kernel(const uint32_t* residues
 // back through the same slot, so that global stores are runs of 64 or 128 bytes. Measured against
 // the earlier form (stage between events): 624 -> 362 us at N = 65536, L = 1747 (1.38 GB, 3.8 TB/s),
 // 142 -> 90 us at N = 32768, L = 868, 49 -> 20.5 us at N = 65536, L = 55.
-
 //
 // Few rows: a thread's chain of L + 2 words is then all there is to wait for, so a row is cut into
 // kSegments segments, one lane each. A segment starts with no carry; afterwards each passes its carry

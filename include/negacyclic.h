@@ -104,7 +104,8 @@ int negacyclic_get_info(const negacyclic_plan* plan, negacyclic_info* info);
  * overlaps the copy-out of chunk k on the way out. Page-locked host memory (cudaHostAlloc /
  * cudaHostRegister) is read and written by DMA directly; pageable memory goes
  * through the plan's page-locked staging buffers, filled and drained by a team of
- * host threads.
+ * host threads that all plans of the process share. Calls on different plans may run
+ * on different threads; their copies take turns on the team.
  */
 int negacyclic_run(negacyclic_plan* plan, const uint32_t* a, const uint32_t* b, uint32_t* c);
 
@@ -119,7 +120,7 @@ int negacyclic_prepare_host(negacyclic_plan* plan);
  * negacyclic_run in two halves, so that a caller can do host work (such as
  * allocating the output array) while the device computes: begin enqueues
  * everything with the result staged in page-locked memory (pageable inputs are
- * packed into staging by the plan's host threads, each chunk handed to the copy
+ * packed into staging by the host threads, each chunk handed to the copy
  * engine as soon as it is packed); finish waits and has the host threads copy
  * each output chunk into c as it lands. a and b must stay valid until finish
  * returns.
@@ -128,7 +129,7 @@ int negacyclic_run_begin(negacyclic_plan* plan, const uint32_t* a, const uint32_
 int negacyclic_run_finish(negacyclic_plan* plan, uint32_t* c);
 
 /*
- * Writes zeros over host memory [ptr, ptr + bytes) with the plan's host threads, so
+ * Writes zeros over host memory [ptr, ptr + bytes) with the host threads, so
  * that the first touch of a freshly allocated output array (page faults and the
  * kernel's zeroing, about 0.35 ms per MB on one core) is paid by all of them at
  * once. For callers that must allocate a new output array per product, as the
